@@ -6,7 +6,8 @@
 // stencil: per node the centre block and the E, S, SE, SW coupling blocks (the other
 // four couplings are the transposes of the neighbours' blocks), each D x D, stored
 // coefficient-major ([row][coef][node]) so a warp reads one coefficient coalesced.
-// The coarsest level is factorised by a block-banded FP64 Cholesky.
+// The coarsest level is factorised in FP64: by odd-even elimination of its grid lines
+// (coarse.cu), or, where its lines are wider than 64 unknowns, as a block-banded matrix.
 #pragma once
 
 #include <atomic>
@@ -44,11 +45,12 @@ struct LevelDesc {
 
 struct CoarseDesc {
   int n;             // dofs of the coarsest level
-  int B;             // block size (>= half bandwidth)
-  int nb;            // blocks, n padded to nb * B
+  int tree;          // 1: odd-even elimination of the grid lines (coarse.cu); 0: banded
+  int B;             // block size: a line's dofs padded to 8 (tree), or >= the half bandwidth
+  int nb;            // blocks: the grid lines (tree), or n padded to nb * B
   int by_col;        // dof ordering: 1 = column-major nodes (nny < nnx), 0 = row-major
-  double* blocks;    // [hrows][nb][4][B][B]: Dinv, Dinv^T, E, E^T (E_k = L_{k,k-1})
-  double* inv;       // [hrows][nb B][nb B] explicit inverse (FP32 cycles, B <= 64), or null
+  double* blocks;    // [hrows][nb][4][B][B]: X, F_l, coupling, F_r (tree), or Dinv, Dinv^T,
+                     // E, E^T (E_k = L_{k,k-1})
 };
 
 // The coarsest level's factorisation runs on a stream of its own, concurrently with the
@@ -58,11 +60,7 @@ struct CoarseSync {
   int device = 0;
   cudaStream_t side = nullptr;
   cudaEvent_t built = nullptr, ready = nullptr;
-  cudaEvent_t factored = nullptr;  // the band factor is done (the inverse may still run)
   std::atomic<int> refs{1};
-  // an FP32 hierarchy's first coarse solve takes the block solves, which need only the
-  // factor, so it does not wait for the explicit inverse (set at the build, taken once)
-  std::atomic<int> first_cycle{0};
   // level 1's FP64 stencil not yet assembled (an FP32 hierarchy swept from the densities
   // builds only the FP32 diagonal its cycle reads); the first entry point that reads the
   // FP64 stencil assembles it, under l1_mu.  Shared by the hierarchy's views.

@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "errors.h"
+#include "coarse.h"
 #include "hier.h"
 #include "modal.h"
 #include "q4.cuh"
@@ -73,7 +74,6 @@ static void galerkin_table(const double* S, const double* K, int nm, int nk, dou
   }
 }
 
-constexpr int kCoarseInvMaxRows = 48;  // hierarchy rows up to which the FP32 cycle uses the coarse inverse
 constexpr int kTableStride = 9 * 64;   // doubles per table (max 9 children x 8 x 8)
 constexpr int kGrandStride = 81 * 64;  // doubles per grandchild table (max 81 x 8 x 8)
 constexpr int kChildStencilSize = 2 * 5 * 4 * 4 * 9;  // stencil_children_kernel tables, D = 2, 9 children
@@ -209,26 +209,8 @@ long long plan_hierarchy(stt_hier_impl& h, char* base) {
         lv.st32 = (float*)carve(p, used, 4LL * h.hrows * (d == 2 ? st32_nsp<2>() : st32_nsp<1>()) * lv.nnode);
     }
   }
-  // coarse factor
-  {
-    const LevelDesc& c = h.lv[L - 1];
-    CoarseDesc& co = h.co;
-    co.n = (int)c.ndof;
-    co.by_col = c.nny < c.nnx ? 1 : 0;
-    const int nmin = co.by_col ? c.nny : c.nnx;
-    const int bw = d * (nmin + 2) - 1;  // max |P - Q| of a nonzero
-    co.B = ((bw + 31) / 32) * 32;
-    if (co.B < 32) co.B = 32;
-    co.nb = (co.n + co.B - 1) / co.B;
-    co.blocks = (double*)carve(p, used, 8LL * h.hrows * co.nb * 4 * co.B * co.B);
-    // the FP32 cycle solves the coarsest level with the explicit inverse (one GEMV) while
-    // the hierarchy has few rows: the GEMV streams np^2 doubles a row per cycle, the block
-    // solves ~8 B^2 nb, and from about 48 rows on (one CTA a row filling the SMs) the
-    // latency-bound block solves cost less than the inverse's bytes and its build
-    const long long np = (long long)co.nb * co.B;
-    co.inv = (f32 && co.B <= 64 && h.hrows <= kCoarseInvMaxRows) ? (double*)carve(p, used, 8LL * h.hrows * np * np)
-                                                                   : nullptr;
-  }
+  coarse_plan(h.lv[L - 1], d, h.co);
+  h.co.blocks = (double*)carve(p, used, 8LL * h.hrows * h.co.nb * 4 * h.co.B * h.co.B);
   h.tables = (double*)carve(p, used, 8LL * kMaxLevels * 3 * kTableStride);
   h.gtables = (double*)carve(p, used, 8LL * (2 * kGrandStride + kChildStencilSize));
   // level 1 is assembled straight from the level-0 densities and level 2's element
@@ -895,239 +877,6 @@ __global__ void __launch_bounds__(256) band_factor_kernel(double* __restrict__ b
   if (tid == 0 && bad) atomicOr(status, 1);
 }
 
-// 16-byte asynchronous global -> shared copies (sm_80+ cp.async), for prefetching the
-// next blocks while the current one factors.
-STT_DEV void cp_async16(void* smem, const void* gmem) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem));
-}
-STT_DEV void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-STT_DEV void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-
-// The same factorisation for B = 16 NA (NA = 2, 4), 256 threads as a 16 x 16 grid:
-//   * thread (ty, tx) owns the strided tile of entries (ty + 16 a, tx + 16 b), a, b < NA,
-//     of every B x B product, so each shared-memory load feeds NA multiply-adds (a warp
-//     reads 2 rows of one operand, broadcast, and 16 rows of the other at a stride of
-//     B + 1 doubles, conflict-free);
-//   * the Cholesky takes two columns per pair of barriers: every thread forms both
-//     pivots and the two scaled columns of its rows and columns in registers (column
-//     j + 1 updated by column j on the fly), then applies the rank-2 trailing update;
-//   * A_{k+1,k+1} and A_{k+1,k} are copied into staging buffers with cp.async while
-//     block k factors; the Schur update and E = A_{k+1,k} X^T read them from there.
-// Upper triangles of the work arrays carry harmless values (only lower triangles are
-// read); X = D^{-1} keeps exact zeros above its diagonal.
-template <int NA>
-__global__ void __launch_bounds__(256) band_factor_tiled_kernel(double* __restrict__ blocks, int nb,
-                                                                int* __restrict__ status) {
-  constexpr int B = 16 * NA, ld = B + 1;
-  extern __shared__ __align__(16) double sm[];
-  double* P0 = sm;           // staged A_{k,k} (B x B, dense rows)
-  double* P1 = P0 + B * B;   // staged A_{k+1,k}
-  double* A = P1 + B * B;    // current diagonal block, then its Cholesky factor (ld)
-  double* X = A + B * ld;    // D_k^{-1}
-  double* Y = X + B * ld;    // E_k
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-  double* bh = blocks + (size_t)blockIdx.x * nb * 4 * B * B;
-  __shared__ int bad;
-  __shared__ double rp[B];  // reciprocals of the current block's pivots
-  if (tid == 0) bad = 0;
-  auto stage = [&](double* dst, const double* src) {
-    for (int t = tid; t < B * B / 2; t += 256) cp_async16(dst + 2 * t, src + 2 * t);
-  };
-  stage(P0, bh);
-  cp_async_commit();
-  for (int k = 0; k < nb; ++k) {
-    double* Dk = bh + (size_t)k * 4 * B * B;
-    cp_async_wait_all();
-    __syncthreads();
-    // A = A_kk - E_k E_k^T (k > 0)
-    {
-      double acc[NA][NA];
-#pragma unroll
-      for (int a = 0; a < NA; ++a)
-#pragma unroll
-        for (int b = 0; b < NA; ++b) acc[a][b] = 0.0;
-      if (k > 0) {
-#pragma unroll 4
-        for (int m = 0; m < B; ++m) {
-          double yi[NA], yl[NA];
-#pragma unroll
-          for (int a = 0; a < NA; ++a) yi[a] = Y[(ty + 16 * a) * ld + m];
-#pragma unroll
-          for (int b = 0; b < NA; ++b) yl[b] = Y[(tx + 16 * b) * ld + m];
-#pragma unroll
-          for (int a = 0; a < NA; ++a)
-#pragma unroll
-            for (int b = 0; b < NA; ++b) acc[a][b] = fma(yi[a], yl[b], acc[a][b]);
-        }
-      }
-#pragma unroll
-      for (int a = 0; a < NA; ++a)
-#pragma unroll
-        for (int b = 0; b < NA; ++b) {
-          const int i = ty + 16 * a, l = tx + 16 * b;
-          A[i * ld + l] = P0[i * B + l] - acc[a][b];
-        }
-    }
-    __syncthreads();  // P0 consumed, A complete
-    if (k + 1 < nb) {
-      double* Dn = bh + (size_t)(k + 1) * 4 * B * B;
-      stage(P0, Dn);                    // A_{k+1,k+1}
-      stage(P1, Dn + (size_t)2 * B * B);  // A_{k+1,k}
-      cp_async_commit();
-    }
-    // Cholesky, a panel of four columns per step: every thread factors the 4 x 4 pivot
-    // block (one rsqrt a pivot, L_jj = t rsqrt(t), its reciprocal kept for the
-    // substitution), then the panel entries of its rows and a rank-4 update
-    for (int j = 0; j < B; j += 4) {
-      double a[4][4];
-#pragma unroll
-      for (int p = 0; p < 4; ++p)
-#pragma unroll
-        for (int q = 0; q <= p; ++q) a[p][q] = A[(j + p) * ld + j + q];
-      double l[4][4], r[4];
-      bool ok = true;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        double t = a[q][q];
-#pragma unroll
-        for (int m = 0; m < q; ++m) t = fma(-l[q][m], l[q][m], t);
-        ok = ok && t > 0.0;
-        const double tt = t > 0.0 ? t : 1.0;
-        r[q] = rsqrt(tt);
-        l[q][q] = tt * r[q];
-#pragma unroll
-        for (int p = q + 1; p < 4; ++p) {
-          double v = a[p][q];
-#pragma unroll
-          for (int m = 0; m < q; ++m) v = fma(-l[p][m], l[q][m], v);
-          l[p][q] = v * r[q];
-        }
-      }
-      // the panel columns of rows i (this thread's rows) and of rows c (its columns)
-      auto panel = [&](int i, double (&cv)[4]) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          double v = 0.0;
-          if (i > j + q) {
-            v = A[i * ld + j + q];
-#pragma unroll
-            for (int m = 0; m < q; ++m) v = fma(-cv[m], l[q][m], v);
-            v *= r[q];
-          }
-          cv[q] = v;
-        }
-      };
-      double ci[NA][4], cl[NA][4];
-#pragma unroll
-      for (int a2 = 0; a2 < NA; ++a2) panel(ty + 16 * a2, ci[a2]);
-#pragma unroll
-      for (int b = 0; b < NA; ++b) panel(tx + 16 * b, cl[b]);
-      __syncthreads();
-      if (tx == 0) {
-#pragma unroll
-        for (int a2 = 0; a2 < NA; ++a2) {
-          const int i = ty + 16 * a2;
-#pragma unroll
-          for (int q = 0; q < 4; ++q)
-            if (i > j + q) A[i * ld + j + q] = ci[a2][q];
-        }
-      }
-      if (tid == 0) {
-        if (!ok) bad = 1;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          A[(j + q) * ld + j + q] = l[q][q];
-          rp[j + q] = r[q];
-        }
-      }
-#pragma unroll
-      for (int a2 = 0; a2 < NA; ++a2)
-#pragma unroll
-        for (int b = 0; b < NA; ++b) {
-          const int i = ty + 16 * a2, c = tx + 16 * b;
-          if (i > j + 3 && c > j + 3) {
-            double v = A[i * ld + c];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) v = fma(-ci[a2][q], cl[b][q], v);
-            A[i * ld + c] = v;
-          }
-        }
-      __syncthreads();
-    }
-    // X = A^{-1}: forward substitution with the pivots' reciprocals, a quad of threads a
-    // column, each thread's share of a dot product in two independent chains
-    {
-      const int q = tid & 3;
-      for (int c0 = 0; c0 < B; c0 += 64) {
-        const int c = c0 + tid / 4;
-        const bool col = c < B;
-        if (col && q == 0) {
-          for (int i = 0; i < c; ++i) X[i * ld + c] = 0.0;
-          X[c * ld + c] = rp[c];
-        }
-        __syncwarp();
-        for (int i = c0 + 1; i < B; ++i) {
-          double s0 = 0.0, s1 = 0.0;
-          if (col && i > c) {
-            int l2 = c + q;
-            for (; l2 + 4 < i; l2 += 8) {
-              s0 = fma(A[i * ld + l2], X[l2 * ld + c], s0);
-              s1 = fma(A[i * ld + l2 + 4], X[(l2 + 4) * ld + c], s1);
-            }
-            if (l2 < i) s0 = fma(A[i * ld + l2], X[l2 * ld + c], s0);
-          }
-          double sacc = s0 + s1;
-          sacc += __shfl_xor_sync(0xffffffffu, sacc, 1);
-          sacc += __shfl_xor_sync(0xffffffffu, sacc, 2);
-          if (col && i > c && q == 0) X[i * ld + c] = -sacc * rp[i];
-          __syncwarp();
-        }
-      }
-    }
-    __syncthreads();
-    for (int t = tid; t < B * B; t += 256) {
-      const int i = t / B, j = t % B;
-      Dk[t] = X[i * ld + j];                  // Dinv
-      Dk[(size_t)B * B + t] = X[j * ld + i];  // Dinv^T
-    }
-    if (k + 1 < nb) {
-      double* Dn = bh + (size_t)(k + 1) * 4 * B * B;
-      cp_async_wait_all();
-      __syncthreads();  // P1 (and P0) landed for every thread
-      // E = A_{k+1,k} X^T (X is zero above its diagonal)
-      double acc[NA][NA];
-#pragma unroll
-      for (int a = 0; a < NA; ++a)
-#pragma unroll
-        for (int b = 0; b < NA; ++b) acc[a][b] = 0.0;
-#pragma unroll 4
-      for (int l = 0; l < B; ++l) {
-        double ai[NA], xj[NA];
-#pragma unroll
-        for (int a = 0; a < NA; ++a) ai[a] = P1[(ty + 16 * a) * B + l];
-#pragma unroll
-        for (int b = 0; b < NA; ++b) xj[b] = X[(tx + 16 * b) * ld + l];
-#pragma unroll
-        for (int a = 0; a < NA; ++a)
-#pragma unroll
-          for (int b = 0; b < NA; ++b) acc[a][b] = fma(ai[a], xj[b], acc[a][b]);
-      }
-#pragma unroll
-      for (int a = 0; a < NA; ++a)
-#pragma unroll
-        for (int b = 0; b < NA; ++b) {
-          const int i = ty + 16 * a, j = tx + 16 * b;
-          Y[i * ld + j] = acc[a][b];
-          Dn[(size_t)2 * B * B + i * B + j] = acc[a][b];  // E
-        }
-      __syncthreads();
-      for (int t = tid; t < B * B; t += 256) Dn[(size_t)3 * B * B + t] = Y[(t % B) * ld + t / B];  // E^T
-    }
-  }
-  if (tid == 0 && bad) atomicOr(status, 1);
-}
-
 }  // namespace stt
 
 using namespace stt;
@@ -1330,213 +1079,7 @@ static int build_levels(stt_hier* h, const double* rho, long long rho_rs, const 
   return STT_OK;
 }
 
-// The explicit inverse of the coarsest matrix from its block-bidiagonal Cholesky factor
-// (for the FP32 cycle, whose coarse solve is then one GEMV instead of 2 nb dependent
-// block steps).  CTA (kc, h) solves A X = I for the B columns of block kc: forward
-// Y_k = Dinv_k (I_k - E_k Y_{k-1}) from block kc on (Y is zero above it), then backward
-// X_k = Dinv_k^T (Y_k - E_{k+1}^T X_{k+1}); Y is parked in the output rows it precedes.
-// Same arithmetic as coarse_solve_kernel, so the GEMV's result matches the block solve
-// to the conditioning of the coarse matrix.  B <= 64 (three B x B FP64 tiles in shared
-// memory).
-__global__ void __launch_bounds__(256) coarse_inverse_kernel(const double* __restrict__ blocks, int B, int nb,
-                                                             double* __restrict__ inv) {
-  extern __shared__ double sm[];
-  double* Y = sm;              // the current block of the solution, B x B (row-major)
-  double* R = Y + B * B;       // right-hand side of the step
-  double* M = R + B * B;       // the step's matrix
-  const int kc = blockIdx.x, h = blockIdx.y;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const long long np = (long long)nb * B;
-  const double* bh = blocks + (size_t)h * nb * 4 * B * B;
-  double* ih = inv + (size_t)h * np * np;
-  auto load = [&](const double* src, double* dst) {
-    for (int t = tid; t < B * B; t += nt) dst[t] = src[t];
-  };
-  // dst = A src (all B x B); A from shared memory
-  auto mm = [&](const double* A, const double* src, double* dst, double sign) {
-    for (int t = tid; t < B * B; t += nt) {
-      const int i = t / B, j = t % B;
-      double acc = 0.0;
-      for (int l = 0; l < B; ++l) acc = fma(A[i * B + l], src[l * B + j], acc);
-      dst[t] = sign * acc;
-    }
-  };
-  auto park = [&](int k, const double* src) {  // rows of block k, columns of block kc
-    for (int t = tid; t < B * B; t += nt) {
-      const int i = t / B, j = t % B;
-      ih[((size_t)k * B + i) * np + (size_t)kc * B + j] = src[t];
-    }
-  };
-  // forward
-  for (int k = kc; k < nb; ++k) {
-    if (k == kc) {
-      for (int t = tid; t < B * B; t += nt) R[t] = (t / B == t % B) ? 1.0 : 0.0;
-    } else {
-      load(bh + ((size_t)k * 4 + 2) * B * B, M);  // E_k
-      __syncthreads();
-      mm(M, Y, R, -1.0);
-    }
-    __syncthreads();
-    load(bh + ((size_t)k * 4 + 0) * B * B, M);  // Dinv_k
-    __syncthreads();
-    mm(M, R, Y, 1.0);
-    __syncthreads();
-    park(k, Y);
-    __syncthreads();
-  }
-  // backward (Y holds X_{k+1} after each step)
-  for (int k = nb - 1; k >= 0; --k) {
-    for (int t = tid; t < B * B; t += nt) {
-      const int i = t / B, j = t % B;
-      R[t] = k >= kc ? ih[((size_t)k * B + i) * np + (size_t)kc * B + j] : 0.0;
-    }
-    if (k < nb - 1) {
-      __syncthreads();
-      load(bh + ((size_t)(k + 1) * 4 + 3) * B * B, M);  // E_{k+1}^T
-      __syncthreads();
-      for (int t = tid; t < B * B; t += nt) {
-        const int i = t / B, j = t % B;
-        double acc = 0.0;
-        for (int l = 0; l < B; ++l) acc = fma(M[i * B + l], Y[l * B + j], acc);
-        R[t] -= acc;
-      }
-    }
-    __syncthreads();
-    load(bh + ((size_t)k * 4 + 1) * B * B, M);  // Dinv_k^T
-    __syncthreads();
-    mm(M, R, Y, 1.0);
-    __syncthreads();
-    park(k, Y);
-    __syncthreads();
-  }
-}
-
-// coarse_inverse_kernel for B = 16 NA (NA = 2, 4) with register-tiled products (thread
-// (ty, tx) owns entries (ty + 16 a, tx + 16 b), as band_factor_tiled_kernel), computing only
-// the block rows k >= kc of column block kc: A^{-1} is symmetric, so coarse_mirror_kernel
-// fills the blocks above the diagonal from their transposes afterwards.
-template <int NA>
-__global__ void __launch_bounds__(256) coarse_inverse_tiled_kernel(const double* __restrict__ blocks, int nb,
-                                                                   double* __restrict__ inv) {
-  constexpr int B = 16 * NA, ld = B + 1;
-  extern __shared__ double sm[];
-  double* Y = sm;           // the current block of the solution (ld)
-  double* R = Y + B * ld;   // right-hand side of the step
-  double* M = R + B * ld;   // the step's matrix
-  const int kc = blockIdx.x, h = blockIdx.y;
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-  const long long np = (long long)nb * B;
-  const double* bh = blocks + (size_t)h * nb * 4 * B * B;
-  double* ih = inv + (size_t)h * np * np;
-  auto load = [&](const double* src, double* dst) {
-    for (int t = tid; t < B * B; t += 256) dst[(t / B) * ld + t % B] = src[t];
-  };
-  // acc = A src over this thread's tile
-  auto mm = [&](const double* A, const double* src, double (&acc)[NA][NA]) {
-#pragma unroll
-    for (int a = 0; a < NA; ++a)
-#pragma unroll
-      for (int b = 0; b < NA; ++b) acc[a][b] = 0.0;
-#pragma unroll 4
-    for (int l = 0; l < B; ++l) {
-      double ai[NA], sj[NA];
-#pragma unroll
-      for (int a = 0; a < NA; ++a) ai[a] = A[(ty + 16 * a) * ld + l];
-#pragma unroll
-      for (int b = 0; b < NA; ++b) sj[b] = src[l * ld + tx + 16 * b];
-#pragma unroll
-      for (int a = 0; a < NA; ++a)
-#pragma unroll
-        for (int b = 0; b < NA; ++b) acc[a][b] = fma(ai[a], sj[b], acc[a][b]);
-    }
-  };
-  auto park_ptr = [&](int k, int i, int j) { return ih + ((size_t)k * B + i) * np + (size_t)kc * B + j; };
-  double acc[NA][NA];
-  // forward: Y_k = Dinv_k (I_k - E_k Y_{k-1}), k = kc .. nb - 1
-  for (int k = kc; k < nb; ++k) {
-    if (k == kc) {
-      for (int t = tid; t < B * B; t += 256) R[(t / B) * ld + t % B] = (t / B == t % B) ? 1.0 : 0.0;
-    } else {
-      load(bh + ((size_t)k * 4 + 2) * B * B, M);  // E_k
-      __syncthreads();
-      mm(M, Y, acc);
-#pragma unroll
-      for (int a = 0; a < NA; ++a)
-#pragma unroll
-        for (int b = 0; b < NA; ++b) R[(ty + 16 * a) * ld + tx + 16 * b] = -acc[a][b];
-    }
-    __syncthreads();
-    load(bh + ((size_t)k * 4 + 0) * B * B, M);  // Dinv_k
-    __syncthreads();
-    mm(M, R, acc);
-    __syncthreads();  // everyone has read Y (the E_k product) and R
-#pragma unroll
-    for (int a = 0; a < NA; ++a)
-#pragma unroll
-      for (int b = 0; b < NA; ++b) {
-        const int i = ty + 16 * a, j = tx + 16 * b;
-        Y[i * ld + j] = acc[a][b];
-        *park_ptr(k, i, j) = acc[a][b];
-      }
-    __syncthreads();
-  }
-  // backward: X_k = Dinv_k^T (Y_k - E_{k+1}^T X_{k+1}), k = nb - 1 .. kc (Y holds X_{k+1})
-  for (int k = nb - 1; k >= kc; --k) {
-    double rv[NA][NA];
-#pragma unroll
-    for (int a = 0; a < NA; ++a)
-#pragma unroll
-      for (int b = 0; b < NA; ++b) rv[a][b] = *park_ptr(k, ty + 16 * a, tx + 16 * b);
-    if (k < nb - 1) {
-      load(bh + ((size_t)(k + 1) * 4 + 3) * B * B, M);  // E_{k+1}^T
-      __syncthreads();
-      mm(M, Y, acc);
-#pragma unroll
-      for (int a = 0; a < NA; ++a)
-#pragma unroll
-        for (int b = 0; b < NA; ++b) rv[a][b] -= acc[a][b];
-    }
-#pragma unroll
-    for (int a = 0; a < NA; ++a)
-#pragma unroll
-      for (int b = 0; b < NA; ++b) R[(ty + 16 * a) * ld + tx + 16 * b] = rv[a][b];
-    __syncthreads();
-    load(bh + ((size_t)k * 4 + 1) * B * B, M);  // Dinv_k^T
-    __syncthreads();
-    mm(M, R, acc);
-    __syncthreads();
-#pragma unroll
-    for (int a = 0; a < NA; ++a)
-#pragma unroll
-      for (int b = 0; b < NA; ++b) {
-        const int i = ty + 16 * a, j = tx + 16 * b;
-        Y[i * ld + j] = acc[a][b];
-        *park_ptr(k, i, j) = acc[a][b];
-      }
-    __syncthreads();
-  }
-}
-
-// inv[r][c] = inv[c][r] for the block rows above the diagonal block (row block < column
-// block), a 32 x 32 tile through shared memory per CTA (reads and writes coalesced).
-// Grid: (np / 32, np / 32, rows); tiles wholly below the block diagonal return at once.
-__global__ void __launch_bounds__(256) coarse_mirror_kernel(double* __restrict__ inv, int B, long long np) {
-  __shared__ double tile[32][33];
-  const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;  // destination tile (rows r0.., cols c0..)
-  if (r0 / B >= (c0 + 31) / B) return;                    // no destination entry above the block diagonal
-  double* ih = inv + (size_t)blockIdx.z * np * np;
-  for (int j = threadIdx.y; j < 32; j += 8) {  // source rows c0 + j, columns r0 + threadIdx.x
-    const long long sr = c0 + j, sc = r0 + threadIdx.x;
-    tile[j][threadIdx.x] = (sr < np && sc < np) ? ih[sr * np + sc] : 0.0;
-  }
-  __syncthreads();
-  for (int i = threadIdx.y; i < 32; i += 8) {
-    const long long r = r0 + i, c = c0 + threadIdx.x;
-    if (r < np && c < np && r / B < c / B) ih[r * np + c] = tile[threadIdx.x][i];
-  }
-}
-
-// The dynamic shared-memory ceiling of the coarse kernels, raised once per device to the// The dynamic shared-memory ceiling of the coarse kernels, raised once per device to the
+// The dynamic shared-memory ceiling of the banded factorisation, raised once per device to the
 // device's opt-in maximum.  (Setting it per call to the call's own size raced between
 // host threads building hierarchies of different block sizes: a launch could meet
 // another thread's smaller ceiling and fail.)
@@ -1558,11 +1101,6 @@ static int allow_large_smem() {
                                            max_optin - (int)fa.sharedSizeBytes), "smem attr");
   };
   STT_TRY(raise_to((const void*)band_factor_kernel));
-  STT_TRY(raise_to((const void*)band_factor_tiled_kernel<2>));
-  STT_TRY(raise_to((const void*)band_factor_tiled_kernel<4>));
-  STT_TRY(raise_to((const void*)coarse_inverse_kernel));
-  STT_TRY(raise_to((const void*)coarse_inverse_tiled_kernel<2>));
-  STT_TRY(raise_to((const void*)coarse_inverse_tiled_kernel<4>));
   if (dev >= 0 && dev < 64) done[dev] = true;
   return STT_OK;
 }
@@ -1585,7 +1123,6 @@ static int acquire_sync(CoarseSync** out) {
         g_sync_free.erase(g_sync_free.begin() + (long)i);
         s->refs.store(1);
         s->l1_pending.store(0);
-        s->first_cycle.store(0);
         *out = s;
         return STT_OK;
       }
@@ -1597,9 +1134,7 @@ static int acquire_sync(CoarseSync** out) {
   if (rc == STT_OK) rc = check_cuda(cudaStreamCreateWithPriority(&s->side, cudaStreamNonBlocking, hi), "side stream");
   if (rc == STT_OK) rc = check_cuda(cudaEventCreateWithFlags(&s->built, cudaEventDisableTiming), "event");
   if (rc == STT_OK) rc = check_cuda(cudaEventCreateWithFlags(&s->ready, cudaEventDisableTiming), "event");
-  if (rc == STT_OK) rc = check_cuda(cudaEventCreateWithFlags(&s->factored, cudaEventDisableTiming), "event");
   if (rc != STT_OK) {
-    if (s->factored) cudaEventDestroy(s->factored);
     if (s->ready) cudaEventDestroy(s->ready);
     if (s->built) cudaEventDestroy(s->built);
     if (s->side) cudaStreamDestroy(s->side);
@@ -1624,6 +1159,7 @@ static int build_coarse(stt_hier* h, cudaStream_t st) {
   CoarseDesc& co = h->co;
   const LevelDesc& cl = h->lv[h->nlevels - 1];
   const int H = h->hrows;
+  if (co.tree) return coarse_factor(h, st);
   const long long per = (long long)co.nb * 4 * co.B * co.B;
   STT_TRY(check_cuda(cudaMemsetAsync(co.blocks, 0, 8 * H * per, st), "memset coarse"));
   const long long threads = cl.nnode + ((long long)co.nb * co.B - cl.ndof);
@@ -1632,32 +1168,8 @@ static int build_coarse(stt_hier* h, cudaStream_t st) {
   STT_TRY(check_launch("band assemble"));
   const size_t smem = (size_t)3 * co.B * (co.B + 1) * sizeof(double);
   STT_TRY(allow_large_smem());
-  const size_t tsmem = smem + (size_t)2 * co.B * co.B * sizeof(double);  // + two staging blocks
-  if (co.B == 32)
-    band_factor_tiled_kernel<2><<<H, 256, tsmem, st>>>(co.blocks, co.nb, h->status);
-  else if (co.B == 64)
-    band_factor_tiled_kernel<4><<<H, 256, tsmem, st>>>(co.blocks, co.nb, h->status);
-  else
-    band_factor_kernel<<<H, 256, smem, st>>>(co.blocks, co.B, co.nb, h->status);
-  STT_TRY(check_launch("band factor"));
-  STT_TRY(check_cuda(cudaEventRecord(h->sync->factored, st), "record factor"));
-  if (co.inv) {
-    if (co.B == 32 || co.B == 64) {
-      const size_t tsm = (size_t)3 * co.B * (co.B + 1) * sizeof(double);
-      if (co.B == 32)
-        coarse_inverse_tiled_kernel<2><<<dim3(co.nb, H), 256, tsm, st>>>(co.blocks, co.nb, co.inv);
-      else
-        coarse_inverse_tiled_kernel<4><<<dim3(co.nb, H), 256, tsm, st>>>(co.blocks, co.nb, co.inv);
-      const long long np = (long long)co.nb * co.B;
-      const unsigned nt = (unsigned)((np + 31) / 32);
-      coarse_mirror_kernel<<<dim3(nt, nt, H), dim3(32, 8), 0, st>>>(co.inv, co.B, np);
-    } else {
-      const size_t ism = (size_t)3 * co.B * co.B * sizeof(double);
-      coarse_inverse_kernel<<<dim3(co.nb, H), 256, ism, st>>>(co.blocks, co.B, co.nb, co.inv);
-    }
-    STT_TRY(check_launch("coarse inverse"));
-  }
-  return STT_OK;
+  band_factor_kernel<<<H, 256, smem, st>>>(co.blocks, co.B, co.nb, h->status);
+  return check_launch("band factor");
 }
 
 extern "C" int stt_hier_create(stt_hier** out, void* workspace, long long ws_bytes, int d, int nelx,
@@ -1700,7 +1212,6 @@ extern "C" int stt_hier_create(stt_hier** out, void* workspace, long long ws_byt
   if (rc == STT_OK) rc = check_cuda(cudaStreamWaitEvent(h->sync->side, h->sync->built, 0), "side wait");
   if (rc == STT_OK) rc = d == 2 ? build_coarse<2>(h, h->sync->side) : build_coarse<1>(h, h->sync->side);
   if (rc == STT_OK) rc = check_cuda(cudaEventRecord(h->sync->ready, h->sync->side), "record coarse");
-  if (rc == STT_OK) h->sync->first_cycle.store(h->co.inv ? 1 : 0);
   // level 1's stencil (deferred by build_levels) beside the factorisation; an FP32
   // hierarchy swept from the densities only its FP32 diagonal, the FP64 stencil on first use
   if (rc == STT_OK && h->nlevels > 2) {

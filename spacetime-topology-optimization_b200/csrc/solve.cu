@@ -12,6 +12,7 @@
 #include <mutex>
 #include <vector>
 
+#include "coarse.h"
 #include "errors.h"
 #include "hier.h"
 #include "mg.cuh"
@@ -88,7 +89,7 @@ struct SolveWS {
   void* b[kMaxLevels];
   void* acc[kMaxLevels];       // gamma > 1 only
   void* rhs2[kMaxLevels];
-  double* cscratch;            // [nrows][nb * B]
+  double* cscratch;            // [nrows][nb * B] (banded coarse solves)
   int nblk_max;
   long long bytes;
 };
@@ -135,7 +136,7 @@ static long long plan_solve(const stt_hier* h, int nrows, int gamma, char* base,
       w.rhs2[l] = carve(base, used, (long long)es * nrows * nd);
     }
   }
-  w.cscratch = (double*)carve(base, used, 8LL * nrows * h->co.nb * h->co.B);
+  if (!h->co.tree) w.cscratch = (double*)carve(base, used, 8LL * nrows * h->co.nb * h->co.B);
   w.bytes = used;
   return used;
 }
@@ -154,8 +155,7 @@ struct Cycle {
   KEq<D, T> ke;
   MQ<T> mq;
   T* final_out = nullptr;  // where level 0's last sweep writes (row stride vstride(ndof0))
-  bool waited_factor = false;  // the stream has waited for the coarse factorisation
-  bool waited_ready = false;   // ... and for the explicit inverse
+  bool waited_ready = false;  // the stream has waited for the coarse factorisation
   RzFuse<T> rzf{};         // the PCG's dots for level 0's chained passes to take (rzf.rst set)
   bool mix_done = false;   // the pre-smoothing pass took r . z_old
   bool rz_done = false;    // the post-smoothing pass took r . z and set beta
@@ -272,28 +272,16 @@ struct Cycle {
     }
   }
 
-  // The factorisation (and an FP32 hierarchy's explicit inverse after it) runs on the
-  // hierarchy's side stream.  The first coarse solve on a fresh FP32 hierarchy takes the
-  // block solves, which need only the factor, so the first cycle does not wait for the
-  // inverse; every later one takes the inverse's GEMV (equal to FP64 rounding).
+  // The coarsest level's solve; the factorisation runs on the hierarchy's side stream.
   void coarse(int l, const T* b, T* x) {
     const LevelDesc& lv = h->lv[l];
     const CoarseDesc& co = h->co;
-    bool use_inv = sizeof(T) == 4 && co.inv;
-    if (use_inv && h->sync->first_cycle.load() && h->sync->first_cycle.exchange(0) == 1) use_inv = false;
-    if (use_inv && !waited_ready) {
+    if (!waited_ready) {
       cudaStreamWaitEvent(st, h->sync->ready, 0);
-      waited_ready = waited_factor = true;
-    } else if (!use_inv && !waited_factor) {
-      cudaStreamWaitEvent(st, h->sync->factored, 0);
-      waited_factor = true;
+      waited_ready = true;
     }
-    if (use_inv) {
-      const int np = co.nb * co.B;
-      coarse_inv_solve_kernel<D, T><<<dim3((np + kInvRowsPerCta - 1) / kInvRowsPerCta, nrows), 256,
-                                      sizeof(double) * np, st>>>(b, x, vstride(lv.ndof), co.inv, np, co.by_col,
-                                                                 lv.nnx, lv.nny, lv.fixed, h->row_map, h->hrows,
-                                                                 rst);
+    if (co.tree) {
+      coarse_tree_solve<T>(h, nrows, b, x, vstride(lv.ndof), rst, st);
       return;
     }
 #define STT_COARSE(NC)                                                                          \

@@ -25,8 +25,10 @@ namespace stt {
 
 namespace cg = cooperative_groups;
 
-constexpr int kTreeCluster = 8;         // CTAs a row
-constexpr int kTreeMaxUnknowns = 5376;  // nb * B, held five times over in a CTA's shared memory
+constexpr int kTreeCluster = 8;                    // CTAs a row
+constexpr int kTreeGroups = 2;                     // thread groups of 4 B threads a CTA
+constexpr int kTreeAll = kTreeCluster * kTreeGroups;
+constexpr int kTreeMaxUnknowns = 5376;   // nb * B, held in every CTA's shared memory
 constexpr size_t kTreeSmem = 225 << 10;  // dynamic shared memory a CTA of the solve may take
 
 // One 8 x 8 tile product on the FP64 tensor cores (tcgen05 has no FP64 kind): lane
@@ -348,17 +350,6 @@ __global__ void __cluster_dims__(kTreeCluster, 1, 1) __launch_bounds__(256)
 // ---- solve ---------------------------------------------------------------------------
 
 template <int NB>
-struct TreeSolve {
-  static constexpr int B = 8 * NB, NC = 2 * NB;   // a group of 4 B threads, NC columns (rows) a thread
-  static constexpr int kGroups = NB <= 5 ? 2 : 1;  // groups a CTA
-  static constexpr int kThreads = kGroups * 4 * B;
-  static constexpr int kAll = kGroups * kTreeCluster;
-  static constexpr int kScratch = 10 * B;          // doubles of group scratch
-  static size_t vectors(int nb) { return sizeof(double) * (5 * (size_t)nb * B + kGroups * kScratch); }
-  static constexpr size_t kTask = sizeof(double) * 3 * B * B;  // X, F_l, F_r of one block
-};
-
-template <int NB>
 STT_DEV void group_sync(int grp) {
   asm volatile("bar.sync %0, %1;" ::"r"(grp + 1), "r"(32 * NB) : "memory");
 }
@@ -366,6 +357,15 @@ STT_DEV void tree_cp16(void* smem, const void* gmem) {
   const unsigned a = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(a), "l"(gmem));
 }
+
+// Shared memory of a CTA (doubles): the solution in block order, then for each group its
+// blocks' right-hand sides, the updates that arrive for them and scratch, then the staged
+// matrices.
+__host__ __device__ inline int tree_own(int nb) { return (nb + kTreeAll - 1) / kTreeAll; }  // blocks a group
+__host__ __device__ inline size_t tree_vectors(int nb, int B) {
+  return (size_t)nb * B + kTreeGroups * (5 * (size_t)tree_own(nb) * B + 10 * B);
+}
+__host__ __device__ inline size_t tree_task(int B) { return 3 * (size_t)B * B; }  // X, F_l, F_r of one block
 
 // One row's solve on a cluster: 2 log2(nb) steps, each a group of 4 B threads' two dependent
 // block products.  Bound by the steps' latency, so the blocks (constant over the solve) are
@@ -380,57 +380,85 @@ STT_DEV void tree_cp16(void* smem, const void* gmem) {
 // neighbours' updates arrive there by remote stores into a buffer a side (two sets, used by
 // alternate strides, so that a set is read before it is written again) and are added by the
 // owner in a fixed order; a solution block is written to all eight CTAs.
-template <int NB, int D, typename T>
-__global__ void __cluster_dims__(kTreeCluster, 1, 1) __launch_bounds__(TreeSolve<NB>::kThreads)
-    tree_solve_kernel(const T* __restrict__ b, T* __restrict__ x, long long rs, const double* __restrict__ blocks,
-                      int nb, int staged, int by_col, int nnx, int nny, const uint8_t* __restrict__ fixed,
-                      const int* __restrict__ row_map, int hrows, const RowState* __restrict__ rst) {
-  using TS = TreeSolve<NB>;
-  constexpr int B = TS::B, NC = TS::NC, BB = B * B, kGroup = 4 * B;
-  extern __shared__ __align__(16) double sm[];
-  const int srow = blockIdx.y;
-  if (rst && !rst[srow].active) return;  // the whole cluster
-  cg::cluster_group cluster = cg::this_cluster();
-  const int rank = (int)cluster.block_rank();
-  const int np = nb * B, tid = threadIdx.x;
-  const int grp = tid / kGroup, t = tid - grp * kGroup, gi = rank * TS::kGroups + grp;
-  double* vb = sm;      // right-hand sides, then y (own blocks)
-  double* in = vb + np;  // [set][side]: updates from the left (0) and right (1) neighbours
-  double* vx = in;       // solution blocks (the updates are all read by then)
-  double* tv = vb + 5 * (size_t)np + grp * TS::kScratch;  // this group's scratch
-  double* part = tv + 2 * B;
-  double* stage = vb + 5 * (size_t)np + TS::kGroups * TS::kScratch + (size_t)grp * staged * 3 * BB;
-  const double* bh = blocks + (size_t)hier_row(row_map, hrows, srow) * nb * 4 * BB;
-  const T* bs = b + (size_t)srow * rs;
-  T* xs = x + (size_t)srow * rs;
-  const int used = D * (by_col ? nny : nnx);
-  auto dof_of = [&](int k, int ii, long long& node, int& d) {
-    const int pos = ii / D;
-    d = ii - pos * D;
-    node = by_col ? (long long)pos * nnx + k : (long long)k * nnx + pos;
-  };
+template <int NB>
+struct TreeRow {
+  static constexpr int B = 8 * NB, NC = 2 * NB, BB = B * B, kGroup = 4 * B;
+  static constexpr int kThreads = kTreeGroups * kGroup;
+
+  const double* bh;  // the row's factor [nb][4][B][B]
+  int nb, staged, own, levels, rank, grp, t, gi;
+  double *vx, *vb, *in, *tv, *part, *stage;
+
+  STT_DEV void init(double* sm, const double* factor, int nblocks, int nstaged) {
+    cg::cluster_group cluster = cg::this_cluster();
+    bh = factor;
+    nb = nblocks;
+    staged = nstaged;
+    own = tree_own(nb);
+    levels = 0;
+    while ((1 << levels) < nb) ++levels;
+    rank = (int)cluster.block_rank();
+    grp = (int)threadIdx.x / kGroup;
+    t = (int)threadIdx.x - grp * kGroup;
+    gi = rank * kTreeGroups + grp;
+    vx = sm;
+    vb = vx + (size_t)nb * B;                       // [grp][own][B]: right-hand sides, then y
+    in = vb + (size_t)kTreeGroups * own * B;        // [set][side][grp][own][B]
+    tv = in + (size_t)4 * kTreeGroups * own * B + grp * 10 * B;
+    part = tv + 2 * B;
+    stage = vx + tree_vectors(nb, B) + (size_t)grp * staged * 3 * BB;
+  }
+
   // blocks in the order of elimination: those of stride 2^l are numbers base(l) .. base(l + 1),
-  // the root (block 0) is the last; number o belongs to group o % kAll
-  auto base = [&](int l) { return nb - ((nb + (1 << l) - 1) >> l); };
-  auto number = [&](int e) {
+  // the root (block 0) is the last; number o is the o / kTreeAll-th block of group o % kTreeAll
+  STT_DEV int base(int l) const { return nb - ((nb + (1 << l) - 1) >> l); }
+  STT_DEV int number(int e) const {
     if (e == 0) return nb - 1;
     const int l = __ffs(e) - 1;
     return base(l) + (e >> (l + 1));
-  };
-  auto owner = [&](int e) { return (number(e) % TS::kAll) / TS::kGroups; };
-  auto block_of = [&](int o, int l) { return (1 << l) * (2 * (o - base(l)) + 1); };
-  int levels = 0;
-  while ((1 << levels) < nb) ++levels;
+  }
+  STT_DEV int block_of(int o, int l) const { return (1 << l) * (2 * (o - base(l)) + 1); }
+  // where block e's vectors live: the CTA, and the offset in an array [grp][own][B]
+  STT_DEV int owner(int e) const { return (number(e) % kTreeAll) / kTreeGroups; }
+  STT_DEV int place(int e) const {
+    const int o = number(e);
+    return ((o % kTreeGroups) * own + o / kTreeAll) * B;
+  }
+  STT_DEV double* updates(int set, int side) const { return in + (size_t)((2 * set + side) * kTreeGroups) * own * B; }
+  // calls f(block, j) for the group's blocks in their order, j = 0, 1, ...
+  template <typename F>
+  STT_DEV void each_block(F f) const {
+    int l = 0, j = 0;
+    for (int o = gi; o < nb; o += kTreeAll, ++j) {
+      while (l < levels && o >= base(l + 1)) ++l;
+      f(o == nb - 1 ? 0 : block_of(o, l), j, l);
+    }
+  }
 
-  const int i4 = t >> 2, q = t & 3;  // row-wise products: row i4, column pairs q, q + 4, ...
-  const int j4 = t % B, p4 = t / B;  // column-wise: column j4, quarter p4 of its rows
+  // starts fetching the blocks (the first in a copy group of its own)
+  STT_DEV void prefetch() {
+    each_block([&](int i, int j, int l) {
+      if (j < staged) {
+        double* dst = stage + (size_t)j * 3 * BB;
+        const double* src = bh + (size_t)i * 4 * BB;
+        const int n01 = i == 0 ? BB : 2 * BB;  // X and F_l lie side by side
+        for (int c = 2 * t; c < n01; c += 2 * kGroup) tree_cp16(dst + c, src + c);
+        if (i != 0 && i + (1 << l) < nb)
+          for (int c = 2 * t; c < BB; c += 2 * kGroup) tree_cp16(dst + 2 * BB + c, src + 3 * BB + c);
+      }
+      if (j == 0) asm volatile("cp.async.commit_group;\n" ::);
+    });
+    asm volatile("cp.async.commit_group;\n" ::);
+  }
+
   // the matrices (k = 0: X, 1: F_l, 2: F_r) of the group's j-th block, i
-  auto matrix = [&](int j, int i, int k) -> const double* {
+  STT_DEV const double* matrix(int j, int i, int k) const {
     return j < staged ? stage + ((size_t)j * 3 + k) * BB : bh + ((size_t)i * 4 + (k == 2 ? 3 : k)) * BB;
-  };
-  // row-wise product, summed over the quad; column-wise partial product of a quarter
-  auto row_dot = [&](const double* M, const double* v) {
-    const double2* m = reinterpret_cast<const double2*>(M + (size_t)i4 * B) + q;
+  }
+  // row-wise product: row t / 4, column pairs t % 4, t % 4 + 4, ...; summed over the quad
+  STT_DEV double row_dot(const double* M, const double* v) const {
+    const int q = t & 3;
+    const double2* m = reinterpret_cast<const double2*>(M + (size_t)(t >> 2) * B) + q;
     const double2* w = reinterpret_cast<const double2*>(v) + q;
     double s0 = 0.0, s1 = 0.0;
 #pragma unroll
@@ -440,13 +468,15 @@ __global__ void __cluster_dims__(kTreeCluster, 1, 1) __launch_bounds__(TreeSolve
       s1 = fma(mm.y, ww.y, s1);
     }
     return s0 + s1;
-  };
-  auto quad = [&](double s) {
+  }
+  STT_DEV static double quad(double s) {
     s += __shfl_xor_sync(0xffffffffu, s, 1);
     s += __shfl_xor_sync(0xffffffffu, s, 2);
     return s;
-  };
-  auto col_dot = [&](const double* M, const double* v) {
+  }
+  // column-wise partial product: column t % B, quarter t / B of the rows
+  STT_DEV double col_dot(const double* M, const double* v) const {
+    const int p4 = t / B, j4 = t - p4 * B;
     const double* m = M + (size_t)(p4 * NC) * B + j4;
     const double2* w = reinterpret_cast<const double2*>(v + p4 * NC);
     double s0 = 0.0, s1 = 0.0;
@@ -457,131 +487,149 @@ __global__ void __cluster_dims__(kTreeCluster, 1, 1) __launch_bounds__(TreeSolve
       s1 = fma(m[(2 * c + 1) * B], ww.y, s1);
     }
     return s0 + s1;
-  };
-  auto parts = [&](const double* pp, int j) { return (pp[j] + pp[B + j]) + (pp[2 * B + j] + pp[3 * B + j]); };
+  }
+  STT_DEV static double parts(const double* pp, int j) { return (pp[j] + pp[B + j]) + (pp[2 * B + j] + pp[3 * B + j]); }
 
-  // stage the blocks (the first in a copy group of its own) and read the right-hand sides
-  {
-    int l = 0, j = 0;
-    for (int o = gi; o < nb; o += TS::kAll, ++j) {
-      while (l < levels && o >= base(l + 1)) ++l;
-      const int i = o == nb - 1 ? 0 : block_of(o, l);
-      if (j < staged) {
-        double* dst = stage + (size_t)j * 3 * BB;
-        const double* src = bh + (size_t)i * 4 * BB;
-        const int n01 = i == 0 ? BB : 2 * BB;  // X and F_l lie side by side
-        for (int c = 2 * t; c < n01; c += 2 * kGroup) tree_cp16(dst + c, src + c);
-        if (i != 0 && i + (1 << l) < nb)
-          for (int c = 2 * t; c < BB; c += 2 * kGroup) tree_cp16(dst + 2 * BB + c, src + 3 * BB + c);
+  // Solves for the right-hand sides in vb (complete and visible: the caller synchronises the
+  // cluster first); publish(i, t, v) is called by the owner for each unknown t of block i.
+  template <typename Publish>
+  STT_DEV void solve(Publish publish) {
+    cg::cluster_group cluster = cg::this_cluster();
+    int o = gi, j = 0;  // the group's next block
+    bool landed = false;
+    auto wait_stage = [&](bool first) {
+      if (landed) return;
+      if (first) asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+      else asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+      landed = !first;
+    };
+    const int q = t & 3, i4 = t >> 2;
+    const size_t go = (size_t)grp * own * B;
+    double* vg = vb + go;
+    for (int l = 0; l < levels; ++l) {
+      const int s = 1 << l, end = base(l + 1);
+      double* inL = updates(l & 1, 0);
+      double* inR = updates(l & 1, 1);
+      for (; o < end; o += kTreeAll, ++j) {
+        const int i = block_of(o, l);
+        const bool right = i + s < nb;
+        wait_stage(j == 0);
+        if (t < B) tv[t] = vg[j * B + t];
+        group_sync<NB>(grp);
+        const double y = quad(row_dot(matrix(j, i, 0), tv));
+        if (q == 0) {
+          tv[B + i4] = y;
+          vg[j * B + i4] = y;
+        }
+        group_sync<NB>(grp);
+        part[t] = col_dot(matrix(j, i, 1), tv + B);
+        if (right) part[4 * B + t] = col_dot(matrix(j, i, 2), tv + B);
+        group_sync<NB>(grp);
+        if (t < B)
+          cluster.map_shared_rank(inR, owner(i - s))[place(i - s) + t] = parts(part, t);
+        else if (t < 2 * B && right)
+          cluster.map_shared_rank(inL, owner(i + s))[place(i + s) + (t - B)] = parts(part + 4 * B, t - B);
+        group_sync<NB>(grp);
       }
-      if (j == 0) asm volatile("cp.async.commit_group;\n" ::);
+      cluster.sync();
+      // the updates of the own blocks that are left
       if (t < B) {
-        double v = 0.0;
-        if (t < used) {
-          long long node;
-          int d;
-          dof_of(i, t, node, d);
-          v = (double)bs[node * D + d];
-        }
-        vb[i * B + t] = v;
-      }
-    }
-    asm volatile("cp.async.commit_group;\n" ::);
-  }
-  cluster.sync();
-
-  int o = gi, j = 0;  // the group's next block
-  bool landed = false;
-  auto wait_stage = [&](bool first) {
-    if (landed) return;
-    if (first) asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-    else asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    landed = !first;
-  };
-  for (int l = 0; l < levels; ++l) {
-    const int s = 1 << l, end = base(l + 1);
-    double* inL = in + (size_t)(2 * (l & 1)) * np;
-    double* inR = inL + np;
-    for (; o < end; o += TS::kAll, ++j) {
-      const int i = block_of(o, l);
-      const bool right = i + s < nb;
-      wait_stage(j == 0);
-      if (t < B) tv[t] = vb[i * B + t];
-      group_sync<NB>(grp);
-      const double y = quad(row_dot(matrix(j, i, 0), tv));
-      if (q == 0) {
-        tv[B + i4] = y;
-        vb[i * B + i4] = y;
-      }
-      group_sync<NB>(grp);
-      part[p4 * B + j4] = col_dot(matrix(j, i, 1), tv + B);
-      if (right) part[(4 + p4) * B + j4] = col_dot(matrix(j, i, 2), tv + B);
-      group_sync<NB>(grp);
-      if (t < B)
-        cluster.map_shared_rank(inR, owner(i - s))[(i - s) * B + t] = parts(part, t);
-      else if (t < 2 * B && right)
-        cluster.map_shared_rank(inL, owner(i + s))[(i + s) * B + (t - B)] = parts(part + 4 * B, t - B);
-      group_sync<NB>(grp);
-    }
-    cluster.sync();
-    // the updates of the own blocks that are left
-    if (t < B) {
-      int l2 = l + 1;
-      for (int o2 = o; o2 < nb; o2 += TS::kAll) {
-        while (l2 < levels && o2 >= base(l2 + 1)) ++l2;
-        if (o2 == nb - 1) {
-          vb[t] -= inR[t];
-        } else {
-          const int i = block_of(o2, l2);
-          vb[i * B + t] = (vb[i * B + t] - inL[i * B + t]) - (i + s < nb ? inR[i * B + t] : 0.0);
+        int l2 = l + 1, j2 = j;
+        for (int o2 = o; o2 < nb; o2 += kTreeAll, ++j2) {
+          while (l2 < levels && o2 >= base(l2 + 1)) ++l2;
+          const int a = j2 * B + t;
+          if (o2 == nb - 1)
+            vg[a] -= inR[go + a];
+          else
+            vg[a] = (vg[a] - inL[go + a]) - (block_of(o2, l2) + s < nb ? inR[go + a] : 0.0);
         }
       }
     }
-  }
-
-  auto publish = [&](int i, bool share) {  // x_i = X_i^T z from the group's partial sums
-    if (t < B) {
-      const double v = parts(part, t);
-      if (share)
+    auto finish = [&](int i, bool share) {  // x_i = X_i^T z from the group's partial sums
+      if (t < B) {
+        const double v = parts(part, t);
+        if (share)
 #pragma unroll
-        for (int rk = 0; rk < kTreeCluster; ++rk) cluster.map_shared_rank(vx, rk)[i * B + t] = v;
-      if (t < used) {
-        long long node;
-        int d;
-        dof_of(i, t, node, d);
-        xs[node * D + d] = ((fixed[node] >> d) & 1) ? T(0) : T(v);
+          for (int rk = 0; rk < kTreeCluster; ++rk) cluster.map_shared_rank(vx, rk)[i * B + t] = v;
+        publish(i, t, v);
+      }
+    };
+    if (o == nb - 1) {  // the root's group
+      wait_stage(j == 0);
+      if (t < B) tv[t] = vg[j * B + t];
+      group_sync<NB>(grp);
+      const double y = quad(row_dot(matrix(j, 0, 0), tv));
+      if (q == 0) tv[B + i4] = y;
+      group_sync<NB>(grp);
+      part[t] = col_dot(matrix(j, 0, 0), tv + B);
+      group_sync<NB>(grp);
+      finish(0, nb > 1);
+    }
+    o -= kTreeAll;
+    --j;
+    for (int l = levels - 1; l >= 0; --l) {
+      const int s = 1 << l, begin = base(l);
+      cluster.sync();
+      for (; o >= begin; o -= kTreeAll, --j) {
+        const int i = block_of(o, l);
+        group_sync<NB>(grp);
+        double z = row_dot(matrix(j, i, 1), vx + (i - s) * B);
+        if (i + s < nb) z += row_dot(matrix(j, i, 2), vx + (i + s) * B);
+        z = quad(z);
+        if (q == 0) tv[i4] = vg[j * B + i4] - z;
+        group_sync<NB>(grp);
+        part[t] = col_dot(matrix(j, i, 0), tv);
+        group_sync<NB>(grp);
+        finish(i, l > 0);
       }
     }
+  }
+};
+
+// One row's coarse solve on a cluster (TreeRow), between global vectors.
+template <int NB, int D, typename T>
+__global__ void __cluster_dims__(kTreeCluster, 1, 1) __launch_bounds__(TreeRow<NB>::kThreads)
+    tree_solve_kernel(const T* __restrict__ b, T* __restrict__ x, long long rs, const double* __restrict__ blocks,
+                      int nb, int staged, int by_col, int nnx, int nny, const uint8_t* __restrict__ fixed,
+                      const int* __restrict__ row_map, int hrows, const RowState* __restrict__ rst) {
+  constexpr int B = 8 * NB;
+  extern __shared__ __align__(16) double sm[];
+  const int srow = blockIdx.y;
+  TreeRow<NB> tree;
+  tree.init(sm, blocks + (size_t)hier_row(row_map, hrows, srow) * nb * 4 * B * B, nb, staged);
+  tree.prefetch();  // beside the kernel before (the factor is complete when its solves are launched)
+  grid_wait();
+  if (rst && !rst[srow].active) {  // the whole cluster
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    return;
+  }
+  const T* bs = b + (size_t)srow * rs;
+  T* xs = x + (size_t)srow * rs;
+  const int used = D * (by_col ? nny : nnx);
+  auto dof_of = [&](int k, int ii, long long& node, int& d) {
+    const int pos = ii / D;
+    d = ii - pos * D;
+    node = by_col ? (long long)pos * nnx + k : (long long)k * nnx + pos;
   };
-  if (o == nb - 1) {  // the root's group
-    wait_stage(j == 0);
-    if (t < B) tv[t] = vb[t];
-    group_sync<NB>(grp);
-    const double y = quad(row_dot(matrix(j, 0, 0), tv));
-    if (q == 0) tv[B + i4] = y;
-    group_sync<NB>(grp);
-    part[p4 * B + j4] = col_dot(matrix(j, 0, 0), tv + B);
-    group_sync<NB>(grp);
-    publish(0, nb > 1);
-  }
-  o -= TS::kAll;
-  --j;
-  for (int l = levels - 1; l >= 0; --l) {
-    const int s = 1 << l, begin = base(l);
-    cluster.sync();
-    for (; o >= begin; o -= TS::kAll, --j) {
-      const int i = block_of(o, l);
-      group_sync<NB>(grp);
-      double z = row_dot(matrix(j, i, 1), vx + (i - s) * B);
-      if (i + s < nb) z += row_dot(matrix(j, i, 2), vx + (i + s) * B);
-      z = quad(z);
-      if (q == 0) tv[i4] = vb[i * B + i4] - z;
-      group_sync<NB>(grp);
-      part[p4 * B + j4] = col_dot(matrix(j, i, 0), tv);
-      group_sync<NB>(grp);
-      publish(i, l > 0);
+  tree.each_block([&](int i, int j, int) {
+    if (tree.t >= B) return;
+    double v = 0.0;
+    if (tree.t < used) {
+      long long node;
+      int d;
+      dof_of(i, tree.t, node, d);
+      v = (double)bs[node * D + d];
     }
-  }
+    tree.vb[(tree.grp * tree.own + j) * B + tree.t] = v;
+  });
+  cg::this_cluster().sync();
+  tree.solve([&](int i, int ii, double v) {
+    if (ii >= used) return;
+    long long node;
+    int d;
+    dof_of(i, ii, node, d);
+    xs[node * D + d] = ((fixed[node] >> d) & 1) ? T(0) : T(v);
+  });
 }
 
 // ---- host ----------------------------------------------------------------------------
@@ -644,14 +692,12 @@ static int tree_factor(const CoarseDesc& co, int hrows, int* status, cudaStream_
 template <int NB, int D, typename T>
 static int tree_solve(const stt_hier* h, int nrows, const T* b, T* x, long long rs, const RowState* rst,
                       cudaStream_t st) {
-  using TS = TreeSolve<NB>;
   const LevelDesc& lv = h->lv[h->nlevels - 1];
   const CoarseDesc& co = h->co;
   STT_TRY(allow_smem<tree_solve_kernel<NB, D, T>>());
-  const size_t room = kTreeSmem - TS::vectors(co.nb);
-  const int staged = (int)std::min<size_t>((co.nb + TS::kAll - 1) / TS::kAll, room / (TS::kGroups * TS::kTask));
-  tree_solve_kernel<NB, D, T><<<dim3(kTreeCluster, nrows), TS::kThreads,
-                                TS::vectors(co.nb) + (size_t)staged * TS::kGroups * TS::kTask, st>>>(
+  const size_t vec = 8 * tree_vectors(co.nb, co.B), task = 8 * kTreeGroups * tree_task(co.B);
+  const int staged = (int)std::min<size_t>(tree_own(co.nb), (kTreeSmem - vec) / task);
+  launch((tree_solve_kernel<NB, D, T>), dim3(kTreeCluster, nrows), TreeRow<NB>::kThreads, vec + staged * task, st, 
       b, x, rs, co.blocks, co.nb, staged, co.by_col, lv.nnx, lv.nny, lv.fixed, h->row_map, h->hrows, rst);
   return check_launch("coarse solve");
 }

@@ -12,6 +12,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <utility>
+
 #include "../../include/sttb200.h"
 
 #define STT_DEV __device__ __forceinline__
@@ -69,6 +71,34 @@ __host__ __device__ constexpr int corner_dc(int k) { return (k == 1 || k == 2) ?
 template <typename T>
 STT_DEV T ldg(const T* p) {
   return __ldg(p);
+}
+
+// ---- dependent launches ------------------------------------------------------------
+//
+// The solves' kernels are launched with programmatic stream serialisation: a kernel's blocks
+// may become resident while the kernel before it drains, and wait there.  Every thread of
+// every such kernel calls grid_wait() before anything else (an early return included), so
+// that a grid's completion implies its predecessors'; it returns when the kernels before
+// have completed and their writes are visible, and lets the next kernel's blocks in.  A
+// kernel boundary of the solves' many short kernels costs about 1 us less that way.
+STT_DEV void grid_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(std::forward<A>(args))...);
 }
 
 // ---- block reductions (kNT threads) ---------------------------------------------

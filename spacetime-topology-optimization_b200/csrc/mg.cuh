@@ -96,6 +96,7 @@ __global__ void __launch_bounds__(kQThreads) l0_sweep_kernel(
     const T* __restrict__ rdiag, long long rd_rs, const uint8_t* __restrict__ fixed,
     const int* __restrict__ row_map, int hrows, const RowState* __restrict__ rst, int nelx,
     int nely, T omega, KEq<D, T> ke, int proj_in, ProlongSrc<T> pro) {
+  grid_wait();
   const int s = blockIdx.z;
   if (rst && !rst[s].active) return;
   const int nnx = nelx + 1, nny = nely + 1;
@@ -163,6 +164,7 @@ __global__ void __launch_bounds__(kQThreads) l0_sweep_modal_kernel(
     const T* __restrict__ rdiag, long long rd_rs, const uint8_t* __restrict__ fixed,
     const int* __restrict__ row_map, int hrows, const RowState* __restrict__ rst, int nelx,
     int nely, T omega, MQ<T> mq, ProlongSrc<T> pro) {
+  grid_wait();
   const int s = blockIdx.z;
   if (rst && !rst[s].active) return;
   const int nnx = nelx + 1, nny = nely + 1;
@@ -431,6 +433,7 @@ __global__ void __launch_bounds__(kQThreads, sizeof(T) == 4 ? 6 : 3) l0_presmoot
     long long or_rs, const T* __restrict__ rho, long long rho_rs, const T* __restrict__ rdiag,
     long long rd_rs, const uint8_t* __restrict__ fixed, const int* __restrict__ row_map, int hrows,
     const RowState* __restrict__ rst, int nelx, int nely, T omega, MQ<T> q, RzFuse<T> mx = RzFuse<T>{}) {
+  grid_wait();
   constexpr int LO = 3, HI = 29;
   static_assert(HI - LO + 1 == kPreCols, "strip width");
   const int s = blockIdx.z;
@@ -579,6 +582,7 @@ __global__ void __launch_bounds__(kQThreads, sizeof(T) == 4 ? 6 : 3) l0_postsmoo
     long long o_rs, const T* __restrict__ rho, long long rho_rs, const T* __restrict__ rdiag, long long rd_rs,
     const uint8_t* __restrict__ fixed, const int* __restrict__ row_map, int hrows,
     const RowState* __restrict__ rst, int nelx, int nely, T omega, MQ<T> q, RzFuse<T> rz = RzFuse<T>{}) {
+  grid_wait();
   constexpr int LO = 2, HI = 29;
   static_assert(HI - LO + 1 == kPostCols, "strip width");
   const int s = blockIdx.z;
@@ -795,6 +799,7 @@ __global__ void __launch_bounds__(kQThreads) st_sweep_kernel(
     const T* __restrict__ st, const uint8_t* __restrict__ fixed, int nnx, int nny,
     const int* __restrict__ row_map, int hrows, const RowState* __restrict__ rst, T omega,
     ProlongSrc<T> pro) {
+  grid_wait();
   constexpr int DD = D * D, NS = 5 * DD;
   constexpr bool KU = MODE != SW_FIRST;
   const int s = blockIdx.z;
@@ -964,6 +969,7 @@ __global__ void __launch_bounds__(kQThreads) st_sweep2_kernel(
     const T* __restrict__ x, const T* __restrict__ b, T* __restrict__ out, long long vec_rs,
     const T* __restrict__ st, const uint8_t* __restrict__ fixed, int nnx, int nny,
     const int* __restrict__ row_map, int hrows, const RowState* __restrict__ rst, T omega, int dcompact = 0) {
+  grid_wait();
   static_assert(MODE != SW_POST, "no folded prolongation on stencil levels");
   constexpr int DD = D * D, NS = 5 * DD;
   constexpr bool KU = MODE != SW_FIRST;
@@ -1220,6 +1226,7 @@ __global__ void __launch_bounds__(kQThreads, 6) st_chain_kernel(
     const T* __restrict__ x0, const T* __restrict__ b, T* __restrict__ out_x, T* __restrict__ out_r,
     long long vec_rs, const T* __restrict__ st, const uint8_t* __restrict__ fixed, int nnx, int nny,
     const int* __restrict__ row_map, int hrows, const RowState* __restrict__ rst, T omega) {
+  grid_wait();
   constexpr int DD = D * D, NS = 5 * DD, LO = 2, HI = 29;
   static_assert(HI - LO + 1 == kStChainCols, "strip width");
   const int s = blockIdx.z;
@@ -1383,6 +1390,7 @@ __global__ void __launch_bounds__(kQThreads) l1_sweep_kernel(
     const T* __restrict__ rho0, long long rho_rs, int fnelx, const T* __restrict__ st,
     const uint8_t* __restrict__ fixed, int nnx, int nny, const int* __restrict__ row_map, int hrows,
     const RowState* __restrict__ rst, T omega, L1Mat<T, MIR ? 1 : KX * KY> M) {
+  grid_wait();
   static_assert(MODE == SW_SWEEP || MODE == SW_RESID, "sweep and residual only");
   constexpr int D = 2, NM = KX * KY;
   const int s = blockIdx.z;
@@ -1635,6 +1643,7 @@ __global__ void __launch_bounds__(kQThreads, 4) l1_chain_kernel(
     long long vec_rs, const T* __restrict__ rho0, long long rho_rs, int fnelx, const T* __restrict__ st,
     const uint8_t* __restrict__ fixed, int nnx, int nny, const int* __restrict__ row_map, int hrows,
     const RowState* __restrict__ rst, T omega, L1Mat<T, MIR ? 1 : 4> M) {
+  grid_wait();
   constexpr int D = 2, LO = 2, HI = 29;
   static_assert(HI - LO + 1 == kL1ChainCols, "strip width");
   const int s = blockIdx.z;
@@ -1778,6 +1787,7 @@ __global__ void __launch_bounds__(kQThreads) restrict_kernel(
     const T* __restrict__ rf, long long f_rs, int fnnx, int fnny, T* __restrict__ rc, long long c_rs,
     int cnnx, int cnny, int kx, int ky, const uint8_t* __restrict__ cfixed,
     const RowState* __restrict__ rst) {
+  grid_wait();
   const int s = blockIdx.z;
   if (rst && !rst[s].active) return;
   const T* f = rf + (size_t)s * f_rs;
@@ -1882,6 +1892,7 @@ template <int D, typename T, int KX, int KY>
 __global__ void __launch_bounds__(kQThreads) restrict_t_kernel(
     const T* __restrict__ rf, long long f_rs, int fnnx, int fnny, T* __restrict__ rc, long long c_rs,
     int cnnx, int cnny, const uint8_t* __restrict__ cfixed, const RowState* __restrict__ rst) {
+  grid_wait();
   const int s = blockIdx.z;
   if (rst && !rst[s].active) return;
   const T* f = rf + (size_t)s * f_rs;
@@ -2028,6 +2039,7 @@ template <int D, typename T>
 __global__ void __launch_bounds__(kQThreads) prolong2_kernel(
     const T* __restrict__ ec, long long c_rs, int cnnx, int cnny, T* __restrict__ xf, long long f_rs, int fnnx,
     int fnny, int kx, int ky, const uint8_t* __restrict__ ffixed, const RowState* __restrict__ rst) {
+  grid_wait();
   const int s = blockIdx.z;
   if (rst && !rst[s].active) return;
   const T* e = ec + (size_t)s * c_rs;
@@ -2118,6 +2130,7 @@ template <int D, typename T, int KX, int KY>
 __global__ void __launch_bounds__(kQThreads) prolong_t_kernel(
     const T* __restrict__ ec, long long c_rs, int cnnx, int cnny, T* __restrict__ xf, long long f_rs, int fnnx,
     int fnny, const uint8_t* __restrict__ ffixed, const RowState* __restrict__ rst) {
+  grid_wait();
   constexpr int NQ = KY == 3 ? 6 : 4;  // fine rows in flight, a multiple of KY
   constexpr int CR = NQ / KY;          // coarse rows a step
   const int s = blockIdx.z;
@@ -2237,6 +2250,7 @@ __global__ void __launch_bounds__(4 * 4 * NC) coarse_solve_kernel(
     int nb, int by_col, int nnx, int nny, const uint8_t* __restrict__ fixed,
     double* __restrict__ scratch, const int* __restrict__ row_map, int hrows,
     const RowState* __restrict__ rst) {
+  grid_wait();
   constexpr int B = 4 * NC;
   __shared__ double vp[B];  // previous step's block solution
   __shared__ double tv[B];  // current step's right-hand side
@@ -2330,6 +2344,7 @@ __global__ void __launch_bounds__(4 * 4 * NC) coarse_solve_kernel(
 template <typename TI, typename TO>
 __global__ void rows_convert_kernel(const TI* __restrict__ in, long long in_rs, TO* __restrict__ out,
                                     long long out_rs, long long n, const RowState* __restrict__ rst) {
+  grid_wait();
   const int s = blockIdx.y;
   if (rst && !rst[s].active) return;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
@@ -2340,6 +2355,7 @@ __global__ void rows_convert_kernel(const TI* __restrict__ in, long long in_rs, 
 template <typename T>
 __global__ void rows_axpy_kernel(const T* __restrict__ a, T* __restrict__ y, long long rs, long long n,
                                  const RowState* __restrict__ rst) {
+  grid_wait();
   const int s = blockIdx.y;
   if (rst && !rst[s].active) return;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;

@@ -194,14 +194,14 @@ struct Cycle {
     L1Mat<T, KX * KY> M;                                                                             \
     for (int m = 0; m < KX * KY; ++m)                                                                \
       for (int e = 0; e < 21; ++e) M.m[m][e] = T(h->l1m[m][e]);                                      \
-    l1_sweep_kernel<T, MODE, KX, KY><<<g, kQThreads, 0, st>>>(x, b, out, vstride(lv.ndof), r0, f.rs_rho, \
+    launch((l1_sweep_kernel<T, MODE, KX, KY>), g, kQThreads, 0, st, x, b, out, vstride(lv.ndof), r0, f.rs_rho, \
                                                               f.nelx, stl(1), lv.fixed, lv.nnx, lv.nny,  \
                                                               h->row_map, h->hrows, rst, omega, M);      \
   } while (0)
       if (f.kx == 2 && f.ky == 2 && h->l1par) {
         L1Mat<T, 1> M;  // M_0 only
         for (int e = 0; e < 21; ++e) M.m[0][e] = T(h->l1m[0][e]);
-        l1_sweep_kernel<T, MODE, 2, 2, 2, true><<<g, kQThreads, 0, st>>>(
+        launch((l1_sweep_kernel<T, MODE, 2, 2, 2, true>), g, kQThreads, 0, st, 
             x, b, out, vstride(lv.ndof), r0, f.rs_rho, f.nelx, stl(1), lv.fixed, lv.nnx, lv.nny, h->row_map, h->hrows,
             rst, omega, M);
       } else if (f.kx == 2 && f.ky == 2) STT_L1(2, 2);
@@ -220,20 +220,20 @@ struct Cycle {
   void transfer_down(const LevelDesc& lv, const LevelDesc& cl, const T* rf, long long nd, T* rc, long long cnd) {
     const dim3 g = coarse_grid(cl.nelx, cl.nely, nrows);
 #define STT_RESTRICT(KX, KY)                                                                       \
-  restrict_t_kernel<D, T, KX, KY><<<g, kQThreads, 0, st>>>(rf, nd, lv.nnx, lv.nny, rc, cnd, cl.nnx, \
+  launch((restrict_t_kernel<D, T, KX, KY>), g, kQThreads, 0, st, rf, nd, lv.nnx, lv.nny, rc, cnd, cl.nnx, \
                                                            cl.nny, cl.fixed, rst)
     STT_KXKY_DISPATCH(lv.kx, lv.ky, STT_RESTRICT,
-                      (restrict_kernel<D, T><<<g, kQThreads, 0, st>>>(rf, nd, lv.nnx, lv.nny, rc, cnd, cl.nnx,
+                      (launch((restrict_kernel<D, T>), g, kQThreads, 0, st, rf, nd, lv.nnx, lv.nny, rc, cnd, cl.nnx,
                                                                       cl.nny, lv.kx, lv.ky, cl.fixed, rst)));
 #undef STT_RESTRICT
   }
   void transfer_up(const LevelDesc& lv, const LevelDesc& cl, const T* ec, long long cnd, T* xf, long long nd) {
     const dim3 g = prolong2_grid(lv.nnx, lv.nny, nrows);
 #define STT_PROLONG(KX, KY)                                                                         \
-  prolong_t_kernel<D, T, KX, KY><<<g, kQThreads, 0, st>>>(ec, cnd, cl.nnx, cl.nny, xf, nd, lv.nnx, lv.nny, \
+  launch((prolong_t_kernel<D, T, KX, KY>), g, kQThreads, 0, st, ec, cnd, cl.nnx, cl.nny, xf, nd, lv.nnx, lv.nny, \
                                                           lv.fixed, rst)
     STT_KXKY_DISPATCH(lv.kx, lv.ky, STT_PROLONG,
-                      (prolong2_kernel<D, T><<<g, kQThreads, 0, st>>>(ec, cnd, cl.nnx, cl.nny, xf, nd, lv.nnx,
+                      (launch((prolong2_kernel<D, T>), g, kQThreads, 0, st, ec, cnd, cl.nnx, cl.nny, xf, nd, lv.nnx,
                                                                       lv.nny, lv.kx, lv.ky, lv.fixed, rst)));
 #undef STT_PROLONG
   }
@@ -247,26 +247,26 @@ struct Cycle {
     if (l == 0) {
       const dim3 g = march_grid<true, T>(lv.nelx, lv.nely, nrows);
       if (h->modal && h->has_reaction)
-        l0_sweep_modal_kernel<D, T, MODE, true><<<g, kQThreads, 0, st>>>(
+        launch((l0_sweep_modal_kernel<D, T, MODE, true>), g, kQThreads, 0, st, 
             x, x_rs, b, b_rs, out, o_rs, rho0(), lv.rs_rho, rdiag0(), lv.ndof, lv.fixed, h->row_map,
             h->hrows, rst, lv.nelx, lv.nely, omega, mq, pro);
       else if (h->modal)
-        l0_sweep_modal_kernel<D, T, MODE, false><<<g, kQThreads, 0, st>>>(
+        launch((l0_sweep_modal_kernel<D, T, MODE, false>), g, kQThreads, 0, st, 
             x, x_rs, b, b_rs, out, o_rs, rho0(), lv.rs_rho, rdiag0(), lv.ndof, lv.fixed, h->row_map,
             h->hrows, rst, lv.nelx, lv.nely, omega, mq, pro);
       else
-        l0_sweep_kernel<D, T, MODE><<<g, kQThreads, 0, st>>>(
+        launch((l0_sweep_kernel<D, T, MODE>), g, kQThreads, 0, st, 
             x, x_rs, b, b_rs, out, o_rs, rho0(), lv.rs_rho, rdiag0(), lv.ndof, lv.fixed, h->row_map,
             h->hrows, rst, lv.nelx, lv.nely, omega, ke, 0, pro);
     } else if (l1_pass<MODE>(l, x, b, out)) {
       // level 1 applied from the level-0 densities
     } else {
       if constexpr (MODE == SW_POST)
-        st_sweep_kernel<D, T, MODE><<<tile_grid(lv.nelx, lv.nely, nrows), kQThreads, 0, st>>>(
+        launch((st_sweep_kernel<D, T, MODE>), tile_grid(lv.nelx, lv.nely, nrows), kQThreads, 0, st, 
             x, b, out, vstride(lv.ndof), stl(l), lv.fixed, lv.nnx, lv.nny, h->row_map, h->hrows, rst, omega,
             pro);
       else
-        st_sweep2_kernel<D, T, MODE><<<coarse_grid(lv.nelx, lv.nely, nrows), kQThreads, 0, st>>>(
+        launch((st_sweep2_kernel<D, T, MODE>), coarse_grid(lv.nelx, lv.nely, nrows), kQThreads, 0, st, 
             x, b, out, vstride(lv.ndof), stl(l), lv.fixed, lv.nnx, lv.nny, h->row_map, h->hrows, rst, omega,
             (sizeof(T) == 4 && l == 1 && h->l1) ? 1 : 0);
     }
@@ -285,7 +285,7 @@ struct Cycle {
       return;
     }
 #define STT_COARSE(NC)                                                                          \
-  coarse_solve_kernel<D, T, NC><<<nrows, 16 * NC, 0, st>>>(b, x, vstride(lv.ndof), co.blocks, co.nb, co.by_col, \
+  launch((coarse_solve_kernel<D, T, NC>), nrows, 16 * NC, 0, st, b, x, vstride(lv.ndof), co.blocks, co.nb, co.by_col, \
                                                           lv.nnx, lv.nny, lv.fixed, w.cscratch,       \
                                                           h->row_map, h->hrows, rst)
     switch (co.B) {
@@ -307,7 +307,7 @@ struct Cycle {
     RzFuse<T> mx = rzf;
     mx.red.nblk = (int)(g.x * g.y);
 #define STT_PRE(RD, MX)                                                                                  \
-  l0_presmooth_kernel<D, T, RD, MX><<<g, kQThreads, 0, st>>>(b, b_rs, out_x, nd, out_r, nd, rho0(), lv.rs_rho, \
+  launch((l0_presmooth_kernel<D, T, RD, MX>), g, kQThreads, 0, st, b, b_rs, out_x, nd, out_r, nd, rho0(), lv.rs_rho, \
                                                            rdiag0(), lv.ndof, lv.fixed, h->row_map, h->hrows,  \
                                                            rst, lv.nelx, lv.nely, omega, mq, mx)
     if (rzf.rst && rzf.zold) {
@@ -340,7 +340,7 @@ struct Cycle {
     L1Mat<T, NM> M;                                                                                           \
     for (int m = 0; m < NM; ++m)                                                                              \
       for (int e = 0; e < 21; ++e) M.m[m][e] = T(h->l1m[m][e]);                                               \
-    l1_chain_kernel<T, PRE, MIR><<<g, kQThreads, 0, st>>>(x0, b, ox, orr, vs, rho0(), f.rs_rho, f.nelx, stl(1), \
+    launch((l1_chain_kernel<T, PRE, MIR>), g, kQThreads, 0, st, x0, b, ox, orr, vs, rho0(), f.rs_rho, f.nelx, stl(1), \
                                                           lv.fixed, lv.nnx, lv.nny, h->row_map, h->hrows, rst,  \
                                                           omega, M);                                            \
   } while (0)
@@ -364,10 +364,10 @@ struct Cycle {
       const dim3 g = st_chain_grid(lv.nelx, lv.nely, nrows);
       const long long vs = vstride(lv.ndof);
       if (pre)
-        st_chain_kernel<D, T, true><<<g, kQThreads, 0, st>>>(x0, b, ox, orr, vs, stl(l), lv.fixed, lv.nnx, lv.nny,
+        launch((st_chain_kernel<D, T, true>), g, kQThreads, 0, st, x0, b, ox, orr, vs, stl(l), lv.fixed, lv.nnx, lv.nny,
                                                              h->row_map, h->hrows, rst, omega);
       else
-        st_chain_kernel<D, T, false><<<g, kQThreads, 0, st>>>(x0, b, ox, orr, vs, stl(l), lv.fixed, lv.nnx,
+        launch((st_chain_kernel<D, T, false>), g, kQThreads, 0, st, x0, b, ox, orr, vs, stl(l), lv.fixed, lv.nnx,
                                                               lv.nny, h->row_map, h->hrows, rst, omega);
       return true;
     }
@@ -383,7 +383,7 @@ struct Cycle {
     rz.red.nblk = (int)(g.x * g.y);
     const bool fuse = rzf.rst && (!rzf.zold || mix_done);
 #define STT_POST(RD, RZ)                                                                                  \
-  l0_postsmooth_kernel<D, T, RD, RZ><<<g, kQThreads, 0, st>>>(x0, nd, b, b_rs, out, nd, rho0(), lv.rs_rho,     \
+  launch((l0_postsmooth_kernel<D, T, RD, RZ>), g, kQThreads, 0, st, x0, nd, b, b_rs, out, nd, rho0(), lv.rs_rho,     \
                                                             rdiag0(), lv.ndof, lv.fixed, h->row_map, h->hrows, \
                                                             rst, lv.nelx, lv.nely, omega, mq, rz)
     if (fuse) {
@@ -405,12 +405,12 @@ struct Cycle {
     if (gamma > 1) {
       T* acc = (T*)w.acc[l + 1];
       T* rhs = (T*)w.rhs2[l + 1];
-      rows_convert_kernel<T, T><<<dim3(ew_blocks(cl.ndof), nrows), kEwThreads, 0, st>>>(ec, cnd, acc, cnd, cl.ndof, rst);
+      launch((rows_convert_kernel<T, T>), dim3(ew_blocks(cl.ndof), nrows), kEwThreads, 0, st, ec, cnd, acc, cnd, cl.ndof, rst);
       for (int g = 1; g < gamma; ++g) {
         // rhs = b_c - A_c acc
         pass<SW_RESID>(l + 1, acc, cnd, bc, cnd, rhs, cnd);
         T* e2 = cycle(l + 1, rhs, cnd);
-        rows_axpy_kernel<T><<<dim3(ew_blocks(cl.ndof), nrows), kEwThreads, 0, st>>>(e2, acc, cnd, cl.ndof, rst);
+        launch(rows_axpy_kernel<T>, dim3(ew_blocks(cl.ndof), nrows), kEwThreads, 0, st, e2, acc, cnd, cl.ndof, rst);
       }
       ec = acc;
     }
@@ -426,7 +426,7 @@ struct Cycle {
       // the coarse solve reads b with the level's own row stride
       const T* bb = b;
       if (b_rs != nd) {
-        rows_convert_kernel<T, T><<<dim3(ew_blocks(lv.ndof), nrows), kEwThreads, 0, st>>>(b, b_rs, Tt(l), nd, lv.ndof, rst);
+        launch((rows_convert_kernel<T, T>), dim3(ew_blocks(lv.ndof), nrows), kEwThreads, 0, st, b, b_rs, Tt(l), nd, lv.ndof, rst);
         bb = Tt(l);
       }
       coarse(l, bb, X(l));
@@ -534,6 +534,7 @@ __global__ void __launch_bounds__(kQThreads) pcg_init_kernel(
     const double* __restrict__ rdiag, long long rd_rs, const uint8_t* __restrict__ fixed,
     const int* __restrict__ row_map, int hrows, RowState* __restrict__ rst, GridRed red,
     int nelx, int nely, KEq<D, double> ke, MQ<double> mq, PcgParams pp, int replace) {
+  grid_wait();
   const int s = blockIdx.z;
   if (replace && !rst[s].active) return;
   const int nnx = nelx + 1, nny = nely + 1;
@@ -614,6 +615,7 @@ __global__ void __launch_bounds__(kQThreads) pcg_init_kernel(
 __global__ void __launch_bounds__(kEwThreads) pcg_init_b_kernel(
     const double* __restrict__ b, long long b_rs, double* __restrict__ r, long long r_rs, long long n,
     float* __restrict__ r32, long long r32_rs, RowState* __restrict__ rst, GridRed red, PcgParams pp) {
+  grid_wait();
   const int s = blockIdx.y;
   const double* bs = b + (size_t)s * b_rs;
   double* rs_ = r + (size_t)s * r_rs;
@@ -656,6 +658,7 @@ __global__ void __launch_bounds__(kQThreads) pcg_pap_kernel(
     const double* __restrict__ rho, long long rho_rs, const double* __restrict__ rdiag, long long rd_rs,
     const uint8_t* __restrict__ fixed, const int* __restrict__ row_map, int hrows, RowState* __restrict__ rst,
     GridRed red, int nelx, int nely, KEq<D, double> ke, MQ<double> mq) {
+  grid_wait();
   static_assert(PMODE == 1 || PMODE == 2, "p = z or p = beta p + z");
   static_assert(!XP || PMODE == 2, "a pending x update follows an earlier p");
   const int s = blockIdx.z;
@@ -749,6 +752,7 @@ __global__ void __launch_bounds__(kQThreads) pcg_pap_kernel(
 __global__ void __launch_bounds__(kEwThreads) pcg_update_kernel(
     double* __restrict__ r, const double* __restrict__ Ap, long long rs, long long n,
     RowState* __restrict__ rst, GridRed red, PcgParams pp, float* __restrict__ r32, long long r32_rs) {
+  grid_wait();
   const int s = blockIdx.y;
   if (!rst[s].active) return;
   const double alpha = rst[s].alpha;
@@ -798,6 +802,7 @@ __global__ void __launch_bounds__(kEwThreads) pcg_update_kernel(
 // converged row stops (its x stays as of this iteration), and when no row is short of
 // rtol all stop.  One warp; rows in order.
 __global__ void pcg_retire_kernel(RowState* __restrict__ rst, int nrows, int* __restrict__ last, int it) {
+  grid_wait();
   const int lane = threadIdx.x;
   int n_left = 0;  // active rows not yet converged
   for (int s = lane; s < nrows; s += 32) n_left += (rst[s].active && !rst[s].conv) ? 1 : 0;
@@ -830,6 +835,7 @@ __global__ void __launch_bounds__(kEwThreads) pcg_xflush_kernel(double* __restri
                                                                 const double* __restrict__ p0,
                                                                 const double* __restrict__ p1, long long rs,
                                                                 long long n, const RowState* __restrict__ rst) {
+  grid_wait();
   const int s = blockIdx.y;
   if (!rst[s].xpend) return;
   const double alpha = rst[s].alpha;
@@ -841,6 +847,7 @@ __global__ void __launch_bounds__(kEwThreads) pcg_xflush_kernel(double* __restri
 }
 
 __global__ void pcg_xclear_kernel(RowState* __restrict__ rst, int nrows) {
+  grid_wait();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s < nrows) rst[s].xpend = 0;
 }
@@ -852,6 +859,7 @@ __global__ void __launch_bounds__(kEwThreads) pcg_rz_kernel(
     const TR* __restrict__ r, const TZ* __restrict__ z, const TZ* __restrict__ zold,
     double* __restrict__ p, long long rs, long long z_rs, long long n, RowState* __restrict__ rst,
     GridRed red, int first, int flexible) {
+  grid_wait();
   const int s = blockIdx.y;
   if (!rst[s].active) return;
   const TR* rsv = r + (size_t)s * rs;
@@ -903,6 +911,7 @@ __global__ void __launch_bounds__(kEwThreads) pcg_rz_kernel(
 
 
 __global__ void rows_zero_kernel(double* __restrict__ x, long long rs, long long n) {
+  grid_wait();
   const int s = blockIdx.y;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x)
@@ -933,7 +942,7 @@ static int run_vcycle(const stt_hier* h, SolveWS& w, int nrows, const double* r,
   if constexpr (sizeof(T) == 4) {
     // the PCG update may have written the FP32 copy of r already
     if (!b0_ready)
-      rows_convert_kernel<double, float><<<dim3(ew_blocks(n), nrows), kEwThreads, 0, st>>>(
+      launch((rows_convert_kernel<double, float>), dim3(ew_blocks(n), nrows), kEwThreads, 0, st, 
           r, r_rs, (float*)w.b0, vs, n, rst);
     b0 = (const T*)w.b0;
     b_rs = vs;
@@ -945,7 +954,7 @@ static int run_vcycle(const stt_hier* h, SolveWS& w, int nrows, const double* r,
   T* res = cyc.cycle(0, b0, b_rs);
   if (rz_done) *rz_done = cyc.rz_done;
   if (res != zout)
-    rows_convert_kernel<T, T><<<dim3(ew_blocks(n), nrows), kEwThreads, 0, st>>>(res, vs, zout, vs, n, rst);
+    launch((rows_convert_kernel<T, T>), dim3(ew_blocks(n), nrows), kEwThreads, 0, st, res, vs, zout, vs, n, rst);
   return check_launch("vcycle");
 }
 
@@ -1024,7 +1033,7 @@ static int run_pcg(const stt_hier* h, SolveWS& w, int nrows, const double* b, lo
   const double* rd0 = h->has_reaction ? l0.rdiag64 : nullptr;
   STT_TRY(check_cuda(cudaMemsetAsync(w.counters, 0, 4LL * nrows, st), "memset counters"));
   STT_TRY(check_cuda(cudaMemsetAsync(w.rs, 0, sizeof(RowState) * nrows, st), "memset rows"));
-  if (!has_x0) rows_zero_kernel<<<dim3(ewb, nrows), kEwThreads, 0, st>>>(x, x_rs, nd);
+  if (!has_x0) launch(rows_zero_kernel, dim3(ewb, nrows), kEwThreads, 0, st, x, x_rs, nd);
   const MQ<double> mq = mq_cast<double>(h->mq);
   bool timing = false;
   if (D == 2) {
@@ -1039,12 +1048,12 @@ static int run_pcg(const stt_hier* h, SolveWS& w, int nrows, const double* b, lo
   float* r32init = sizeof(T) == 4 ? (float*)w.b0 : nullptr;
   auto init = [&](const double* xx, const PcgParams& pq, int replace) {
     if (!xx && !replace) {
-      pcg_init_b_kernel<<<dim3(upb, nrows), kEwThreads, 0, st>>>(b, b_rs, w.r, nd, nd, r32init, vstride(nd), w.rs,
+      launch(pcg_init_b_kernel, dim3(upb, nrows), kEwThreads, 0, st, b, b_rs, w.r, nd, nd, r32init, vstride(nd), w.rs,
                                                                   red_up, pq);
       return;
     }
 #define STT_INIT(MODAL, RD)                                                                              \
-  pcg_init_kernel<D, MODAL, RD><<<tg, kQThreads, 0, st>>>(b, b_rs, xx, x_rs, w.r, nd, l0.rho64, l0.rs_rho, rd0, \
+  launch((pcg_init_kernel<D, MODAL, RD>), tg, kQThreads, 0, st, b, b_rs, xx, x_rs, w.r, nd, l0.rho64, l0.rs_rho, rd0, \
                                                           l0.ndof, l0.fixed, h->row_map, h->hrows, w.rs,        \
                                                           red_tile, h->nelx, h->nely, ke, mq, pq, replace)
     if (h->modal) {
@@ -1058,7 +1067,7 @@ static int run_pcg(const stt_hier* h, SolveWS& w, int nrows, const double* b, lo
   };
   PcgParams pp{rtol, 0, flexible, sched ? 1 : 0};
   init(has_x0 ? x : nullptr, pp, 0);
-  if (sched) pcg_retire_kernel<<<1, 32, 0, st>>>(w.rs, nrows, w.sched_last, 0);
+  if (sched) launch(pcg_retire_kernel, 1, 32, 0, st, w.rs, nrows, w.sched_last, 0);
   STT_TRY(check_launch("pcg init"));
   std::vector<RowState> host(nrows);
   // the reads after the first V-cycle also carry the hierarchy build's status word (the
@@ -1097,8 +1106,8 @@ static int run_pcg(const stt_hier* h, SolveWS& w, int nrows, const double* b, lo
     // adds every row's pending alpha p to x (before a true-residual replacement and at
     // the end); the p.Ap pass of the next iteration does it for rows still iterating
     auto flush_x = [&]() {
-      pcg_xflush_kernel<<<dim3(ewb, nrows), kEwThreads, 0, st>>>(x, x_rs, w.p, w.p2, nd, nd, w.rs);
-      pcg_xclear_kernel<<<(nrows + 127) / 128, 128, 0, st>>>(w.rs, nrows);
+      launch(pcg_xflush_kernel, dim3(ewb, nrows), kEwThreads, 0, st, x, x_rs, w.p, w.p2, nd, nd, w.rs);
+      launch(pcg_xclear_kernel, (nrows + 127) / 128, 128, 0, st, w.rs, nrows);
     };
     bool pending = false;  // the rows still iterating have an x update pending
     // r . z: the mixed cycle's z carries FP32 rounding, so its dots read the FP32 copy of r
@@ -1117,10 +1126,10 @@ static int run_pcg(const stt_hier* h, SolveWS& w, int nrows, const double* b, lo
     };
     auto rz = [&](int first) {
       if constexpr (sizeof(T) == 4)
-        pcg_rz_kernel<T, float><<<dim3(rzb, nrows), kEwThreads, 0, st>>>(
+        launch((pcg_rz_kernel<T, float>), dim3(rzb, nrows), kEwThreads, 0, st, 
             (const float*)w.b0, z, zold, nullptr, vstride(nd), vstride(nd), nd, w.rs, red_rz, first, flexible);
       else
-        pcg_rz_kernel<T, double><<<dim3(ewb, nrows), kEwThreads, 0, st>>>(w.r, z, zold, nullptr, nd, vstride(nd),
+        launch((pcg_rz_kernel<T, double>), dim3(ewb, nrows), kEwThreads, 0, st, w.r, z, zold, nullptr, nd, vstride(nd),
                                                                            nd, w.rs, red_ew, first, flexible);
     };
     {
@@ -1134,7 +1143,7 @@ static int run_pcg(const stt_hier* h, SolveWS& w, int nrows, const double* b, lo
     for (it = 1; it <= max_iter; ++it) {
       pp.it = it;
 #define STT_PAP(MODAL, RD, PM, XP)                                                                         \
-  pcg_pap_kernel<D, MODAL, RD, T, PM, XP><<<tg, kQThreads, 0, st>>>(                                       \
+  launch((pcg_pap_kernel<D, MODAL, RD, T, PM, XP>), tg, kQThreads, 0, st,                                        \
       pcur, pnext, pnext_buf, z, vstride(nd), x, x_rs, w.Ap, nd, l0.rho64, l0.rs_rho, rd0, l0.ndof, l0.fixed, \
       h->row_map, h->hrows, w.rs, red_tile, h->nelx, h->nely, ke, mq)
 #define STT_PAP2(PM, XP)                    \
@@ -1161,9 +1170,9 @@ static int run_pcg(const stt_hier* h, SolveWS& w, int nrows, const double* b, lo
       float* r32 = sizeof(T) == 4 ? (float*)w.b0 : nullptr;
       std::swap(pcur, pnext);
       pnext_buf ^= 1;
-      pcg_update_kernel<<<dim3(upb, nrows), kEwThreads, 0, st>>>(w.r, w.Ap, nd, nd, w.rs, red_up, pp, r32,
+      launch(pcg_update_kernel, dim3(upb, nrows), kEwThreads, 0, st, w.r, w.Ap, nd, nd, w.rs, red_up, pp, r32,
                                                                   vstride(nd));
-      if (sched) pcg_retire_kernel<<<1, 32, 0, st>>>(w.rs, nrows, w.sched_last, it);
+      if (sched) launch(pcg_retire_kernel, 1, 32, 0, st, w.rs, nrows, w.sched_last, it);
       pending = true;
       const bool replaced = replace_every > 0 && it % replace_every == 0;
       if (replaced) {
@@ -1244,12 +1253,12 @@ extern "C" int stt_vcycle(const stt_hier* h, int nrows, const double* r, long lo
     rc = h->d == 2 ? run_vcycle<2, float>(h, w, nrows, r, r_rs, (float*)w.z, omega, n_smooth, gamma, nullptr, st)
                    : run_vcycle<1, float>(h, w, nrows, r, r_rs, (float*)w.z, omega, n_smooth, gamma, nullptr, st);
     if (rc == STT_OK)
-      rows_convert_kernel<float, double><<<dim3(ew_blocks(nd), nrows), kEwThreads, 0, st>>>((float*)w.z, vstride(nd), z, z_rs, nd, nullptr);
+      launch((rows_convert_kernel<float, double>), dim3(ew_blocks(nd), nrows), kEwThreads, 0, st, (float*)w.z, vstride(nd), z, z_rs, nd, nullptr);
   } else {
     rc = h->d == 2 ? run_vcycle<2, double>(h, w, nrows, r, r_rs, (double*)w.z, omega, n_smooth, gamma, nullptr, st)
                    : run_vcycle<1, double>(h, w, nrows, r, r_rs, (double*)w.z, omega, n_smooth, gamma, nullptr, st);
     if (rc == STT_OK)
-      rows_convert_kernel<double, double><<<dim3(ew_blocks(nd), nrows), kEwThreads, 0, st>>>((double*)w.z, vstride(nd), z, z_rs, nd, nullptr);
+      launch((rows_convert_kernel<double, double>), dim3(ew_blocks(nd), nrows), kEwThreads, 0, st, (double*)w.z, vstride(nd), z, z_rs, nd, nullptr);
   }
   if (rc != STT_OK) return rc;
   return check_launch("stt_vcycle");
@@ -1273,15 +1282,15 @@ extern "C" int stt_level_apply(const stt_hier* h, int level, int nrows, const do
 #define STT_L0_APPLY(D)                                                                                  \
   do {                                                                                                   \
     if (h->modal && rd)                                                                                  \
-      l0_sweep_modal_kernel<D, double, SW_APPLY, true><<<g, kQThreads, 0, st>>>(                        \
+      launch((l0_sweep_modal_kernel<D, double, SW_APPLY, true>), g, kQThreads, 0, st,                         \
           v, v_rs, nullptr, 0, out, out_rs, lv.rho64, lv.rs_rho, rd, lv.ndof, lv.fixed, h->row_map,      \
           h->hrows, nullptr, lv.nelx, lv.nely, 1.0, mq, none);                                          \
     else if (h->modal)                                                                                   \
-      l0_sweep_modal_kernel<D, double, SW_APPLY, false><<<g, kQThreads, 0, st>>>(                       \
+      launch((l0_sweep_modal_kernel<D, double, SW_APPLY, false>), g, kQThreads, 0, st,                        \
           v, v_rs, nullptr, 0, out, out_rs, lv.rho64, lv.rs_rho, rd, lv.ndof, lv.fixed, h->row_map,      \
           h->hrows, nullptr, lv.nelx, lv.nely, 1.0, mq, none);                                          \
     else                                                                                                 \
-      l0_sweep_kernel<D, double, SW_APPLY><<<g, kQThreads, 0, st>>>(                                    \
+      launch((l0_sweep_kernel<D, double, SW_APPLY>), g, kQThreads, 0, st,                                     \
           v, v_rs, nullptr, 0, out, out_rs, lv.rho64, lv.rs_rho, rd, lv.ndof, lv.fixed, h->row_map,      \
           h->hrows, nullptr, lv.nelx, lv.nely, 1.0, ke_of<D, double>(h), 1, none);                      \
   } while (0)
@@ -1294,11 +1303,11 @@ extern "C" int stt_level_apply(const stt_hier* h, int level, int nrows, const do
     return set_error(STT_ERR_INVALID, "stt_level_apply: coarse levels need equal row strides");
   STT_TRY(ensure_level1_fp64(h, level, st));
   if (h->d == 2)
-    st_sweep2_kernel<2, double, SW_APPLY><<<tile_grid(lv.nelx, lv.nely, nrows), kQThreads, 0, st>>>(
-        v, nullptr, out, v_rs, lv.st64, lv.fixed, lv.nnx, lv.nny, h->row_map, h->hrows, nullptr, 1.0);
+    launch((st_sweep2_kernel<2, double, SW_APPLY>), tile_grid(lv.nelx, lv.nely, nrows), kQThreads, 0, st, 
+        v, nullptr, out, v_rs, lv.st64, lv.fixed, lv.nnx, lv.nny, h->row_map, h->hrows, nullptr, 1.0, 0);
   else
-    st_sweep2_kernel<1, double, SW_APPLY><<<tile_grid(lv.nelx, lv.nely, nrows), kQThreads, 0, st>>>(
-        v, nullptr, out, v_rs, lv.st64, lv.fixed, lv.nnx, lv.nny, h->row_map, h->hrows, nullptr, 1.0);
+    launch((st_sweep2_kernel<1, double, SW_APPLY>), tile_grid(lv.nelx, lv.nely, nrows), kQThreads, 0, st, 
+        v, nullptr, out, v_rs, lv.st64, lv.fixed, lv.nnx, lv.nny, h->row_map, h->hrows, nullptr, 1.0, 0);
   return check_launch("level apply");
 }
 

@@ -416,11 +416,55 @@ struct RzFuse {
   int first, flexible;
 };
 
+// The launch shapes a solve uses, tunable per hierarchy (stt_hier_tune) and set on the
+// calling host thread for the duration of a solve entry point: pcg_band, the rows a block
+// of the PCG's level-0 passes marches (8, 16 or 32; 0: the heuristic of pcg_tile_grid);
+// waves, the blocks band_rows aims at in units of one block per SM (0: four).
+struct LaunchTuning {
+  int pcg_band = 0;
+  int waves = 0;
+};
+inline LaunchTuning& launch_tuning() {
+  static thread_local LaunchTuning t;
+  return t;
+}
+struct ScopedTuning {
+  LaunchTuning saved;
+  ScopedTuning(int pcg_band, int waves) : saved(launch_tuning()) { launch_tuning() = LaunchTuning{pcg_band, waves}; }
+  ~ScopedTuning() { launch_tuning() = saved; }
+};
+
+// Rows a block marches on the coarse levels: 32 where the grid then fills the GPU,
+// shorter bands on small grids (the heat solve's single row, the coarse levels), whose
+// launches are otherwise latency-bound by the sequential march down 32 rows.  The
+// kernels derive their band from gridDim.y, so any grid.y covers the rows.
+inline int band_rows(int xblocks, int nny, int rows) {
+  const int waves = launch_tuning().waves > 0 ? launch_tuning().waves : 4;
+  const long long target = (long long)waves * 148;  // blocks: waves of one block per B200 SM
+  for (int band = 32; band > 4; band /= 2)
+    if ((long long)xblocks * ((nny + band - 1) / band) * rows >= target) return band;
+  return 4;
+}
+
+// Rows a block of the densities' chained passes (level 0, level 1) marches: 32, or shorter
+// bands (down to 4) while the launch has fewer blocks than fit the SMs at once (`resident` an
+// SM).  The march is a serial chain of a band's rows and three or four more, 0.4 us a row,
+// so a grid that leaves SMs idle is faster with short bands, at up to twice the work.  A
+// V-cycle of 180x60 x 9 rows in FP64: 87 us with 32-row bands, 68 us with these; 256x128 x 8
+// mixed 112 -> 90 us; 540x270 x 4 mixed 138 -> 107 us; past a full wave the two are equal.
+inline int march_band(int xblocks, int nny, int rows, int resident) {
+  int band = kQRows;
+  while (band > 4 && (long long)xblocks * ((nny + band - 1) / band) * rows < 148LL * resident) band /= 2;
+  return band;
+}
+constexpr int l0_resident(int elem_size) { return elem_size == 4 ? 6 : 3; }  // the chained passes' blocks an SM
+
 constexpr int kPreCols = 27;  // output columns per warp strip of l0_presmooth_kernel
 
-inline dim3 presmooth_grid(int nelx, int nely, int rows) {
-  const int strips = (nelx + 1 + kPreCols - 1) / kPreCols;
-  return dim3((strips + kQWarps - 1) / kQWarps, (nely + 1 + kQRows - 1) / kQRows, rows);
+inline dim3 presmooth_grid(int nelx, int nely, int rows, int elem_size) {
+  const int strips = (nelx + 1 + kPreCols - 1) / kPreCols, xb = (strips + kQWarps - 1) / kQWarps;
+  const int band = march_band(xb, nely + 1, rows, l0_resident(elem_size));
+  return dim3(xb, (nely + 1 + band - 1) / band, rows);
 }
 
 // FP32: 6 blocks of 128 threads an SM (<= 80 registers), measured fastest on B200 at
@@ -428,7 +472,7 @@ inline dim3 presmooth_grid(int nelx, int nely, int rows) {
 // fewer blocks).  FP64 needs twice the registers for the same state: 3 blocks.
 // MX: also r.z_old of the PCG (mx.zold), z_old loaded with the front row's b.
 template <int D, typename T, bool RD, bool MX = false, int AHEAD = 2>
-__global__ void __launch_bounds__(kQThreads, sizeof(T) == 4 ? 6 : 3) l0_presmooth_kernel(
+__global__ void __launch_bounds__(kQThreads, l0_resident(sizeof(T))) l0_presmooth_kernel(
     const T* __restrict__ b, long long b_rs, T* __restrict__ out_x, long long ox_rs, T* __restrict__ out_r,
     long long or_rs, const T* __restrict__ rho, long long rho_rs, const T* __restrict__ rdiag,
     long long rd_rs, const uint8_t* __restrict__ fixed, const int* __restrict__ row_map, int hrows,
@@ -451,8 +495,9 @@ __global__ void __launch_bounds__(kQThreads, sizeof(T) == 4 ? 6 : 3) l0_presmoot
   const bool out_lane = lane >= LO && lane <= HI && c < nnx;
   const bool col_ok = c >= 0 && c < nnx;
   const bool ecol_ok = c >= 0 && c < nelx;
-  const int r0 = blockIdx.y * kQRows;
-  const int r1 = min(r0 + kQRows, nny);
+  const int band = (nny + gridDim.y - 1) / gridDim.y;  // rows per block (any grid.y)
+  const int r0 = blockIdx.y * band;
+  const int r1 = min(r0 + band, nny);
   const T* zos = MX ? mx.zold + (size_t)s * mx.zo_rs : nullptr;
   T zq[MX ? AHEAD : 1][D];  // MX: z_old at the front rows in flight
   double mix[1] = {0.0};
@@ -571,13 +616,14 @@ __global__ void __launch_bounds__(kQThreads, sizeof(T) == 4 ? 6 : 3) l0_presmoot
 // arithmetic is the unfused sweeps'.
 constexpr int kPostCols = 28;
 
-inline dim3 postsmooth_grid(int nelx, int nely, int rows) {
-  const int strips = (nelx + 1 + kPostCols - 1) / kPostCols;
-  return dim3((strips + kQWarps - 1) / kQWarps, (nely + 1 + kQRows - 1) / kQRows, rows);
+inline dim3 postsmooth_grid(int nelx, int nely, int rows, int elem_size) {
+  const int strips = (nelx + 1 + kPostCols - 1) / kPostCols, xb = (strips + kQWarps - 1) / kQWarps;
+  const int band = march_band(xb, nely + 1, rows, l0_resident(elem_size));
+  return dim3(xb, (nely + 1 + band - 1) / band, rows);
 }
 
 template <int D, typename T, bool RD, bool RZ = false, int AHEAD = 2>
-__global__ void __launch_bounds__(kQThreads, sizeof(T) == 4 ? 6 : 3) l0_postsmooth_kernel(
+__global__ void __launch_bounds__(kQThreads, l0_resident(sizeof(T))) l0_postsmooth_kernel(
     const T* __restrict__ x0, long long x_rs, const T* __restrict__ b, long long b_rs, T* __restrict__ out,
     long long o_rs, const T* __restrict__ rho, long long rho_rs, const T* __restrict__ rdiag, long long rd_rs,
     const uint8_t* __restrict__ fixed, const int* __restrict__ row_map, int hrows,
@@ -600,8 +646,9 @@ __global__ void __launch_bounds__(kQThreads, sizeof(T) == 4 ? 6 : 3) l0_postsmoo
   const bool out_lane = lane >= LO && lane <= HI && c < nnx;
   const bool col_ok = c >= 0 && c < nnx;
   const bool ecol_ok = c >= 0 && c < nelx;
-  const int r0 = blockIdx.y * kQRows;
-  const int r1 = min(r0 + kQRows, nny);
+  const int band = (nny + gridDim.y - 1) / gridDim.y;  // rows per block (any grid.y)
+  const int r0 = blockIdx.y * band;
+  const int r1 = min(r0 + band, nny);
   struct Front {
     FrontRow<D, T, RD> F;
     T x[D];
@@ -693,36 +740,6 @@ __global__ void __launch_bounds__(kQThreads, sizeof(T) == 4 ? 6 : 3) l0_postsmoo
         pcg_rz_finish(S, t2, rz.first, rz.flexible);
       });
   }
-}
-
-// The launch shapes a solve uses, tunable per hierarchy (stt_hier_tune) and set on the
-// calling host thread for the duration of a solve entry point: pcg_band, the rows a block
-// of the PCG's level-0 passes marches (8, 16 or 32; 0: the heuristic of pcg_tile_grid);
-// waves, the blocks band_rows aims at in units of one block per SM (0: four).
-struct LaunchTuning {
-  int pcg_band = 0;
-  int waves = 0;
-};
-inline LaunchTuning& launch_tuning() {
-  static thread_local LaunchTuning t;
-  return t;
-}
-struct ScopedTuning {
-  LaunchTuning saved;
-  ScopedTuning(int pcg_band, int waves) : saved(launch_tuning()) { launch_tuning() = LaunchTuning{pcg_band, waves}; }
-  ~ScopedTuning() { launch_tuning() = saved; }
-};
-
-// Rows a block marches on the coarse levels: 32 where the grid then fills the GPU,
-// shorter bands on small grids (the heat solve's single row, the coarse levels), whose
-// launches are otherwise latency-bound by the sequential march down 32 rows.  The
-// kernels derive their band from gridDim.y, so any grid.y covers the rows.
-inline int band_rows(int xblocks, int nny, int rows) {
-  const int waves = launch_tuning().waves > 0 ? launch_tuning().waves : 4;
-  const long long target = (long long)waves * 148;  // blocks: waves of one block per B200 SM
-  for (int band = 32; band > 4; band /= 2)
-    if ((long long)xblocks * ((nny + band - 1) / band) * rows >= target) return band;
-  return 4;
 }
 
 inline dim3 coarse_grid(int nelx, int nely, int rows) {
@@ -1561,8 +1578,9 @@ __global__ void __launch_bounds__(kQThreads) l1_sweep_kernel(
 constexpr int kL1ChainCols = 28;
 
 inline dim3 l1_chain_grid(int nelx, int nely, int rows) {
-  const int strips = (nelx + 1 + kL1ChainCols - 1) / kL1ChainCols;
-  return dim3((strips + kQWarps - 1) / kQWarps, (nely + 1 + kQRows - 1) / kQRows, rows);
+  const int strips = (nelx + 1 + kL1ChainCols - 1) / kL1ChainCols, xb = (strips + kQWarps - 1) / kQWarps;
+  const int band = march_band(xb, nely + 1, rows, 4);
+  return dim3(xb, (nely + 1 + band - 1) / band, rows);
 }
 
 // One element-row stage of the level-1 modal operator (l1_sweep_kernel's step).
@@ -1662,8 +1680,9 @@ __global__ void __launch_bounds__(kQThreads, 4) l1_chain_kernel(
   const bool col_ok = c >= 0 && c < nnx;
   const int nelx = nnx - 1, nely = nny - 1;
   const bool ecol_ok = c >= 0 && c < nelx;
-  const int r0 = blockIdx.y * kQRows;
-  const int r1 = min(r0 + kQRows, nny);
+  const int band = (nny + gridDim.y - 1) / gridDim.y;  // rows per block (any grid.y)
+  const int r0 = blockIdx.y * band;
+  const int r1 = min(r0 + band, nny);
   struct Front {
     T b[D], dg[D], x[D], rm[4];
     uint8_t fl;

@@ -49,7 +49,7 @@ static int ew_blocks(long long n) {
 static dim3 tile_grid(int nelx, int nely, int rows) { return q4_grid(nelx, nely, rows); }
 
 // The PCG's level-0 passes (initial residual, p.Ap): bands of 32 grid rows, or shorter
-// ones (down to 8) while the rows give fewer blocks than two waves of six 128-thread
+// ones (down to 4) while the rows give fewer blocks than two waves of six 128-thread
 // blocks on each of the 148 SMs (a single scalar row: the heat solves).  The kernels
 // take the band from the launch (BAND = 0).
 static dim3 pcg_tile_grid(int nelx, int nely, int rows, int min_band = 0) {
@@ -61,7 +61,7 @@ static dim3 pcg_tile_grid(int nelx, int nely, int rows, int min_band = 0) {
   } else if (launch_tuning().pcg_band > 0) {
     band = launch_tuning().pcg_band;
   } else {
-    while (band > 8 && (long long)g.x * ((nny + band - 1) / band) * rows < 2LL * 148 * 6) band /= 2;
+    while (band > 4 && (long long)g.x * ((nny + band - 1) / band) * rows < 2LL * 148 * 6) band /= 2;
   }
   return dim3(g.x, (nny + band - 1) / band, rows);
 }
@@ -110,9 +110,9 @@ static long long plan_solve(const stt_hier* h, int nrows, int gamma, char* base,
   const int es = h->precision == STT_FP32 ? 4 : 8;
   const LevelDesc& l0 = h->lv[0];
   if (pcg) {
-    const dim3 tg = pcg_tile_grid(h->nelx, h->nely, nrows, 8);
+    const dim3 tg = pcg_tile_grid(h->nelx, h->nely, nrows, 4);
     // the level-0 chained passes' blocks may take the r.z reductions
-    const dim3 pg = postsmooth_grid(h->nelx, h->nely, nrows), qg = presmooth_grid(h->nelx, h->nely, nrows);
+    const dim3 pg = postsmooth_grid(h->nelx, h->nely, nrows, es), qg = presmooth_grid(h->nelx, h->nely, nrows, es);
     w.nblk_max = std::max<int>(std::max<int>(tg.x * tg.y, std::max(pg.x * pg.y, qg.x * qg.y)), ew_blocks(l0.ndof));
     w.rs = (RowState*)carve(base, used, sizeof(RowState) * nrows);
     w.partials = (double*)carve(base, used, 8LL * nrows * w.nblk_max * 3);
@@ -303,7 +303,7 @@ struct Cycle {
   void presmooth(const T* b, long long b_rs, T* out_x, T* out_r) {
     const LevelDesc& lv = h->lv[0];
     const long long nd = vstride(lv.ndof);
-    const dim3 g = presmooth_grid(lv.nelx, lv.nely, nrows);
+    const dim3 g = presmooth_grid(lv.nelx, lv.nely, nrows, sizeof(T));
     RzFuse<T> mx = rzf;
     mx.red.nblk = (int)(g.x * g.y);
 #define STT_PRE(RD, MX)                                                                                  \
@@ -378,7 +378,7 @@ struct Cycle {
   void postsmooth(const T* x0, const T* b, long long b_rs, T* out) {
     const LevelDesc& lv = h->lv[0];
     const long long nd = vstride(lv.ndof);
-    const dim3 g = postsmooth_grid(lv.nelx, lv.nely, nrows);
+    const dim3 g = postsmooth_grid(lv.nelx, lv.nely, nrows, sizeof(T));
     RzFuse<T> rz = rzf;
     rz.red.nblk = (int)(g.x * g.y);
     const bool fuse = rzf.rst && (!rzf.zold || mix_done);
@@ -1026,8 +1026,12 @@ static int run_pcg(const stt_hier* h, SolveWS& w, int nrows, const double* b, lo
   // and reduction cost less than with one block per 1024 values)
   const int rzb = (int)std::max<long long>(1, std::min<long long>(ewb, (nd / 4 + 8 * kEwThreads - 1) / (8 * kEwThreads)));
   GridRed red_rz{w.partials, w.counters, rzb};
-  // the r update likewise: eight 128-bit pairs of r and Ap a thread
-  const int upb = (int)std::max<long long>(1, std::min<long long>(ewb, (nd / 2 + 8 * kEwThreads - 1) / (8 * kEwThreads)));
+  // the r update likewise: eight 128-bit pairs of r and Ap a thread, or fewer while that
+  // leaves SMs without a block
+  int per = 8;
+  auto up_blocks = [&]() { return (int)std::max<long long>(1, std::min<long long>(ewb, (nd / 2 + per * kEwThreads - 1) / (per * kEwThreads))); };
+  while (per > 1 && (long long)up_blocks() * nrows < 2 * 148) per /= 2;
+  const int upb = up_blocks();
   GridRed red_up{w.partials, w.counters, upb};
   const KEq<D, double> ke = ke_of<D, double>(h);
   const double* rd0 = h->has_reaction ? l0.rdiag64 : nullptr;

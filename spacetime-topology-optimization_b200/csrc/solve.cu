@@ -4,9 +4,8 @@
 // per-row alpha/beta with safe_div, convergence on ||r|| / ||b|| checked before the
 // first iteration and after every update.  Converged rows stop (every kernel skips
 // rows whose device `active` flag is clear), which is the reference's row retirement
-// without the compaction copies; the host reads the row flags every few iterations
-// instead of syncing on every one.  Reductions are deterministic (block partials
-// summed in block order by the last block).
+// without the compaction copies; the host reads the row flags while the next V-cycle runs.
+// Reductions are deterministic (block partials summed in block order by the last block).
 #include <algorithm>
 #include <cstring>
 #include <mutex>
@@ -1011,6 +1010,84 @@ struct PapEvents {
   }
 };
 
+// What a solve reads its rows' states back with: a copy stream, so that the copy runs beside
+// the V-cycle that follows the update, and page-locked memory.  Pooled (at most kMaxIdle kept
+// idle; a solve on any thread or stream takes one of its device's or makes one).
+struct StateReader {
+  int device = 0, cap = 0;
+  cudaStream_t copy = nullptr;
+  cudaEvent_t updated = nullptr, copied = nullptr;
+  RowState* rows = nullptr;  // [cap], then the hierarchy's status word
+  ~StateReader() {
+    if (rows) cudaFreeHost(rows);
+    if (copied) cudaEventDestroy(copied);
+    if (updated) cudaEventDestroy(updated);
+    if (copy) cudaStreamDestroy(copy);
+  }
+  int* status() const { return reinterpret_cast<int*>(rows + cap); }
+  int reserve(int nrows) {
+    if (nrows <= cap) return STT_OK;
+    if (rows) cudaFreeHost(rows);
+    rows = nullptr;
+    cap = 0;
+    const int n = std::max(nrows, 512);  // few solves have more rows: no second allocation
+    STT_TRY(check_cuda(cudaHostAlloc((void**)&rows, sizeof(RowState) * (n + 1), cudaHostAllocPortable), "row states"));
+    cap = n;
+    return STT_OK;
+  }
+};
+static_assert(sizeof(int) <= sizeof(RowState), "the status word follows the rows");
+
+class StateReaderLease {
+  static constexpr size_t kMaxIdle = 32;
+  static std::mutex& mu() {
+    static std::mutex m;
+    return m;
+  }
+  static std::vector<StateReader*>& idle() {
+    static auto* v = new std::vector<StateReader*>();  // lives as long as the process
+    return *v;
+  }
+  StateReader* r_ = nullptr;
+
+ public:
+  StateReaderLease() = default;
+  StateReaderLease(const StateReaderLease&) = delete;
+  StateReaderLease& operator=(const StateReaderLease&) = delete;
+  StateReader* operator->() const { return r_; }
+  int take(int nrows) {
+    int dev = 0;
+    STT_TRY(check_cuda(cudaGetDevice(&dev), "cudaGetDevice"));
+    {
+      std::lock_guard<std::mutex> lock(mu());
+      for (size_t i = 0; i < idle().size(); ++i)
+        if (idle()[i]->device == dev) {
+          r_ = idle()[i];
+          idle().erase(idle().begin() + (long)i);
+          break;
+        }
+    }
+    if (!r_) {
+      r_ = new StateReader();
+      r_->device = dev;
+      int lo = 0, hi = 0;
+      STT_TRY(check_cuda(cudaDeviceGetStreamPriorityRange(&lo, &hi), "stream priorities"));
+      STT_TRY(check_cuda(cudaStreamCreateWithPriority(&r_->copy, cudaStreamNonBlocking, hi), "copy stream"));
+      STT_TRY(check_cuda(cudaEventCreateWithFlags(&r_->updated, cudaEventDisableTiming), "event"));
+      STT_TRY(check_cuda(cudaEventCreateWithFlags(&r_->copied, cudaEventDisableTiming), "event"));
+    }
+    return r_->reserve(nrows);
+  }
+  ~StateReaderLease() {
+    if (!r_) return;
+    const bool whole = r_->copy && r_->updated && r_->copied;
+    if (whole) cudaStreamSynchronize(r_->copy);  // (an early error return may leave a copy in flight)
+    std::lock_guard<std::mutex> lock(mu());
+    if (whole && idle().size() < kMaxIdle) idle().push_back(r_);
+    else delete r_;
+  }
+};
+
 template <int D, typename T>
 static int run_pcg(const stt_hier* h, SolveWS& w, int nrows, const double* b, long long b_rs,
                    double* x, long long x_rs, int has_x0, double rtol, int max_iter, double omega,
@@ -1073,35 +1150,43 @@ static int run_pcg(const stt_hier* h, SolveWS& w, int nrows, const double* b, lo
   init(has_x0 ? x : nullptr, pp, 0);
   if (sched) launch(pcg_retire_kernel, 1, 32, 0, st, w.rs, nrows, w.sched_last, 0);
   STT_TRY(check_launch("pcg init"));
-  std::vector<RowState> host(nrows);
-  // the reads after the first V-cycle also carry the hierarchy build's status word (the
-  // build does not synchronise, and the coarse factorisation runs on the hierarchy's side
-  // stream, overlapping the initialisation and the first descent): a failed coarse
-  // factorisation surfaces there
-  int hstatus = 0;
+  // The rows' states after a residual: copied on the reader's stream while the caller's goes
+  // on to the V-cycle, and read by the host when that has been enqueued, so the GPU does not
+  // wait for the host between iterations.  The first read after a V-cycle also carries the
+  // hierarchy build's status word (the build does not synchronise, and the coarse
+  // factorisation runs on the hierarchy's side stream): a failed coarse factorisation
+  // surfaces there.
+  StateReaderLease host;
+  STT_TRY(host.take(nrows));
   bool hchecked = false;
-  auto pull = [&](bool with_status) -> int {
-    STT_TRY(check_cuda(cudaMemcpyAsync(host.data(), w.rs, sizeof(RowState) * nrows, cudaMemcpyDeviceToHost, st), "row state"));
-    with_status = with_status && !hchecked;
+  auto fetch = [&](bool with_status) -> int {
+    STT_TRY(check_cuda(cudaEventRecord(host->updated, st), "record states"));
+    STT_TRY(check_cuda(cudaStreamWaitEvent(host->copy, host->updated, 0), "wait states"));
     if (with_status) {
-      STT_TRY(check_cuda(cudaStreamWaitEvent(st, h->sync->ready, 0), "wait coarse"));
-      STT_TRY(check_cuda(cudaMemcpyAsync(&hstatus, h->status, sizeof(int), cudaMemcpyDeviceToHost, st), "status copy"));
+      STT_TRY(check_cuda(cudaStreamWaitEvent(host->copy, h->sync->ready, 0), "wait coarse"));
+      STT_TRY(check_cuda(cudaMemcpyAsync(host->status(), h->status, sizeof(int), cudaMemcpyDeviceToHost, host->copy),
+                         "status copy"));
     }
-    STT_TRY(check_cuda(cudaStreamSynchronize(st), "pcg sync"));
-    if (with_status) {
-      hchecked = true;
-      STT_TRY(hier_status_code(hstatus));
-    }
+    STT_TRY(check_cuda(cudaMemcpyAsync(host->rows, w.rs, sizeof(RowState) * nrows, cudaMemcpyDeviceToHost, host->copy),
+                       "row state"));
+    return check_cuda(cudaEventRecord(host->copied, host->copy), "record copy");
+  };
+  auto arrive = [&](bool with_status) -> int {
+    STT_TRY(check_cuda(cudaEventSynchronize(host->copied), "pcg sync"));
+    if (with_status) STT_TRY(hier_status_code(*host->status()));
     return STT_OK;
   };
   auto n_active = [&]() {
     int a = 0;
-    for (auto& s : host) a += s.active;
+    for (int s = 0; s < nrows; ++s) a += host->rows[s].active;
     return a;
   };
-  STT_TRY(pull(false));
+  // a warm start often converges at once (the adjoints' alpha U): look before the first
+  // V-cycle; from x = 0 only a zero right-hand side does, and the V-cycle skips its rows
+  STT_TRY(fetch(false));
+  if (has_x0) STT_TRY(arrive(false));
   int it = 0;
-  if (n_active() > 0) {
+  if (!has_x0 || n_active() > 0) {
     T* z = (T*)w.z;
     T* zold = (T*)w.zold;
     double* pcur = w.p;    // p of the previous iteration
@@ -1143,8 +1228,10 @@ static int run_pcg(const stt_hier* h, SolveWS& w, int nrows, const double* b, lo
                                r32init != nullptr && !has_x0, &f, &done));
       if (!done) rz(1);
     }
-    int check_every = 1;
-    for (it = 1; it <= max_iter; ++it) {
+    STT_TRY(check_launch("pcg start"));
+    if (!has_x0) STT_TRY(arrive(false));
+    const bool any = n_active() > 0;
+    for (it = 1; any && it <= max_iter; ++it) {
       pp.it = it;
 #define STT_PAP(MODAL, RD, PM, XP)                                                                         \
   launch((pcg_pap_kernel<D, MODAL, RD, T, PM, XP>), tg, kQThreads, 0, st,                                        \
@@ -1184,6 +1271,8 @@ static int run_pcg(const stt_hier* h, SolveWS& w, int nrows, const double* b, lo
         pending = false;
         init(x, pp, 1);
       }
+      const bool check_status = !hchecked;
+      STT_TRY(fetch(check_status));
       if (flexible) std::swap(z, zold);
       {
         const RzFuse<T> f = fuse_of(0);
@@ -1193,25 +1282,24 @@ static int run_pcg(const stt_hier* h, SolveWS& w, int nrows, const double* b, lo
         if (!done) rz(0);
       }
       STT_TRY(check_launch("pcg iteration"));
-      if (it % check_every == 0 || it == max_iter) {
-        STT_TRY(pull(true));
-        if (n_active() == 0) break;
-        // a wider check interval once the solve is evidently long
-        if (it >= 8) check_every = 2;
-        if (it >= 32) check_every = 4;
-      }
+      STT_TRY(arrive(check_status));
+      hchecked = true;
+      if (n_active() == 0) break;
     }
     flush_x();
     STT_TRY(check_launch("pcg flush"));
   }
-  STT_TRY(pull(true));
+  STT_TRY(fetch(!hchecked));
+  STT_TRY(check_cuda(cudaStreamSynchronize(st), "pcg sync"));
+  STT_TRY(arrive(!hchecked));
   if (timing) pev.flush();
   int worst = 0, status = STT_OK;
   for (int s = 0; s < nrows; ++s) {
-    rel_out[s] = host[s].rel;
-    conv_out[s] = host[s].active ? -1 : host[s].conv_iter;
-    worst = std::max(worst, host[s].conv_iter);
-    if (host[s].active) status = STT_ERR_NOT_CONVERGED;
+    const RowState& S = host->rows[s];
+    rel_out[s] = S.rel;
+    conv_out[s] = S.active ? -1 : S.conv_iter;
+    worst = std::max(worst, S.conv_iter);
+    if (S.active) status = STT_ERR_NOT_CONVERGED;
   }
   *n_iter_out = status == STT_OK ? worst : max_iter;
   if (status != STT_OK)

@@ -9,13 +9,15 @@
 // approximation P, Q (m x n) is never stored: each pass rebuilds P_ij, Q_ij from dfdx_ij
 // and three per-variable numbers, so a pass reads one m x n array instead of two.
 //
-// One Newton step is three passes over the variables: assemble (the residual at the
-// current point, the Newton right-hand side and the m x m matrix GG diag(1/diagx) GG^T,
-// formed on the FP64 tensor cores from a shared-memory tile of GG), step (dx and the
-// fraction-to-the-boundary limits) and one search pass per line-search candidate.  The
-// accepted step is applied by the next pass's prologue.  Reductions are deterministic:
-// one partial a block, folded in block order (by the step and search passes' last block,
-// and for the assemble pass's larger product by a separate fold kernel).
+// One Newton step is two passes over the variables: step (dx and the
+// fraction-to-the-boundary limits) and advance (the line search's first candidate: its
+// residual, and there already the next Newton step's right-hand side and m x m matrix
+// GG diag(1/diagx) GG^T, formed on the FP64 tensor cores from a shared-memory tile of GG,
+// for this barrier level and for the next one).  Nearly every first candidate is accepted;
+// a rejected one costs a search pass a further candidate and an assemble pass (advance
+// without a candidate) that applies the accepted step.  Reductions are deterministic: one
+// partial a block, folded in block order (by the step and search passes' last block, and
+// for the larger product by a separate fold kernel).
 //
 // The file is compiled with -fmad=false, so that a * b + c rounds twice as in the
 // reference's tensor arithmetic; the dot products use fma() explicitly.
@@ -439,28 +441,31 @@ STT_DEV void dmma_f64(double (&d)[2], double a, double b) {
                : "d"(a), "d"(b));
 }
 
-// Upper-triangular 8 x 8 tiles (I <= K) of the (m + 1) x (m + 1) product, t8 a side.
-__host__ __device__ inline int gram_side(int m) { return (m + 8) >> 3; }
-__host__ __device__ inline int gram_tiles(int m) { return gram_side(m) * (gram_side(m) + 1) / 2; }
+// Upper-triangular 8 x 8 tiles (I <= K) of the product of the m rows of GG and nd rows of
+// delx (one barrier level, or two), t8 a side.
+__host__ __device__ inline int gram_side(int m, int nd) { return (m + nd + 7) >> 3; }
+__host__ __device__ inline int gram_tiles(int m, int nd) { return gram_side(m, nd) * (gram_side(m, nd) + 1) / 2; }
 __host__ __device__ inline int tile_index(int I, int K, int t8) { return I * t8 - I * (I - 1) / 2 + (K - I); }
-// The product's upper triangle (i <= k <= m, row m being delx), packed row by row.
+// The product's upper triangle (i <= k < m1, rows m and up being delx), packed row by row.
 __host__ __device__ inline int packed_index(int i, int k, int m1) { return i * m1 - i * (i - 1) / 2 + (k - i); }
-// Partial entries of the assemble pass: [gvec (m) | sum of squares | packed product | max].
-__host__ __device__ inline int assemble_kp(int m) { return m + 2 + (m + 1) * (m + 2) / 2; }
+// Partial entries: [gvec (m) | sums of squares (nd) | packed product | maxima (nd)].
+__host__ __device__ inline int assemble_kp(int m, int nd) { return m + 2 * nd + (m + nd) * (m + nd + 1) / 2; }
+// Results: [gvec (m) | A (m x m) | then for each level h (m), sum of squares, max].
+__host__ __device__ inline int assemble_res(int m, int nd) { return m + m * m + nd * (m + 2); }
 // Its dynamic shared memory: the GG tile (or, later, the folded entries), 1/diagx, a
 // block-sum scratch, and when it forms gvec the row-sum slots or shuffle scratch.
-inline size_t assemble_smem(int m, int mb, bool need_g) {
-  const size_t rows = (size_t)gram_side(m) * 8;
+inline size_t assemble_smem(int m, int mb, int nd, bool need_g) {
+  const size_t rows = (size_t)gram_side(m, nd) * 8;
   const size_t tail = !need_g ? 0 : mb <= 24 ? (size_t)mb * kMmaThreads : (size_t)(kMmaThreads / 32) * kMmaMaxM;
-  return 8 * (std::max(rows * kMmaLd8, (size_t)assemble_kp(m)) + kMmaThreads + 8 + tail);
+  return 8 * (std::max(rows * kMmaLd8, (size_t)assemble_kp(m, nd)) + kMmaThreads + 8 + tail);
 }
 inline int mma_bucket(int m) {
   return m <= 4 ? 4 : m <= 8 ? 8 : m <= 12 ? 12 : m <= 16 ? 16 : m <= 20 ? 20 : m <= 24 ? 24 : m <= 32 ? 32
          : m <= 48 ? 48 : 64;
 }
 
-// The assemble pass (sttopt/mma.py:399-489, m < n): applies a pending accepted step,
-// then at the point (x, lam, xsi, eta) and barrier epsi forms, over all variables,
+// The assemble pass (sttopt/mma.py:399-489, m < n): applies a pending accepted step, then
+// at the point (x, lam, xsi, eta) and barrier epsi forms, over all variables,
 //   gvec = P (1/ux1) + Q (1/xl1),  h = GG (delx / diagx),  A = GG diag(1/diagx) GG^T
 // with GG = P diag(1/ux2) - Q diag(1/xl2), and the sum of squares and largest magnitude
 // of the residual's n-sized parts.  A block's 256 variables write their GG column and
@@ -469,19 +474,35 @@ inline int mma_bucket(int m) {
 // warps' sums are folded in warp order; above that the tiles are split among the warps.
 // gvec is formed only with need_g: after a line search it is the accepted candidate's,
 // which the search pass formed at this same point.
-// res = [gvec (m), or zeros | h (m) | A (m x m) | sum of squares | max].
-template <int MB, bool G>
+//
+// ADV, the advance pass: the pending step is the line search's first candidate, of length
+// *tdev (the step pass's steg) and multipliers lam + t dlam; the point goes to xo, xsio,
+// etao (the old one stays, should the candidate be rejected), gvec is formed, and h and the
+// residual's parts also for the next barrier level, 0.1 epsi.  It replaces a search pass and
+// an assemble pass over the same data: at 4.2M variables and 17 constraints 205 + 314 us
+// became 343 us, and one host synchronisation of two went.
+template <int MB, bool G, bool ADV>
 __global__ void __launch_bounds__(kMmaThreads, 2) mma_assemble_kernel(
-    MmaCols c, double* __restrict__ x, double* __restrict__ xsi, double* __restrict__ eta,
-    const double* __restrict__ dx, int pend, double t_pend, double eps_pend, MVec lam, double epsi, int need_g,
-    double* __restrict__ partials) {
+    MmaCols c, const double* x, const double* xsi, const double* eta, double* xo, double* xsio, double* etao,
+    const double* __restrict__ dx, int pend, double t_pend, const double* tdev, double eps_pend, MVec lam0, MVec dlam,
+    double epsi, int need_g_arg, double* __restrict__ partials) {
+  grid_wait();
+  constexpr int ND = ADV ? 2 : 1;
+  const bool need_g = ADV || need_g_arg;
+  __shared__ MVec lam_s;  // the candidate's multipliers, as the host forms them
+  if constexpr (ADV) {
+    t_pend = *tdev;
+    for (int i = threadIdx.x; i < c.m; i += kMmaThreads) lam_s.v[i] = lam0.v[i] + t_pend * dlam.v[i];
+    __syncthreads();
+  }
+  auto lam = [&](int i) { return ADV ? lam_s.v[i] : lam0.v[i]; };
   extern __shared__ double sm[];
-  constexpr int T8 = (MB + 8) / 8;  // tile side for the largest m of the bucket
+  constexpr int T8 = (MB + ND + 7) / 8;  // tile side for the largest m of the bucket
   constexpr int NT = T8 * (T8 + 1) / 2;
   constexpr bool KSPLIT = T8 <= 4;
   constexpr int TPW = KSPLIT ? NT : (NT + 7) / 8;  // tiles a warp accumulates
-  const int m = c.m, t8 = gram_side(m), rows = t8 * 8, ntile = gram_tiles(m);
-  const int head = max(rows * kMmaLd8, assemble_kp(m));
+  const int m = c.m, t8 = gram_side(m, ND), rows = t8 * 8, ntile = gram_tiles(m, ND);
+  const int head = max(rows * kMmaLd8, assemble_kp(m, ND));
   double* gs = sm;                 // [rows][kMmaLd8]
   double* ws = sm + head;          // [kMmaThreads]: 1 / diagx
   double* wred = ws + kMmaThreads; // [8]
@@ -496,8 +517,10 @@ __global__ void __launch_bounds__(kMmaThreads, 2) mma_assemble_kernel(
     if constexpr (use_slots<MB>()) gv.slots = tail;
     gv.zero();
   }
-  double ss = 0.0, mx = 0.0;
-  for (int r = m + 1; r < rows; ++r) gs[r * kMmaLd8 + tid] = 0.0;
+  double ss[ND], mx[ND];
+#pragma unroll
+  for (int e = 0; e < ND; ++e) ss[e] = mx[e] = 0.0;
+  for (int r = m + ND; r < rows; ++r) gs[r * kMmaLd8 + tid] = 0.0;
 
   const long long ntiles = (c.n + kMmaThreads - 1) / kMmaThreads;
   for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
@@ -511,11 +534,11 @@ __global__ void __launch_bounds__(kMmaThreads, 2) mma_assemble_kernel(
       double xv = x[j];
       xs = xsi[j];
       et = eta[j];
-      if (pend) {
+      if (ADV || pend) {
         step_point(xv, xs, et, dx[j], t_pend, eps_pend, f.alfa, f.beta);
-        x[j] = xv;
-        xsi[j] = xs;
-        eta[j] = et;
+        xo[j] = xv;
+        xsio[j] = xs;
+        etao[j] = et;
       }
       p = point_of(f, xv);
     }
@@ -538,24 +561,31 @@ __global__ void __launch_bounds__(kMmaThreads, 2) mma_assemble_kernel(
           if (i < m) {
             double p1, q1;
             rows_pq1<G>(f, ra[u], rb[u], p1, q1);
-            lp = fma(lam.v[i], p1, lp);
-            lq = fma(lam.v[i], q1, lq);
+            lp = fma(lam(i), p1, lp);
+            lq = fma(lam(i), q1, lq);
             if (need_g) gv.add(i, fma(p1, k.A, q1 * k.B));
             gs[i * kMmaLd8 + tid] = fma(p1, k.C, -(q1 * k.D));
           }
         }
       }
     }
-    double w = 0.0, delx = 0.0;
+    double w = 0.0, delx[ND];
+#pragma unroll
+    for (int e = 0; e < ND; ++e) delx[e] = 0.0;
     if (ok) {
       const double plam = f.p0 + f.sp * lp;
       const double qlam = f.q0 + f.sq * lq;
-      resid_n(plam, qlam, p, xs, et, epsi, ss, mx);
       double diagx;
-      newton_col(plam, qlam, p, xs, et, epsi, delx, diagx);
+#pragma unroll
+      for (int e = 0; e < ND; ++e) {
+        const double ep = e == 0 ? epsi : 0.1 * epsi;
+        resid_n(plam, qlam, p, xs, et, ep, ss[e], mx[e]);
+        newton_col(plam, qlam, p, xs, et, ep, delx[e], diagx);
+      }
       w = 1.0 / diagx;
     }
-    gs[m * kMmaLd8 + tid] = delx;
+#pragma unroll
+    for (int e = 0; e < ND; ++e) gs[(m + e) * kMmaLd8 + tid] = delx[e];
     ws[tid] = w;
     // Up to 31 constraints a warp's tiles read only the 32 variables the warp wrote, so
     // the warps need not wait for one another.
@@ -608,9 +638,9 @@ __global__ void __launch_bounds__(kMmaThreads, 2) mma_assemble_kernel(
     }
   }
 
-  // Product partials: entry m + 1 + packed_index(i, k) holds (i, k), i <= k <= m; tile
+  // Product partials: entry m + ND + packed_index(i, k) holds (i, k), i <= k < m + ND; tile
   // t = (I, K) holds (8 I + r, 8 K + c) at r * 8 + c.
-  const int m1 = m + 1;
+  const int m1 = m + ND;
   if constexpr (KSPLIT) {
     __syncthreads();    // every warp's tiles are done before the tile memory is reused
     double* red8 = sm;  // [8 warps][ntile][64]
@@ -631,7 +661,7 @@ __global__ void __launch_bounds__(kMmaThreads, 2) mma_assemble_kernel(
       const size_t at = (size_t)tile_index(i >> 3, k >> 3, t8) * 64 + (i & 7) * 8 + (k & 7);
       double t = 0.0;
       for (int w8 = 0; w8 < kMmaThreads / 32; ++w8) t += red8[(size_t)w8 * ntile * 64 + at];
-      *part(partials, m + 1 + packed_index(i, k, m1)) = t;
+      *part(partials, m + ND + packed_index(i, k, m1)) = t;
     }
   } else {
 #pragma unroll
@@ -647,51 +677,57 @@ __global__ void __launch_bounds__(kMmaThreads, 2) mma_assemble_kernel(
 #pragma unroll
         for (int v = 0; v < 2; ++v) {
           const int i = 8 * I + fr, k = 8 * K + fc * 2 + v;
-          if (i <= k && k <= m) *part(partials, m + 1 + packed_index(i, k, m1)) = acc[q][v];
+          if (i <= k && k < m1) *part(partials, m + ND + packed_index(i, k, m1)) = acc[q][v];
         }
       }
     }
   }
-  const int ks = assemble_kp(m) - 1;
+  const int ks = assemble_kp(m, ND) - ND;
   if (need_g) {
     gv.write(m, partials, 0, tail);
   } else {
     for (int i = tid; i < m; i += kMmaThreads) *part(partials, i) = 0.0;
   }
-  const double t = block_total(ss, wred);
-  if (tid == 0) *part(partials, m) = t;
-  const double u = block_nanmax(mx, wred);
-  if (tid == 0) *part(partials, ks) = u;
+#pragma unroll
+  for (int e = 0; e < ND; ++e) {
+    const double t = block_total(ss[e], wred);
+    if (tid == 0) *part(partials, m + e) = t;
+    const double u = block_nanmax(mx[e], wred);
+    if (tid == 0) *part(partials, ks + e) = u;
+  }
 }
 
-// Folds the assemble pass's block partials (entry-major, nb blocks) in block order, a
-// warp an entry on as many SMs as there are entries / 8, and writes
-// res = [gvec (m) | h (m) | A (m x m) | sum of squares | max].
+// Folds the assemble (nd = 1) or advance (nd = 2) pass's block partials (entry-major, nb
+// blocks) in block order, a warp an entry on as many SMs as there are entries / 8, into the
+// results (assemble_res).
 __global__ void __launch_bounds__(kMmaThreads) mma_fold_kernel(const double* __restrict__ partials, int nb, int m,
-                                                               double* __restrict__ res) {
-  const int kp = assemble_kp(m), ks = kp - 1, m1 = m + 1, lane = threadIdx.x & 31;
+                                                               int nd, double* __restrict__ res) {
+  grid_wait();
+  const int kp = assemble_kp(m, nd), ks = kp - nd, m1 = m + nd, lane = threadIdx.x & 31;
   const int e = blockIdx.x * (kMmaThreads / 32) + (threadIdx.x >> 5);
   if (e >= kp) return;
   const double t = fold_entry(partials + (size_t)e * nb, nb, e < ks, lane);
   if (lane != 0) return;
+  double* const A = res + m;
+  auto level = [&](int q) { return A + m * m + q * (m + 2); };  // h (m), sum of squares, max
   if (e < m) {
     res[e] = t;
-  } else if (e == m) {
-    res[2 * m + m * m] = t;
-  } else if (e == ks) {
-    res[2 * m + m * m + 1] = t;
+  } else if (e < m + nd) {
+    level(e - m)[m] = t;
+  } else if (e >= ks) {
+    level(e - ks)[m + 1] = t;
   } else {
-    int i = 0, pe = e - m - 1;
+    int i = 0, pe = e - m - nd;
     while (pe >= m1 - i) {
       pe -= m1 - i;
       ++i;
     }
     const int k = i + pe;
-    if (k == m) {
-      if (i < m) res[m + i] = t;  // (m, m), delx' diag(1/diagx) delx, is not needed
+    if (k >= m) {
+      if (i < m) level(k - m)[i] = t;  // (the products of delx rows are not needed)
     } else {
-      res[2 * m + i * m + k] = t;
-      res[2 * m + k * m + i] = t;
+      A[i * m + k] = t;
+      A[k * m + i] = t;
     }
   }
 }
@@ -707,6 +743,7 @@ __global__ void __launch_bounds__(kMmaThreads, 3) mma_step_kernel(
     MmaCols c, const double* __restrict__ x, const double* __restrict__ xsi, const double* __restrict__ eta,
     MVec lam, MVec dlam, double epsi, double stm_host, double* __restrict__ dx, double* __restrict__ partials,
     unsigned* __restrict__ counter, double* __restrict__ res) {
+  grid_wait();
   __shared__ double red[kMmaThreads / 32];
   __shared__ double fin[3];
   const int m = c.m;
@@ -775,6 +812,7 @@ __global__ void __launch_bounds__(kMmaThreads, 3) mma_search_kernel(
     MmaCols c, const double* __restrict__ x, const double* __restrict__ xsi, const double* __restrict__ eta,
     const double* __restrict__ dx, double t_arg, const double* tdev, MVec lam0, MVec dlam, double epsi, int resid,
     double* __restrict__ partials, unsigned* __restrict__ counter, double* __restrict__ res) {
+  grid_wait();
   __shared__ double red[kMmaThreads / 32 * (kMmaMaxM + 1)];
   __shared__ double fin[kMmaMaxM + 2];
   __shared__ MVec lam;  // the candidate's multipliers, lam0 + t dlam as the host forms them
@@ -853,20 +891,21 @@ static_assert(kAsmBlocks <= 32 * kFoldMax && kPassBlocks <= 32 * kFoldMax, "a fo
 constexpr int kMaxHalvings = 50;   // sttopt/mma.py:289
 constexpr int kMaxNewton = 200;    // sttopt/mma.py:442
 
-using AsmFn = void (*)(MmaCols, double*, double*, double*, const double*, int, double, double, MVec, double, int,
-                       double*);
+using AsmFn = void (*)(MmaCols, const double*, const double*, const double*, double*, double*, double*, const double*,
+                       int, double, const double*, double, MVec, MVec, double, int, double*);
 using StepFn = void (*)(MmaCols, const double*, const double*, const double*, MVec, MVec, double, double, double*,
                         double*, unsigned*, double*);
 using SearchFn = void (*)(MmaCols, const double*, const double*, const double*, const double*, double, const double*,
                           MVec, MVec, double, int, double*, unsigned*, double*);
 struct Kernels {
-  AsmFn assemble;
+  AsmFn assemble, advance;
   StepFn step;
   SearchFn search;
 };
 template <int MB, bool G>
 Kernels kernels_of() {
-  return {mma_assemble_kernel<MB, G>, mma_step_kernel<MB, G>, mma_search_kernel<MB, G>};
+  return {mma_assemble_kernel<MB, G, false>, mma_assemble_kernel<MB, G, true>, mma_step_kernel<MB, G>,
+          mma_search_kernel<MB, G>};
 }
 template <bool G>
 Kernels pick_kernels(int m) {
@@ -883,14 +922,15 @@ Kernels pick_kernels(int m) {
   }
 }
 
-// Workspace: [alfa | beta | rxm | dx] (n each), block partials, results, counters.
+// Workspace: [alfa | beta | rxm | dx | x, xsi, eta of the candidate] (n each), block
+// partials, results, counters.
 struct MmaWs {
-  double *alfa, *beta, *rxm, *dx, *partials, *res;
+  double *alfa, *beta, *rxm, *dx, *x2, *xsi2, *eta2, *partials, *res;
   unsigned* counters;
 };
 size_t round256(size_t b) { return (b + 255) & ~(size_t)255; }
 size_t partial_doubles(int m) {
-  return std::max({(size_t)kAsmBlocks * assemble_kp(m), (size_t)kPassBlocks * (m + 2), (size_t)kPassBlocks * 3});
+  return std::max({(size_t)kAsmBlocks * assemble_kp(m, 2), (size_t)kPassBlocks * (m + 2), (size_t)kPassBlocks * 3});
 }
 size_t carve(int m, long long n, char* base, MmaWs* w) {
   size_t off = 0;
@@ -899,12 +939,12 @@ size_t carve(int m, long long n, char* base, MmaWs* w) {
     off += round256(bytes);
     return p;
   };
-  double* v[4];
+  double* v[7];
   for (auto& p : v) p = reinterpret_cast<double*>(take(8 * (size_t)n));
   double* parts = reinterpret_cast<double*>(take(8 * partial_doubles(m)));
-  double* res = reinterpret_cast<double*>(take(8 * ((size_t)m * m + 2 * m + 8)));
+  double* res = reinterpret_cast<double*>(take(8 * ((size_t)assemble_res(m, 2) + 8)));
   unsigned* cnt = reinterpret_cast<unsigned*>(take(4 * sizeof(unsigned)));
-  if (w) *w = {v[0], v[1], v[2], v[3], parts, res, cnt};
+  if (w) *w = {v[0], v[1], v[2], v[3], v[4], v[5], v[6], parts, res, cnt};
   return off;
 }
 
@@ -1076,22 +1116,43 @@ int device_subsolv(const MmaCols& c, const MData& D, double epsimin, const MmaWs
   const long long tiles = (c.n + kMmaThreads - 1) / kMmaThreads;
   const int ga = (int)std::min<long long>(tiles, kAsmBlocks), gp = (int)std::min<long long>(tiles, kPassBlocks);
   const Kernels k = pick_kernels<G>(m);
-  const size_t smem_g = assemble_smem(m, mma_bucket(m), true), smem = assemble_smem(m, mma_bucket(m), false);
+  const int mb = mma_bucket(m);
+  const size_t smem_g = assemble_smem(m, mb, 1, true), smem = assemble_smem(m, mb, 1, false);
+  const size_t smem_adv = assemble_smem(m, mb, 2, true);
   STT_TRY(check_cuda(cudaFuncSetAttribute((const void*)k.assemble, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)smem_g),
                      "mma: assemble shared memory"));
+  STT_TRY(check_cuda(cudaFuncSetAttribute((const void*)k.advance, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)smem_adv),
+                     "mma: advance shared memory"));
   STT_TRY(check_cuda(cudaMemsetAsync(w.counters, 0, 4 * sizeof(unsigned), st), "mma: counters"));
   mma_init_kernel<<<gp, kMmaThreads, 0, st>>>(c.n, c.alfa, c.beta, x, xsi, eta);
   STT_TRY(check_launch("mma_init_kernel"));
   init_state(D, S);
 
-  // results of one fetch: the assemble's [gvec | h | A | ss | mx] or the search's
-  // [gvec | ss | mx] with the step's [3 maxima | steg] behind it
-  const size_t nres = (size_t)m * m + 2 * m + 2;
-  std::vector<double> R(std::max(nres, (size_t)m + 6)), gvec(m), h(m), A((size_t)m * m);
+  // the point (x, xsi, eta): in the caller's arrays or, after an odd number of accepted
+  // first candidates, in the workspace's
+  double *px = x, *pxsi = xsi, *peta = eta, *qx = w.x2, *qxsi = w.xsi2, *qeta = w.eta2;
+  // results of one fetch: the assemble's or advance's, or a search's [gvec | ss | mx]; the
+  // step's [3 maxima | steg] sit behind the advance's
+  const size_t step_at = assemble_res(m, 2);
+  double* const res_step = w.res + step_at;
+  std::vector<double> R(step_at + 4), gvec(m), h(m), A((size_t)m * m);
   auto fetch = [&](size_t count, const char* what) -> int {
     STT_TRY(check_cuda(cudaMemcpyAsync(R.data(), w.res, 8 * count, cudaMemcpyDeviceToHost, st), what));
     return check_cuda(cudaStreamSynchronize(st), what);
+  };
+  auto fold = [&](int nd) -> int {
+    const int kp = assemble_kp(m, nd), per = kMmaThreads / 32;
+    launch(mma_fold_kernel, (kp + per - 1) / per, kMmaThreads, 0, st, w.partials, ga, m, nd, w.res);
+    return check_launch("mma_fold_kernel");
+  };
+  // h, sum of squares and max of level q (0: the pass's epsi, 1: 0.1 epsi) of the fetched results
+  auto level = [&](int q, double& ssn, double& mxn) {
+    const double* L = R.data() + m + (size_t)m * m + (size_t)q * (m + 2);
+    std::copy(L, L + m, h.begin());
+    ssn = L[m];
+    mxn = ssn != ssn ? NAN : L[m + 1];
   };
   int pend = 0;
   double t_pend = 0.0, eps_pend = 0.0;
@@ -1100,32 +1161,31 @@ int device_subsolv(const MmaCols& c, const MData& D, double epsimin, const MmaWs
   bool have_g = false;
   auto assemble = [&](double epsi, double& ssn, double& mxn) -> int {
     const int need_g = have_g ? 0 : 1;
-    k.assemble<<<ga, kMmaThreads, need_g ? smem_g : smem, st>>>(c, x, xsi, eta, w.dx, pend, t_pend, eps_pend,
-                                                                mvec(S.lam), epsi, need_g, w.partials);
+    launch(k.assemble, ga, kMmaThreads, need_g ? smem_g : smem, st, c, px, pxsi, peta, px, pxsi, peta, w.dx, pend,
+           t_pend, nullptr, eps_pend, mvec(S.lam), MVec{}, epsi, need_g, w.partials);
     pend = 0;
     STT_TRY(check_launch("mma_assemble_kernel"));
-    const int kp = assemble_kp(m), per = kMmaThreads / 32;
-    mma_fold_kernel<<<(kp + per - 1) / per, kMmaThreads, 0, st>>>(w.partials, ga, m, w.res);
-    STT_TRY(check_launch("mma_fold_kernel"));
-    STT_TRY(fetch(nres, "mma: assemble"));
+    STT_TRY(fold(1));
+    STT_TRY(fetch(assemble_res(m, 1), "mma: assemble"));
     if (!have_g) std::copy(R.begin(), R.begin() + m, gvec.begin());
     have_g = true;
-    std::copy(R.begin() + m, R.begin() + 2 * m, h.begin());
-    std::copy(R.begin() + 2 * m, R.begin() + 2 * m + (size_t)m * m, A.begin());
-    ssn = R[nres - 2];
-    mxn = ssn != ssn ? NAN : R[nres - 1];
+    std::copy(R.begin() + m, R.begin() + m + (size_t)m * m, A.begin());
+    level(0, ssn, mxn);
     return STT_OK;
   };
 
   double epsi = 1.0;
+  double ready = 0.0;  // the next level's epsi when the last pass was an accepted advance (its results are in R)
   while (epsi > epsimin) {
     double ssn, mxn;
-    STT_TRY(assemble(epsi, ssn, mxn));
+    if (ready == epsi) level(1, ssn, mxn);
+    else STT_TRY(assemble(epsi, ssn, mxn));
+    ready = 0.0;
     double ssm = 0.0, mxm = -INFINITY;
     resid_m(D, S, gvec.data(), epsi, ssm, mxm);
     double residunorm = std::sqrt(ssn + ssm), residumax = hmax(mxn, mxm);
     int ittt = 0;
-    bool fresh = true;
+    bool fresh = true;  // h and A are those of the current point and epsi
     while (residumax > 0.9 * epsi && ittt < kMaxNewton) {
       ++ittt;
       ++cap.steps;
@@ -1150,44 +1210,59 @@ int device_subsolv(const MmaCols& c, const MData& D, double epsimin, const MmaWs
       T.dlam.assign(bb.begin(), bb.begin() + m);
       T.dz = bb[m];
       // The step pass forms steg on the device and the line search's first candidate
-      // (t = steg) is evaluated right behind it: one sync for both.  The step's results sit
-      // behind the search's in res: [search (m + 2) | step maxima (3) | steg].
+      // (t = steg) is evaluated right behind it by the advance pass: one sync for both and
+      // for the next Newton step's matrix.
       const double stm_m = step_m(D, S, N, epsi, T);
       const MVec lam_now = mvec(S.lam), dlam = mvec(T.dlam);
-      double* const res_step = w.res + m + 2;
-      k.step<<<gp, kMmaThreads, 0, st>>>(c, x, xsi, eta, lam_now, dlam, epsi, stm_m, w.dx, w.partials,
-                                         w.counters + 1, res_step);
+      launch(k.step, gp, kMmaThreads, 0, st, c, px, pxsi, peta, lam_now, dlam, epsi, stm_m, w.dx, w.partials,
+             w.counters + 1, res_step);
       STT_TRY(check_launch("mma_step_kernel"));
-      k.search<<<gp, kMmaThreads, 0, st>>>(c, x, xsi, eta, w.dx, 0.0, res_step + 3, lam_now, dlam, epsi, 1,
-                                           w.partials, w.counters + 2, w.res);
-      STT_TRY(check_launch("mma_search_kernel"));
-      STT_TRY(fetch((size_t)m + 6, "mma: step and first candidate"));
-      const double steg = R[m + 5];  // 1 / max(stmalfa, stmbeta, stmxx, 1), as formed on the device
+      launch(k.advance, ga, kMmaThreads, smem_adv, st, c, px, pxsi, peta, qx, qxsi, qeta, w.dx, 1, 0.0, res_step + 3,
+             epsi, lam_now, dlam, epsi, 1, w.partials);
+      STT_TRY(check_launch("mma_assemble_kernel"));
+      STT_TRY(fold(2));
+      STT_TRY(fetch(step_at + 4, "mma: step and first candidate"));
+      const double steg = R[step_at + 3];  // 1 / max(stmalfa, stmbeta, stmxx, 1), as formed on the device
       // Backtracking on the residual norm: the first halving whose norm does not exceed
       // the current one, else the last (sttopt/mma.py:297-343).
-      MState C;
-      double resinew = 0.0, mxc = 0.0, t = 0.0;
-      for (int jj = 0; jj < kMaxHalvings; ++jj) {
-        t = steg / std::ldexp(1.0, jj);
-        C = moved(S, T, t);
-        ++cap.tries;
-        if (jj > 0) {
-          k.search<<<gp, kMmaThreads, 0, st>>>(c, x, xsi, eta, w.dx, t, nullptr, lam_now, dlam, epsi, 1, w.partials,
-                                               w.counters + 2, w.res);
-          STT_TRY(check_launch("mma_search_kernel"));
-          STT_TRY(fetch((size_t)m + 2, "mma: line search"));
-        }
-        double ssc = R[m], mxcn = ssc != ssc ? NAN : R[m + 1], ssmc = 0.0, mxmc = -INFINITY;
+      MState C = moved(S, T, steg);
+      double resinew = 0.0, mxc = 0.0, t = steg;
+      auto judge = [&](double ssc, double mxs) {
+        double ssmc = 0.0, mxmc = -INFINITY;
         resid_m(D, C, R.data(), epsi, ssmc, mxmc);
         resinew = std::sqrt(ssc + ssmc);
-        mxc = hmax(mxcn, mxmc);
-        if (!(resinew > residunorm)) break;
+        mxc = hmax(ssc != ssc ? NAN : mxs, mxmc);
+        return !(resinew > residunorm);
+      };
+      const double* L0 = R.data() + m + (size_t)m * m;
+      ++cap.tries;
+      if (judge(L0[m], L0[m + 1])) {  // the first candidate: its pass has formed the next step's system
+        std::copy(R.begin(), R.begin() + m, gvec.begin());
+        std::copy(R.begin() + m, R.begin() + m + (size_t)m * m, A.begin());
+        level(0, ssn, mxn);
+        std::swap(px, qx);
+        std::swap(pxsi, qxsi);
+        std::swap(peta, qeta);
+        fresh = true;
+        ready = 0.1 * epsi;
+      } else {
+        for (int jj = 1; jj < kMaxHalvings; ++jj) {
+          t = steg / std::ldexp(1.0, jj);
+          C = moved(S, T, t);
+          ++cap.tries;
+          launch(k.search, gp, kMmaThreads, 0, st, c, px, pxsi, peta, w.dx, t, nullptr, lam_now, dlam, epsi, 1,
+                 w.partials, w.counters + 2, w.res);
+          STT_TRY(check_launch("mma_search_kernel"));
+          STT_TRY(fetch((size_t)m + 2, "mma: line search"));
+          if (judge(R[m], R[m + 1])) break;
+        }
+        std::copy(R.begin(), R.begin() + m, gvec.begin());  // the accepted candidate's gvec
+        pend = 1;
+        t_pend = t;
+        eps_pend = epsi;
+        ready = 0.0;
       }
       S = C;
-      std::copy(R.begin(), R.begin() + m, gvec.begin());  // the accepted candidate's gvec
-      pend = 1;
-      t_pend = t;
-      eps_pend = epsi;
       residunorm = resinew;
       residumax = mxc;
     }
@@ -1198,8 +1273,14 @@ int device_subsolv(const MmaCols& c, const MData& D, double epsimin, const MmaWs
     epsi = 0.1 * epsi;
   }
   if (pend) {
-    mma_apply_kernel<<<gp, kMmaThreads, 0, st>>>(c.n, c.alfa, c.beta, w.dx, t_pend, eps_pend, x, xsi, eta);
+    mma_apply_kernel<<<gp, kMmaThreads, 0, st>>>(c.n, c.alfa, c.beta, w.dx, t_pend, eps_pend, px, pxsi, peta);
     STT_TRY(check_launch("mma_apply_kernel"));
+  }
+  if (px != x) {
+    const size_t bytes = 8 * (size_t)c.n;
+    STT_TRY(check_cuda(cudaMemcpyAsync(x, px, bytes, cudaMemcpyDeviceToDevice, st), "mma: x"));
+    STT_TRY(check_cuda(cudaMemcpyAsync(xsi, pxsi, bytes, cudaMemcpyDeviceToDevice, st), "mma: xsi"));
+    STT_TRY(check_cuda(cudaMemcpyAsync(eta, peta, bytes, cudaMemcpyDeviceToDevice, st), "mma: eta"));
   }
   return STT_OK;
 }

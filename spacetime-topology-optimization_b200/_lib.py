@@ -139,7 +139,9 @@ def check(rc: int) -> None:
 
 
 def stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # the raw handle: building torch's Stream object for it costs 3.2 us a call against 0.3,
+    # 2 to 37 times an evaluation
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def ptr(t: torch.Tensor | None) -> int | None:

@@ -57,7 +57,7 @@ struct MmaCols {
   const double *xval, *df0dx, *dfdx, *rxm;
 };
 
-STT_DEV double nanmax(double a, double b) { return (a != a || b != b) ? NAN : (a > b ? a : b); }
+STT_DEV double nanmax(double a, double b) { return b > a || b != b ? b : a; }  // a NaN stays
 
 // The separable approximation of one gradient entry g (sttopt/mma.py:263-284), factored
 // as P = P' ux2 and Q = Q' xl2 with P' = max(g, 0) + (0.001 |g| + r) and
@@ -75,26 +75,38 @@ struct ColFixed {
   double low, upp, alfa, beta, p0, q0, sp, sq, r;
 };
 
+// A thread's variable as the block's first one and the thread's place behind it: the first is
+// uniform, so a load's address is a uniform pointer and a 32-bit offset (with a 64-bit index
+// a thread, forming addresses was a third of the passes' instructions).
+struct ColIdx {
+  long long base;
+  unsigned t;
+  template <typename T>
+  STT_DEV T& of(T* p) const {
+    return (p + base)[t];
+  }
+};
+
 template <bool G>
-STT_DEV ColFixed load_fixed(const MmaCols& c, long long j) {
+STT_DEV ColFixed load_fixed(const MmaCols& c, const ColIdx& j) {
   ColFixed f;
-  f.low = c.low[j];
-  f.upp = c.upp[j];
-  f.alfa = c.alfa[j];
-  f.beta = c.beta[j];
+  f.low = j.of(c.low);
+  f.upp = j.of(c.upp);
+  f.alfa = j.of(c.alfa);
+  f.beta = j.of(c.beta);
   if constexpr (G) {
-    const double xv = c.xval[j];
+    const double xv = j.of(c.xval);
     const double ux1 = f.upp - xv, xl1 = xv - f.low;
     f.sp = ux1 * ux1;
     f.sq = xl1 * xl1;
-    f.r = c.rxm[j];
+    f.r = j.of(c.rxm);
     double p1, q1;
-    approx_pq1(c.df0dx[j], f.r, p1, q1);
+    approx_pq1(j.of(c.df0dx), f.r, p1, q1);
     f.p0 = p1 * f.sp;
     f.q0 = q1 * f.sq;
   } else {
-    f.p0 = c.p0[j];
-    f.q0 = c.q0[j];
+    f.p0 = j.of(c.p0);
+    f.q0 = j.of(c.q0);
     f.sp = f.sq = 1.0;
     f.r = 0.0;
   }
@@ -122,31 +134,49 @@ constexpr int row_chunk() {
   }
 }
 template <int CH, bool G>
-STT_DEV void load_rows(const MmaCols& c, int i0, long long j, double (&a)[CH], double (&b)[CH]) {
+STT_DEV void load_rows(const MmaCols& c, int i0, const ColIdx& j, double (&a)[CH], double (&b)[CH]) {
   const int nv = c.m - i0;
-  long long o = (long long)i0 * c.ld + j;
+  long long o = (long long)i0 * c.ld;
 #pragma unroll
   for (int u = 0; u < CH; ++u) {
     a[u] = b[u] = 0.0;
     if (u < nv) {
       if constexpr (G) {
-        a[u] = __ldg(c.dfdx + o);
+        a[u] = __ldg(&j.of(c.dfdx + o));
       } else {
-        a[u] = __ldg(c.P + o);
-        b[u] = __ldg(c.Q + o);
+        a[u] = __ldg(&j.of(c.P + o));
+        b[u] = __ldg(&j.of(c.Q + o));
       }
     }
     o += c.ld;
   }
 }
-// P', Q' of one entry from what load_rows read.
+// One entry as the two terms the passes sum, from what load_rows read.  The passes are bound by
+// instruction issue and the latency of their loads, so an entry costs as little as it can:
+// the gradient's positive and negative parts (of which at most one is not zero; a NaN has neither, as in
+// fmax), or P and Q themselves.
 template <bool G>
-STT_DEV void rows_pq1(const ColFixed& f, double a, double b, double& p1, double& q1) {
+STT_DEV void row_parts(double a, double b, double& u, double& v) {
   if constexpr (G) {
-    approx_pq1(a, f.r, p1, q1);
+    u = a > 0.0 ? a : 0.0;
+    v = a < 0.0 ? -a : 0.0;
   } else {
-    p1 = a;
-    q1 = b;
+    u = a;
+    v = b;
+  }
+}
+// lam . P' and lam . Q' from the sums su, sv of lam u, lam v and the sum of lam: P' is
+// 1.001 u + 0.001 v + r, Q' is 0.001 u + 1.001 v + r (approx_pq1, with the weights taken out of
+// the sum over the rows: nothing of opposite sign is added).
+template <bool G>
+STT_DEV void pq_sums(const ColFixed& f, double su, double sv, double lam_sum, double& lp, double& lq) {
+  if constexpr (G) {
+    const double r = f.r * lam_sum;
+    lp = fma(1.001, su, fma(0.001, sv, r));
+    lq = fma(1.001, sv, fma(0.001, su, r));
+  } else {
+    lp = su;
+    lq = sv;
   }
 }
 
@@ -155,6 +185,16 @@ STT_DEV void rows_pq1(const ColFixed& f, double a, double b, double& p1, double&
 struct ColFactors {
   double A, B, C, D;
 };
+// The same on an entry's parts: a term is u * U + v * V + R.
+struct PartFactors {
+  double U, V, R;
+  STT_DEV double of(double u, double v) const { return fma(u, U, fma(v, V, R)); }
+};
+template <bool G>
+STT_DEV PartFactors part_factors(const ColFixed& f, double a, double b) {  // P' a + Q' b
+  if constexpr (G) return {fma(1.001, a, 0.001 * b), fma(1.001, b, 0.001 * a), f.r * (a + b)};
+  else return {a, b, 0.0};
+}
 
 // Divisions by the point's four distances are multiplications by these reciprocals (one
 // division each), which rounds within an ulp of the reference's quotients.
@@ -480,7 +520,8 @@ inline int mma_bucket(int m) {
 // etao (the old one stays, should the candidate be rejected), gvec is formed, and h and the
 // residual's parts also for the next barrier level, 0.1 epsi.  It replaces a search pass and
 // an assemble pass over the same data: at 4.2M variables and 17 constraints 205 + 314 us
-// became 343 us, and one host synchronisation of two went.
+// became 343 us, and one host synchronisation of two went.  (304 us with the rows summed by
+// sign, uniform addresses and the first chunk of rows in flight beside the variable's data.)
 template <int MB, bool G, bool ADV>
 __global__ void __launch_bounds__(kMmaThreads, 2) mma_assemble_kernel(
     MmaCols c, const double* x, const double* xsi, const double* eta, double* xo, double* xsio, double* etao,
@@ -496,6 +537,8 @@ __global__ void __launch_bounds__(kMmaThreads, 2) mma_assemble_kernel(
     __syncthreads();
   }
   auto lam = [&](int i) { return ADV ? lam_s.v[i] : lam0.v[i]; };
+  double lam_sum = 0.0;
+  for (int i = 0; i < c.m; ++i) lam_sum += lam(i);
   extern __shared__ double sm[];
   constexpr int T8 = (MB + ND + 7) / 8;  // tile side for the largest m of the bucket
   constexpr int NT = T8 * (T8 + 1) / 2;
@@ -524,47 +567,52 @@ __global__ void __launch_bounds__(kMmaThreads, 2) mma_assemble_kernel(
 
   const long long ntiles = (c.n + kMmaThreads - 1) / kMmaThreads;
   for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const long long j = tile * kMmaThreads + tid;
-    const bool ok = j < c.n;
+    const ColIdx j{tile * kMmaThreads, threadIdx.x};
+    const bool ok = j.base + tid < c.n;
+    constexpr int CH = row_chunk<MB, G>();
+    double ra[CH], rb[CH];
+    auto rows_from = [&](int i0) {
+      if (ok) {
+        load_rows<CH, G>(c, i0, j, ra, rb);
+      } else {
+#pragma unroll
+        for (int u = 0; u < CH; ++u) ra[u] = rb[u] = 0.0;
+      }
+    };
+    rows_from(0);  // in flight beside the variable's own loads
     ColFixed f{};
     ColPoint p{};
     double xs = 0.0, et = 0.0;
     if (ok) {
       f = load_fixed<G>(c, j);
-      double xv = x[j];
-      xs = xsi[j];
-      et = eta[j];
+      double xv = j.of(x);
+      xs = j.of(xsi);
+      et = j.of(eta);
       if (ADV || pend) {
-        step_point(xv, xs, et, dx[j], t_pend, eps_pend, f.alfa, f.beta);
-        xo[j] = xv;
-        xsio[j] = xs;
-        etao[j] = et;
+        step_point(xv, xs, et, j.of(dx), t_pend, eps_pend, f.alfa, f.beta);
+        j.of(xo) = xv;
+        j.of(xsio) = xs;
+        j.of(etao) = et;
       }
       p = point_of(f, xv);
     }
     const ColFactors k = factors_of(f, p);
-    double lp = 0.0, lq = 0.0;  // sum of lam_i P'_i, lam_i Q'_i
-    constexpr int CH = row_chunk<MB, G>();
+    const PartFactors kg = part_factors<G>(f, k.A, k.B), kn = part_factors<G>(f, k.C, -k.D);
+    double su = 0.0, sv = 0.0;  // sum of lam_i u_i, lam_i v_i
 #pragma unroll
     for (int i0 = 0; i0 < MB; i0 += CH) {
       if (i0 < m) {
-        double ra[CH], rb[CH];
-        if (ok) {
-          load_rows<CH, G>(c, i0, j, ra, rb);
-        } else {
-#pragma unroll
-          for (int u = 0; u < CH; ++u) ra[u] = rb[u] = 0.0;
-        }
+        if (i0 > 0) rows_from(i0);
 #pragma unroll
         for (int u = 0; u < CH; ++u) {
           const int i = i0 + u;
           if (i < m) {
-            double p1, q1;
-            rows_pq1<G>(f, ra[u], rb[u], p1, q1);
-            lp = fma(lam(i), p1, lp);
-            lq = fma(lam(i), q1, lq);
-            if (need_g) gv.add(i, fma(p1, k.A, q1 * k.B));
-            gs[i * kMmaLd8 + tid] = fma(p1, k.C, -(q1 * k.D));
+            double gu, gw;
+            row_parts<G>(ra[u], rb[u], gu, gw);
+            su = fma(lam(i), gu, su);
+            sv = fma(lam(i), gw, sv);
+            if (need_g) gv.add(i, kg.of(gu, gw));
+            gs[i * kMmaLd8 + tid] = kn.of(gu, gw);
           }
         }
       }
@@ -573,9 +621,10 @@ __global__ void __launch_bounds__(kMmaThreads, 2) mma_assemble_kernel(
 #pragma unroll
     for (int e = 0; e < ND; ++e) delx[e] = 0.0;
     if (ok) {
+      double lp, lq, diagx;
+      pq_sums<G>(f, su, sv, lam_sum, lp, lq);
       const double plam = f.p0 + f.sp * lp;
       const double qlam = f.q0 + f.sq * lq;
-      double diagx;
 #pragma unroll
       for (int e = 0; e < ND; ++e) {
         const double ep = e == 0 ? epsi : 0.1 * epsi;
@@ -747,13 +796,18 @@ __global__ void __launch_bounds__(kMmaThreads, 3) mma_step_kernel(
   __shared__ double red[kMmaThreads / 32];
   __shared__ double fin[3];
   const int m = c.m;
+  double lam_sum = 0.0, dlam_sum = 0.0;
+  for (int i = 0; i < m; ++i) {
+    lam_sum += lam.v[i];
+    dlam_sum += dlam.v[i];
+  }
   double m1 = -INFINITY, m2 = -INFINITY, m3 = -INFINITY;
-  for (long long j = blockIdx.x * (long long)kMmaThreads + threadIdx.x; j < c.n;
-       j += (long long)gridDim.x * kMmaThreads) {
+  for (long long base = blockIdx.x * (long long)kMmaThreads; base < c.n; base += (long long)gridDim.x * kMmaThreads) {
+    const ColIdx j{base, threadIdx.x};
+    if (base + threadIdx.x >= c.n) break;
     const ColFixed f = load_fixed<G>(c, j);
-    const double xv = x[j], xs = xsi[j], et = eta[j];
-    const ColPoint p = point_of(f, xv);
-    double lp = 0.0, lq = 0.0, dp = 0.0, dq = 0.0;  // lam . P', lam . Q', dlam . P', dlam . Q'
+    const double xv = j.of(x), xs = j.of(xsi), et = j.of(eta);
+    double su = 0.0, sv = 0.0, du = 0.0, dv = 0.0;  // lam . u, lam . v, dlam . u, dlam . v
     constexpr int CH = pass_chunk<MB, G>();
 #pragma unroll
     for (int i0 = 0; i0 < MB; i0 += CH) {
@@ -764,24 +818,28 @@ __global__ void __launch_bounds__(kMmaThreads, 3) mma_step_kernel(
         for (int u = 0; u < CH; ++u) {
           const int i = i0 + u;
           if (i < m) {
-            double p1, q1;
-            rows_pq1<G>(f, ra[u], rb[u], p1, q1);
-            lp = fma(lam.v[i], p1, lp);
-            lq = fma(lam.v[i], q1, lq);
-            dp = fma(dlam.v[i], p1, dp);
-            dq = fma(dlam.v[i], q1, dq);
+            double gu, gw;
+            row_parts<G>(ra[u], rb[u], gu, gw);
+            su = fma(lam.v[i], gu, su);
+            sv = fma(lam.v[i], gw, sv);
+            du = fma(dlam.v[i], gu, du);
+            dv = fma(dlam.v[i], gw, dv);
           }
         }
       }
     }
+    const ColPoint p = point_of(f, xv);
     const ColFactors k = factors_of(f, p);
+    double lp, lq, dp, dq;  // lam . P', lam . Q', dlam . P', dlam . Q'
+    pq_sums<G>(f, su, sv, lam_sum, lp, lq);
+    pq_sums<G>(f, du, dv, dlam_sum, dp, dq);
     const double plam = f.p0 + f.sp * lp, qlam = f.q0 + f.sq * lq;
     const double gd = fma(dp, k.C, -(dq * k.D));  // GG^T dlam
     double delx, diagx;
     newton_col(plam, qlam, p, xs, et, epsi, delx, diagx);
     const double w = 1.0 / diagx;
     const double d = -delx * w - gd * w;
-    dx[j] = d;
+    j.of(dx) = d;
     const double dxsi = -xs + epsi * p.xainv - (xs * d) * p.xainv;
     const double deta = -et + epsi * p.bxinv + (et * d) * p.bxinv;
     m1 = nanmax(m1, (-1.01 * d) * p.xainv);
@@ -819,6 +877,8 @@ __global__ void __launch_bounds__(kMmaThreads, 3) mma_search_kernel(
   const double t = tdev ? *tdev : t_arg;
   for (int i = threadIdx.x; i < c.m; i += kMmaThreads) lam.v[i] = lam0.v[i] + t * dlam.v[i];
   __syncthreads();
+  double lam_sum = 0.0;
+  for (int i = 0; i < c.m; ++i) lam_sum += lam.v[i];
   constexpr bool kSlots = MB <= 20;  // static shared memory stays under 48 KB
   __shared__ double slots[kSlots ? MB * kMmaThreads : 1];
   const int m = c.m;
@@ -827,23 +887,24 @@ __global__ void __launch_bounds__(kMmaThreads, 3) mma_search_kernel(
   gv.zero();
   double ss = 0.0, mx = 0.0;
   for (long long base = blockIdx.x * (long long)kMmaThreads; base < c.n; base += (long long)gridDim.x * kMmaThreads) {
-    const long long j = base + threadIdx.x;
-    const bool ok = j < c.n;
+    const ColIdx j{base, threadIdx.x};
+    const bool ok = base + threadIdx.x < c.n;
     ColFixed f{};
     ColPoint p{};
     double xs = 0.0, et = 0.0;
     if (ok) {
       f = load_fixed<G>(c, j);
-      double xv = x[j];
+      double xv = j.of(x);
       if (resid) {
-        xs = xsi[j];
-        et = eta[j];
+        xs = j.of(xsi);
+        et = j.of(eta);
       }
-      if (dx) step_point(xv, xs, et, dx[j], t, epsi, f.alfa, f.beta);
+      if (dx) step_point(xv, xs, et, j.of(dx), t, epsi, f.alfa, f.beta);
       p = point_of(f, xv);
     }
     const ColFactors k = factors_of(f, p);
-    double lp = 0.0, lq = 0.0;
+    const PartFactors kg = part_factors<G>(f, k.A, k.B);
+    double su = 0.0, sv = 0.0;
     constexpr int CH = pass_chunk<MB, G>();
 #pragma unroll
     for (int i0 = 0; i0 < MB; i0 += CH) {
@@ -859,16 +920,20 @@ __global__ void __launch_bounds__(kMmaThreads, 3) mma_search_kernel(
         for (int u = 0; u < CH; ++u) {
           const int i = i0 + u;
           if (i < m) {
-            double p1, q1;
-            rows_pq1<G>(f, ra[u], rb[u], p1, q1);
-            lp = fma(lam.v[i], p1, lp);
-            lq = fma(lam.v[i], q1, lq);
-            gv.add(i, fma(p1, k.A, q1 * k.B));
+            double gu, gw;
+            row_parts<G>(ra[u], rb[u], gu, gw);
+            su = fma(lam.v[i], gu, su);
+            sv = fma(lam.v[i], gw, sv);
+            gv.add(i, kg.of(gu, gw));
           }
         }
       }
     }
-    if (ok && resid) resid_n(f.p0 + f.sp * lp, f.q0 + f.sq * lq, p, xs, et, epsi, ss, mx);
+    if (ok && resid) {
+      double lp, lq;
+      pq_sums<G>(f, su, sv, lam_sum, lp, lq);
+      resid_n(f.p0 + f.sp * lp, f.q0 + f.sq * lq, p, xs, et, epsi, ss, mx);
+    }
   }
   const int kp = m + 2, ks = m + 1;
   gv.write(m, partials, 0, red + kMmaThreads / 32);
@@ -1137,9 +1202,10 @@ int device_subsolv(const MmaCols& c, const MData& D, double epsimin, const MmaWs
   // step's [3 maxima | steg] sit behind the advance's
   const size_t step_at = assemble_res(m, 2);
   double* const res_step = w.res + step_at;
-  std::vector<double> R(step_at + 4), gvec(m), h(m), A((size_t)m * m);
-  auto fetch = [&](size_t count, const char* what) -> int {
-    STT_TRY(check_cuda(cudaMemcpyAsync(R.data(), w.res, 8 * count, cudaMemcpyDeviceToHost, st), what));
+  std::vector<double> Rv(step_at + 4), gvec(m), h(m), A((size_t)m * m);
+  double* const R = Rv.data();
+  auto fetch = [&](const char* what) -> int {
+    STT_TRY(check_cuda(cudaMemcpyAsync(R, w.res, 8 * Rv.size(), cudaMemcpyDeviceToHost, st), what));
     return check_cuda(cudaStreamSynchronize(st), what);
   };
   auto fold = [&](int nd) -> int {
@@ -1149,7 +1215,7 @@ int device_subsolv(const MmaCols& c, const MData& D, double epsimin, const MmaWs
   };
   // h, sum of squares and max of level q (0: the pass's epsi, 1: 0.1 epsi) of the fetched results
   auto level = [&](int q, double& ssn, double& mxn) {
-    const double* L = R.data() + m + (size_t)m * m + (size_t)q * (m + 2);
+    const double* L = R + m + (size_t)m * m + (size_t)q * (m + 2);
     std::copy(L, L + m, h.begin());
     ssn = L[m];
     mxn = ssn != ssn ? NAN : L[m + 1];
@@ -1166,10 +1232,10 @@ int device_subsolv(const MmaCols& c, const MData& D, double epsimin, const MmaWs
     pend = 0;
     STT_TRY(check_launch("mma_assemble_kernel"));
     STT_TRY(fold(1));
-    STT_TRY(fetch(assemble_res(m, 1), "mma: assemble"));
-    if (!have_g) std::copy(R.begin(), R.begin() + m, gvec.begin());
+    STT_TRY(fetch("mma: assemble"));
+    if (!have_g) std::copy(R, R + m, gvec.begin());
     have_g = true;
-    std::copy(R.begin() + m, R.begin() + m + (size_t)m * m, A.begin());
+    std::copy(R + m, R + m + (size_t)m * m, A.begin());
     level(0, ssn, mxn);
     return STT_OK;
   };
@@ -1221,7 +1287,7 @@ int device_subsolv(const MmaCols& c, const MData& D, double epsimin, const MmaWs
              epsi, lam_now, dlam, epsi, 1, w.partials);
       STT_TRY(check_launch("mma_assemble_kernel"));
       STT_TRY(fold(2));
-      STT_TRY(fetch(step_at + 4, "mma: step and first candidate"));
+      STT_TRY(fetch("mma: step and first candidate"));
       const double steg = R[step_at + 3];  // 1 / max(stmalfa, stmbeta, stmxx, 1), as formed on the device
       // Backtracking on the residual norm: the first halving whose norm does not exceed
       // the current one, else the last (sttopt/mma.py:297-343).
@@ -1229,16 +1295,16 @@ int device_subsolv(const MmaCols& c, const MData& D, double epsimin, const MmaWs
       double resinew = 0.0, mxc = 0.0, t = steg;
       auto judge = [&](double ssc, double mxs) {
         double ssmc = 0.0, mxmc = -INFINITY;
-        resid_m(D, C, R.data(), epsi, ssmc, mxmc);
+        resid_m(D, C, R, epsi, ssmc, mxmc);
         resinew = std::sqrt(ssc + ssmc);
         mxc = hmax(ssc != ssc ? NAN : mxs, mxmc);
         return !(resinew > residunorm);
       };
-      const double* L0 = R.data() + m + (size_t)m * m;
+      const double* L0 = R + m + (size_t)m * m;
       ++cap.tries;
       if (judge(L0[m], L0[m + 1])) {  // the first candidate: its pass has formed the next step's system
-        std::copy(R.begin(), R.begin() + m, gvec.begin());
-        std::copy(R.begin() + m, R.begin() + m + (size_t)m * m, A.begin());
+        std::copy(R, R + m, gvec.begin());
+        std::copy(R + m, R + m + (size_t)m * m, A.begin());
         level(0, ssn, mxn);
         std::swap(px, qx);
         std::swap(pxsi, qxsi);
@@ -1253,10 +1319,10 @@ int device_subsolv(const MmaCols& c, const MData& D, double epsimin, const MmaWs
           launch(k.search, gp, kMmaThreads, 0, st, c, px, pxsi, peta, w.dx, t, nullptr, lam_now, dlam, epsi, 1,
                  w.partials, w.counters + 2, w.res);
           STT_TRY(check_launch("mma_search_kernel"));
-          STT_TRY(fetch((size_t)m + 2, "mma: line search"));
+          STT_TRY(fetch("mma: line search"));
           if (judge(R[m], R[m + 1])) break;
         }
-        std::copy(R.begin(), R.begin() + m, gvec.begin());  // the accepted candidate's gvec
+        std::copy(R, R + m, gvec.begin());  // the accepted candidate's gvec
         pend = 1;
         t_pend = t;
         eps_pend = epsi;

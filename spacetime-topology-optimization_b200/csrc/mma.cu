@@ -23,6 +23,7 @@
 // reference's tensor arithmetic; the dot products use fma() explicitly.
 #include <algorithm>
 #include <cmath>
+#include <mutex>
 #include <type_traits>
 #include <vector>
 
@@ -748,10 +749,13 @@ __global__ void __launch_bounds__(kMmaThreads, 2) mma_assemble_kernel(
 
 // Folds the assemble (nd = 1) or advance (nd = 2) pass's block partials (entry-major, nb
 // blocks) in block order, a warp an entry on as many SMs as there are entries / 8, into the
-// results (assemble_res).
+// results (assemble_res), in page-locked host memory; `step`, when given: the step pass's
+// four, which go behind them.
 __global__ void __launch_bounds__(kMmaThreads) mma_fold_kernel(const double* __restrict__ partials, int nb, int m,
-                                                               int nd, double* __restrict__ res) {
+                                                               int nd, const double* __restrict__ step,
+                                                               double* __restrict__ res) {
   grid_wait();
+  if (step && blockIdx.x == 0 && threadIdx.x < 4) res[assemble_res(m, nd) + threadIdx.x] = step[threadIdx.x];
   const int kp = assemble_kp(m, nd), ks = kp - nd, m1 = m + nd, lane = threadIdx.x & 31;
   const int e = blockIdx.x * (kMmaThreads / 32) + (threadIdx.x >> 5);
   if (e >= kp) return;
@@ -1171,6 +1175,50 @@ struct CapStats {
 
 namespace {
 
+// The page-locked memory that the passes write their results to and the host reads after the
+// stream's synchronisation, with no copy between (a copy to pageable memory and its set-up cost
+// a Newton step of a small problem a fifth of its time).  Taken for one call from a
+// pool of idle ones (any thread; at most kMaxIdle kept) and given back with no pass in flight.
+class Results {
+  static constexpr size_t kMaxIdle = 32;
+  static std::mutex& mu() {
+    static std::mutex m;
+    return m;
+  }
+  static std::vector<double*>& idle() {
+    static auto* v = new std::vector<double*>();  // lives as long as the process
+    return *v;
+  }
+  cudaStream_t st_;
+  double* p_ = nullptr;
+
+ public:
+  explicit Results(cudaStream_t st) : st_(st) {}
+  Results(const Results&) = delete;
+  Results& operator=(const Results&) = delete;
+  double* data() const { return p_; }
+  int take() {
+    {
+      std::lock_guard<std::mutex> lock(mu());
+      if (!idle().empty()) {
+        p_ = idle().back();
+        idle().pop_back();
+        return STT_OK;
+      }
+    }
+    return check_cuda(cudaHostAlloc((void**)&p_, 8 * (size_t)(assemble_res(kMmaMaxM, 2) + 8),
+                                    cudaHostAllocPortable | cudaHostAllocMapped),
+                      "mma: results");
+  }
+  ~Results() {
+    if (!p_) return;
+    const bool clean = cudaStreamSynchronize(st_) == cudaSuccess;  // (an early return may leave a pass in flight)
+    std::lock_guard<std::mutex> lock(mu());
+    if (clean && idle().size() < kMaxIdle) idle().push_back(p_);
+    else cudaFreeHost(p_);
+  }
+};
+
 // subsolv's barrier path and Newton loop for m < n (sttopt/mma.py:346-557) with the
 // per-variable work on the device.  x, xsi, eta (device) receive the solution; S the
 // m-sized part.
@@ -1201,16 +1249,15 @@ int device_subsolv(const MmaCols& c, const MData& D, double epsimin, const MmaWs
   // results of one fetch: the assemble's or advance's, or a search's [gvec | ss | mx]; the
   // step's [3 maxima | steg] sit behind the advance's
   const size_t step_at = assemble_res(m, 2);
-  double* const res_step = w.res + step_at;
-  std::vector<double> Rv(step_at + 4), gvec(m), h(m), A((size_t)m * m);
-  double* const R = Rv.data();
-  auto fetch = [&](const char* what) -> int {
-    STT_TRY(check_cuda(cudaMemcpyAsync(R, w.res, 8 * Rv.size(), cudaMemcpyDeviceToHost, st), what));
-    return check_cuda(cudaStreamSynchronize(st), what);
-  };
+  double* const res_step = w.res;  // on the device: the advance pass reads steg there
+  Results results(st);
+  STT_TRY(results.take());
+  double* const R = results.data();
+  std::vector<double> gvec(m), h(m), A((size_t)m * m);
+  auto fetch = [&](const char* what) -> int { return check_cuda(cudaStreamSynchronize(st), what); };
   auto fold = [&](int nd) -> int {
     const int kp = assemble_kp(m, nd), per = kMmaThreads / 32;
-    launch(mma_fold_kernel, (kp + per - 1) / per, kMmaThreads, 0, st, w.partials, ga, m, nd, w.res);
+    launch(mma_fold_kernel, (kp + per - 1) / per, kMmaThreads, 0, st, w.partials, ga, m, nd, nd == 2 ? res_step : nullptr, R);
     return check_launch("mma_fold_kernel");
   };
   // h, sum of squares and max of level q (0: the pass's epsi, 1: 0.1 epsi) of the fetched results
@@ -1317,7 +1364,7 @@ int device_subsolv(const MmaCols& c, const MData& D, double epsimin, const MmaWs
           C = moved(S, T, t);
           ++cap.tries;
           launch(k.search, gp, kMmaThreads, 0, st, c, px, pxsi, peta, w.dx, t, nullptr, lam_now, dlam, epsi, 1,
-                 w.partials, w.counters + 2, w.res);
+                 w.partials, w.counters + 2, R);
           STT_TRY(check_launch("mma_search_kernel"));
           STT_TRY(fetch("mma: line search"));
           if (judge(R[m], R[m + 1])) break;

@@ -15,6 +15,7 @@
 #include "errors.h"
 #include "hier.h"
 #include "mg.cuh"
+#include "pair.cuh"
 
 namespace stt {
 
@@ -112,7 +113,8 @@ static long long plan_solve(const stt_hier* h, int nrows, int gamma, char* base,
     const dim3 tg = pcg_tile_grid(h->nelx, h->nely, nrows, 4);
     // the level-0 chained passes' blocks may take the r.z reductions
     const dim3 pg = postsmooth_grid(h->nelx, h->nely, nrows, es), qg = presmooth_grid(h->nelx, h->nely, nrows, es);
-    w.nblk_max = std::max<int>(std::max<int>(tg.x * tg.y, std::max(pg.x * pg.y, qg.x * qg.y)), ew_blocks(l0.ndof));
+    const dim3 rg = pair_grid(kPairPostCols, h->nelx, h->nely, nrows).g;
+    w.nblk_max = std::max<int>({(int)(tg.x * tg.y), (int)(pg.x * pg.y), (int)(qg.x * qg.y), (int)rg.x, ew_blocks(l0.ndof)});
     w.rs = (RowState*)carve(base, used, sizeof(RowState) * nrows);
     w.partials = (double*)carve(base, used, 8LL * nrows * w.nblk_max * 3);
     w.counters = (unsigned*)carve(base, used, 4LL * nrows);
@@ -320,6 +322,51 @@ struct Cycle {
 #undef STT_PRE
   }
 
+  // Level 0's passes with two columns a lane (plane stress in FP32 without a reaction or the
+  // flexible dot): `paired` when they apply, `joined` when the 2 x 2 transfers run in them too.
+  bool paired() const {
+    if constexpr (D != 2 || sizeof(T) != 4) return false;
+    else return !h->has_reaction && !(rzf.rst && rzf.zold);
+  }
+  bool joined() const { return paired() && h->lv[0].kx == 2 && h->lv[0].ky == 2; }
+  // x2 into out_x and the residual (joined: level 1's right-hand side) into out_r
+  void pre_pair(const T* b, long long b_rs, T* out_x, T* out_r) {
+    if constexpr (D == 2 && sizeof(T) == 4) {
+      const LevelDesc& lv = h->lv[0];
+      const long long nd = vstride(lv.ndof);
+      const PairGrid p = pair_grid(kPairPreCols, lv.nelx, lv.nely, nrows);
+#define STT_PRE2(DOWN, RS, CF)                                                                                     \
+  launch(l0_pre_pair_kernel<DOWN>, p.g, kQThreads, 0, st, b, b_rs, out_x, nd, out_r, RS, rho0(), lv.rs_rho, lv.fixed, \
+         CF, h->row_map, h->hrows, rst, lv.nelx, lv.nely, p.strips, p.band, omega, pair_q(mq))
+      if (joined()) STT_PRE2(true, vstride(h->lv[1].ndof), h->lv[1].fixed);
+      else STT_PRE2(false, nd, nullptr);
+#undef STT_PRE2
+    }
+  }
+  // from x0 (joined: x0 + P ec) into out; with rzf set also the PCG's r.z
+  void post_pair(const T* x0, const T* ec, const T* b, long long b_rs, T* out) {
+    if constexpr (D == 2 && sizeof(T) == 4) {
+      const LevelDesc& lv = h->lv[0];
+      const long long nd = vstride(lv.ndof);
+      const PairGrid p = pair_grid(kPairPostCols, lv.nelx, lv.nely, nrows);
+      RzFuse<T> rz = rzf;
+      rz.red.nblk = (int)p.g.x;
+#define STT_POST2(UP, RZ)                                                                                            \
+  launch((l0_post_pair_kernel<UP, RZ>), p.g, kQThreads, 0, st, x0, nd, ec, vstride(h->lv[1].ndof), b, b_rs, out, nd, \
+         rho0(), lv.rs_rho, lv.fixed, h->row_map, h->hrows, rst, lv.nelx, lv.nely, p.strips, p.band, omega,          \
+         pair_q(mq), rz)
+      if (rzf.rst) {
+        if (joined()) STT_POST2(true, true);
+        else STT_POST2(false, true);
+        rz_done = true;
+      } else {
+        if (joined()) STT_POST2(true, false);
+        else STT_POST2(false, false);
+      }
+#undef STT_POST2
+    }
+  }
+
   // Level 1's smoothing chained in one pass from the level-0 densities (FP32, 2 x 2
   // mirror-form children, two sweeps each way): PRE writes x2 to ox and the residual to
   // orr; POST sweeps twice from x0 into ox.  False when the hierarchy does not allow it
@@ -439,7 +486,13 @@ struct Cycle {
     const bool modal0 = l == 0 && h->modal;
     bool chained1 = false;  // level 1's smoothing chained in one pass each way
     bool chainedS = false;  // a stencil level's, likewise
-    if (modal0 && n_smooth == 2) {
+    const LevelDesc& cl = h->lv[l + 1];
+    const long long cnd = vstride(cl.ndof);
+    T* bc = (T*)w.b[l + 1];
+    const bool pair0 = modal0 && n_smooth == 2 && paired();
+    if (pair0) {
+      pre_pair(b, b_rs, xa, joined() ? bc : xb);
+    } else if (modal0 && n_smooth == 2) {
       presmooth(b, b_rs, xa, xb);
     } else if (l == 1 && b_rs == nd && l1_chain(true, nullptr, b, xa, xb)) {
       chained1 = true;
@@ -455,18 +508,16 @@ struct Cycle {
       pass<SW_RESID>(l, xa, nd, b, b_rs, xb, nd);
     }
     // restricted into b_{l+1}
-    const LevelDesc& cl = h->lv[l + 1];
-    const long long cnd = vstride(cl.ndof);
-    T* bc = (T*)w.b[l + 1];
-    transfer_down(lv, cl, xb, nd, bc, cnd);
+    if (!(pair0 && joined())) transfer_down(lv, cl, xb, nd, bc, cnd);
     T* ec = coarse_correction(l, bc);
-    transfer_up(lv, cl, ec, cnd, xa, nd);
+    if (!(pair0 && joined())) transfer_up(lv, cl, ec, cnd, xa, nd);
     // post-smoothing; level 0's last sweep writes straight into final_out when given
     if (modal0 && n_smooth == 2) {
       // the fused pass reads b a few rows ahead of its writes, so it never writes over b
       // (an in-place V-cycle, z = r, goes through xb and the final copy)
       T* dst = (final_out && final_out != b) ? final_out : xb;
-      postsmooth(xa, b, b_rs, dst);
+      if (pair0) post_pair(xa, ec, b, b_rs, dst);
+      else postsmooth(xa, b, b_rs, dst);
       return dst;
     }
     if (chained1) {

@@ -362,8 +362,9 @@ def run_mma(dev, steps=3, warmup=1, cpu_sample=1 << 18, n=2 * NELX * NELY):
     torch.cuda.synchronize()
     ms = a.elapsed_time(b) / steps
     newton, tries = stats["subsolv_newton_steps"], stats["subsolv_line_search_tries"]
-    # bytes a variable: assemble 8m + 112 (with the pending step), step 8m + 88, search 8m + 88
-    per_var = newton * (8 * m + 112 + 8 * m + 88) + tries * (8 * m + 88) + (8 * m + 112)
+    # bytes a variable: a Newton step's step pass 8m + 88 and advance pass (the first candidate and
+    # the next step's system) 8m + 112, a further candidate's search pass 8m + 88, one assemble
+    per_var = newton * (8 * m + 88 + 8 * m + 112) + (tries - newton) * (8 * m + 88) + (8 * m + 88)
     achieved = per_var * n / (ms / 1e3) / 1e9
     peaks = json.loads((ROOT / "MEASURED_PEAKS.json").read_text()) if (ROOT / "MEASURED_PEAKS.json").exists() else {}
     peak = float(peaks.get("hbm_gbs", 6650.0))

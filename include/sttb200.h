@@ -150,7 +150,8 @@ long long stt_hier_workspace_bytes(int d, int nelx, int nely, int hrows,
 
 /* Build the Galerkin hierarchy on the device (torch_mg.build_hierarchy): level 0 is
  * K(rho) (+ lumped reaction), coarser levels the exact Galerkin products stored as
- * symmetric 9-point block stencils, the coarsest factorised by FP64 Cholesky.
+ * symmetric 9-point block stencils, the coarsest factorised in FP64 (odd-even elimination
+ * of its grid lines; block-banded Cholesky for lines above 64 unknowns).
  * precision STT_FP32 keeps FP32 copies for an FP32 V-cycle.  reaction may be NULL. */
 int stt_hier_create(stt_hier** out, void* workspace, long long ws_bytes, int d, int nelx,
                     int nely, int hrows, const double* rho, long long rho_rs,
@@ -159,7 +160,7 @@ int stt_hier_create(stt_hier** out, void* workspace, long long ws_bytes, int d, 
                     stt_stream_t stream);
 
 /* The build does not synchronise.  The levels are built on `stream`; the coarsest
- * level's factorisation (and its explicit inverse for STT_FP32) then runs on a stream of
+ * level's factorisation then runs on a stream of
  * the library's own, ordered after them, while `stream` goes on: every coarse solve on
  * any stream (stt_vcycle, stt_pcg_mg, ...) waits for it on the device.  The build's
  * device checks (a coarse pivot <= 0, a coarse operator beyond its planned band) are

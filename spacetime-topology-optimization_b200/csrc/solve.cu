@@ -317,7 +317,7 @@ struct Cycle {
       mix_done = true;
     } else {
       if (h->has_reaction) STT_PRE(true, false);
-      else STT_PRE(false, false);
+      else if constexpr (D != 2 || sizeof(T) != 4) STT_PRE(false, false);  // (there pre_pair runs)
     }
 #undef STT_PRE
   }
@@ -438,7 +438,7 @@ struct Cycle {
       rz_done = true;
     } else {
       if (h->has_reaction) STT_POST(true, false);
-      else STT_POST(false, false);
+      else if constexpr (D != 2 || sizeof(T) != 4) STT_POST(false, false);  // (there post_pair runs)
     }
 #undef STT_POST
   }

@@ -4,9 +4,10 @@
 ``mmasub`` and ``subsolv`` keep the reference's signatures and return values.  Every
 n-sized and m x n-sized quantity stays on the GPU and is handled by fused FP64 passes in
 ``libsttb200.so`` (``stt_mma_sub``, ``stt_mma_subsolv``): the asymptotes and move limits,
-and for each Newton step of the primal-dual interior-point solve one pass that forms the
-residual, the Newton right-hand side and the m x m matrix ``GG diag(1/diagx) GG^T``, one
-pass for ``dx`` with its step limits and one pass per line-search halving.  ``mmasub``
+and for each Newton step of the primal-dual interior-point solve one pass for ``dx`` with its
+step limits and one that evaluates the line search's first candidate and forms there the
+next step's residual, right-hand side and m x m matrix ``GG diag(1/diagx) GG^T`` (a rejected
+candidate costs a pass a halving and one to form them again).  ``mmasub``
 never stores the approximation ``P, Q``: the passes rebuild it from ``dfdx``.  The
 m-sized algebra (y, z, lam, mu, zet, s and the bordered Newton system) runs on the host,
 where the reference also solves that system.  With ``m >= n`` the whole subproblem has

@@ -3,7 +3,8 @@
 ``build_hierarchy`` builds every level on the device in one call (``stt_hier_create``):
 exact Galerkin element products ``sum_m S_m^T K_child S_m`` (sttopt/torch_mg.py:355-370),
 stored as symmetric 9-point block stencils, coarse masks sampled at collocated nodes
-(:376), and the coarsest level factorised by a block-banded FP64 Cholesky (:269-290).
+(:376), and the coarsest level factorised in FP64 (:269-290): odd-even elimination of its grid
+lines, or a block-banded Cholesky where the lines are too long for it.
 The hierarchy policy is the reference's: factors 2 or 3 per dimension
 (``coarsening_factors``), stop at ``max_coarse_elements``.
 

@@ -25,7 +25,7 @@ namespace stt {
 // restriction 263 + 60 -> 245 us, prolongation and post-smoothing 105 + 296 -> 244 us, the
 // V-cycle 1718 -> 1434 us; without the ring 343 and 445; at 128 registers and 16 warps an SM,
 // spilled, 468 and 634.  They are as good on small grids (540x270 x 4 rows: a V-cycle of 110 us
-// either way; 256x128 x 8: 92 and 91), so they run wherever they apply.
+// with the old passes, 105 with these; 256x128 x 8: 92 and 91), so they run wherever they apply.
 struct PairQ {
   float2 m00, m01, m11, m22, m44, m55;  // MQ's coefficients, twice each
   float2 neg, half;                     // -1 and 1/2: the paired instructions have no negation
@@ -203,11 +203,13 @@ struct PairStrip {
 
 constexpr int kPairPreCols = 58, kPairPostCols = 60;
 
-// Rows a warp marches: even, so that a band starts on a coarse row; as march_band, the longest
-// while the SMs have warps for 64 rows each (at up to 6 rows of halo a band).
+// Rows a warp marches: even, so that a band starts on a coarse row; the longest that gives each
+// SM its 12 warps, but 4 rows (with 6 of halo) only where 8 would leave it fewer than 8 warps.
+// A V-cycle of 540x270 x 4 rows: 110 us with 4-row bands, 105 with 8; 256x128 x 8: 92 with 4, 97
+// with 8; 512x256 x 33: 362 with 32, 372 with 64.
 inline int pair_band(int strips, int nny, int rows) {
   int band = 64;
-  while (band > 4 && (long long)strips * ((nny + band - 1) / band) * rows < 148LL * 16) band /= 2;
+  while (band > 4 && (long long)strips * ((nny + band - 1) / band) * rows < 148LL * (band > 8 ? 12 : 8)) band /= 2;
   return band;
 }
 // A launch: warps numbered (band, strip), kQWarps a block.

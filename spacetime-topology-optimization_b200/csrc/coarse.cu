@@ -17,9 +17,9 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
-#include <mutex>
 
 #include "errors.h"
+#include "smem.h"
 
 namespace stt {
 
@@ -660,26 +660,6 @@ void coarse_plan(const LevelDesc& c, int d, CoarseDesc& co) {
   const int bw = d * (nmin + 2) - 1;  // max |P - Q| of a nonzero
   co.B = (bw + 31) / 32 * 32;
   co.nb = (co.n + co.B - 1) / co.B;
-}
-
-// Raises a kernel's dynamic shared-memory ceiling to the device's opt-in maximum, once per
-// device and kernel (a per-call ceiling would race between host threads).
-template <auto Kernel>
-static int allow_smem() {
-  static std::mutex mu;
-  static bool done[64] = {};
-  int dev = 0;
-  STT_TRY(check_cuda(cudaGetDevice(&dev), "cudaGetDevice"));
-  std::lock_guard<std::mutex> lock(mu);
-  if (dev >= 0 && dev < 64 && done[dev]) return STT_OK;
-  int optin = 0;
-  cudaFuncAttributes fa;
-  STT_TRY(check_cuda(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "smem attribute"));
-  STT_TRY(check_cuda(cudaFuncGetAttributes(&fa, Kernel), "function attributes"));
-  STT_TRY(check_cuda(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          optin - (int)fa.sharedSizeBytes), "smem attr"));
-  if (dev >= 0 && dev < 64) done[dev] = true;
-  return STT_OK;
 }
 
 template <int NB>

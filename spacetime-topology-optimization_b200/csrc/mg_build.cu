@@ -11,6 +11,7 @@
 #include "hier.h"
 #include "modal.h"
 #include "q4.cuh"
+#include "smem.h"
 
 namespace stt {
 
@@ -1079,32 +1080,6 @@ static int build_levels(stt_hier* h, const double* rho, long long rho_rs, const 
   return STT_OK;
 }
 
-// The dynamic shared-memory ceiling of the banded factorisation, raised once per device to the
-// device's opt-in maximum.  (Setting it per call to the call's own size raced between
-// host threads building hierarchies of different block sizes: a launch could meet
-// another thread's smaller ceiling and fail.)
-static int allow_large_smem() {
-  static std::mutex mu;
-  static bool done[64] = {};
-  int dev = 0;
-  STT_TRY(check_cuda(cudaGetDevice(&dev), "cudaGetDevice"));
-  std::lock_guard<std::mutex> lock(mu);
-  if (dev >= 0 && dev < 64 && done[dev]) return STT_OK;
-  int max_optin = 0;
-  STT_TRY(check_cuda(cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev),
-                     "smem attribute"));
-  // the ceiling counts the kernel's static shared memory too
-  auto raise_to = [&](const void* fn) -> int {
-    cudaFuncAttributes fa;
-    STT_TRY(check_cuda(cudaFuncGetAttributes(&fa, fn), "function attributes"));
-    return check_cuda(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           max_optin - (int)fa.sharedSizeBytes), "smem attr");
-  };
-  STT_TRY(raise_to((const void*)band_factor_kernel));
-  if (dev >= 0 && dev < 64) done[dev] = true;
-  return STT_OK;
-}
-
 // Pool of coarse-factorisation streams and events (creating a stream per hierarchy would
 // cost more than the overlap gains). The side streams have the highest priority: the
 // factorisation is on the critical path of the first coarse solve, and its few CTAs
@@ -1167,7 +1142,7 @@ static int build_coarse(stt_hier* h, cudaStream_t st) {
       cl.st64, cl.fixed, cl.nnx, cl.nny, co.by_col, co.B, co.nb, co.blocks, h->status);
   STT_TRY(check_launch("band assemble"));
   const size_t smem = (size_t)3 * co.B * (co.B + 1) * sizeof(double);
-  STT_TRY(allow_large_smem());
+  STT_TRY(allow_smem<band_factor_kernel>());
   band_factor_kernel<<<H, 256, smem, st>>>(co.blocks, co.B, co.nb, h->status);
   return check_launch("band factor");
 }

@@ -29,6 +29,7 @@
 
 #include "common.cuh"
 #include "errors.h"
+#include "smem.h"
 
 namespace stt {
 
@@ -970,11 +971,17 @@ struct Kernels {
   AsmFn assemble, advance;
   StepFn step;
   SearchFn search;
+  int (*allow_assemble)();
+  int (*allow_advance)();
 };
 template <int MB, bool G>
 Kernels kernels_of() {
-  return {mma_assemble_kernel<MB, G, false>, mma_assemble_kernel<MB, G, true>, mma_step_kernel<MB, G>,
-          mma_search_kernel<MB, G>};
+  return {mma_assemble_kernel<MB, G, false>,
+          mma_assemble_kernel<MB, G, true>,
+          mma_step_kernel<MB, G>,
+          mma_search_kernel<MB, G>,
+          allow_smem<mma_assemble_kernel<MB, G, false>>,
+          allow_smem<mma_assemble_kernel<MB, G, true>>};
 }
 template <bool G>
 Kernels pick_kernels(int m) {
@@ -1232,12 +1239,8 @@ int device_subsolv(const MmaCols& c, const MData& D, double epsimin, const MmaWs
   const int mb = mma_bucket(m);
   const size_t smem_g = assemble_smem(m, mb, 1, true), smem = assemble_smem(m, mb, 1, false);
   const size_t smem_adv = assemble_smem(m, mb, 2, true);
-  STT_TRY(check_cuda(cudaFuncSetAttribute((const void*)k.assemble, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem_g),
-                     "mma: assemble shared memory"));
-  STT_TRY(check_cuda(cudaFuncSetAttribute((const void*)k.advance, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem_adv),
-                     "mma: advance shared memory"));
+  STT_TRY(k.allow_assemble());
+  STT_TRY(k.allow_advance());
   STT_TRY(check_cuda(cudaMemsetAsync(w.counters, 0, 4 * sizeof(unsigned), st), "mma: counters"));
   mma_init_kernel<<<gp, kMmaThreads, 0, st>>>(c.n, c.alfa, c.beta, x, xsi, eta);
   STT_TRY(check_launch("mma_init_kernel"));

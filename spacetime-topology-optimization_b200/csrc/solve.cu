@@ -157,6 +157,7 @@ struct Cycle {
   MQ<T> mq;
   T* final_out = nullptr;  // where level 0's last sweep writes (row stride vstride(ndof0))
   bool waited_ready = false;  // the stream has waited for the coarse factorisation
+  int rc = STT_OK;            // of the coarse solves, which take the launch error with them
   RzFuse<T> rzf{};         // the PCG's dots for level 0's chained passes to take (rzf.rst set)
   bool mix_done = false;   // the pre-smoothing pass took r . z_old
   bool rz_done = false;    // the post-smoothing pass took r . z and set beta
@@ -282,7 +283,8 @@ struct Cycle {
       waited_ready = true;
     }
     if (co.tree) {
-      coarse_tree_solve<T>(h, nrows, b, x, vstride(lv.ndof), rst, st);
+      const int solved = coarse_tree_solve<T>(h, nrows, b, x, vstride(lv.ndof), rst, st);
+      if (rc == STT_OK) rc = solved;
       return;
     }
 #define STT_COARSE(NC)                                                                          \
@@ -1005,7 +1007,8 @@ static int run_vcycle(const stt_hier* h, SolveWS& w, int nrows, const double* r,
   if (rz_done) *rz_done = cyc.rz_done;
   if (res != zout)
     launch((rows_convert_kernel<T, T>), dim3(ew_blocks(n), nrows), kEwThreads, 0, st, res, vs, zout, vs, n, rst);
-  return check_launch("vcycle");
+  const int launched = check_launch("vcycle");
+  return cyc.rc != STT_OK ? cyc.rc : launched;
 }
 
 // Optional live timing of the plane-stress solves' steady-state p.Ap passes (the step's

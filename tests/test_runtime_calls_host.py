@@ -93,3 +93,50 @@ print(json.dumps(dict(rcs=rcs, launches=lib.fake_launches(b"mma_assemble_kernel"
 """, first=first, then=then)
     assert got["launches"] > 0 and 5 not in got["rcs"], got  # 5: a CUDA call failed
     assert got["lowest"] >= got["largest"], got
+
+
+CYCLE = r"""
+from oracle import sttopt_oracle as O
+
+d, nelx, nely, mce, prec, rows = (case[k] for k in ("d", "nelx", "nely", "mce", "prec", "rows"))
+KE = arr(O.plane_stress_KE(0.3) if d == 2 else O.diffusion_KE())
+wb = lib.stt_hier_workspace_bytes(I(d), I(nelx), I(nely), I(rows), I(mce), I(prec))
+h = P()
+rho = mem(rows * nelx * nely)
+assert lib.stt_hier_create(ctypes.byref(h), mem(wb, np.uint8), L(wb), I(d), I(nelx), I(nely), I(rows), rho,
+                           L(nelx * nely), None, L(0), None, KE, I(mce), I(prec), None) == 0, lib.stt_last_error()
+nd = d * (nelx + 1) * (nely + 1)
+nd += nd % 2
+r, z = mem(rows * nd), mem(rows * nd)
+ws = lib.stt_solve_workspace_bytes(h, I(rows), I(1))
+w = mem(ws, np.uint8)
+
+def vcycle():
+    return lib.stt_vcycle(h, I(rows), r, L(nd), z, L(nd), D(0.6), I(2), I(1), w, L(ws), None)
+
+def pcg():
+    rel, conv, n = mem(rows), mem(rows, np.int32), mem(1, np.int32)
+    return lib.stt_pcg_mg(h, I(rows), r, L(nd), z, L(nd), I(0), D(1e-8), I(5), D(0.6), I(2), I(1), I(0), I(0), I(0),
+                          rel, conv, n, w, L(ws), None)
+"""
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("d,nelx,nely,mce,kernel", [
+    (2, 40, 20, 200, "tree_solve_kernel"), (1, 40, 20, 200, "tree_solve_kernel"), (2, 16, 8, 700, "tree_solve_kernel"),
+    (2, 72, 70, 1300, "coarse_solve_kernel")])
+def test_a_refused_coarse_solve_fails_the_call(fake, d, nelx, nely, mce, kernel, prec):
+    """A coarse solve that does not run leaves the level's vector as it was: the V-cycle and the
+    PCG must say so, whatever the launches after it did, and a later call must not."""
+    got = fake(CYCLE + r"""
+kernel = case["kernel"].encode()
+before = [vcycle(), pcg(), lib.fake_launches(kernel)]
+lib.fake_refuse(kernel)
+refused = [vcycle(), pcg()]
+message = lib.stt_last_error().decode()
+lib.fake_refuse(b"")
+print(json.dumps(dict(before=before, refused=refused, message=message, after=[vcycle(), pcg()])))
+""", d=d, nelx=nelx, nely=nely, mce=mce, prec=prec, rows=2, kernel=kernel)
+    assert got["before"][:2] == [0, 0] and got["before"][2] > 0, got
+    assert got["refused"] == [5, 5] and "refused by the test" in got["message"], got  # STT_ERR_CUDA
+    assert got["after"] == [0, 0], got

@@ -596,9 +596,13 @@ __global__ void __cluster_dims__(kTreeCluster, 1, 1) __launch_bounds__(TreeRow<N
   extern __shared__ __align__(16) double sm[];
   const int srow = blockIdx.y;
   TreeRow<NB> tree;
+  // The factor is fetched beside the kernel before: it is complete when its solves are launched
+  // (the stream has waited for its event).  A row map is the caller's, and on a hierarchy of one
+  // level the kernel before may be the one that writes it.
+  if (row_map) grid_wait();
   tree.init(sm, blocks + (size_t)hier_row(row_map, hrows, srow) * nb * 4 * B * B, nb, staged);
-  tree.prefetch();  // beside the kernel before (the factor is complete when its solves are launched)
-  grid_wait();
+  tree.prefetch();
+  if (!row_map) grid_wait();
   if (rst && !rst[srow].active) {  // the whole cluster
     asm volatile("cp.async.wait_all;\n" ::: "memory");
     return;

@@ -77,10 +77,12 @@ STT_DEV T ldg(const T* p) {
 //
 // The solves' kernels are launched with programmatic stream serialisation: a kernel's blocks
 // may become resident while the kernel before it drains, and wait there.  Every thread of
-// every such kernel calls grid_wait() before anything else (an early return included), so
+// every such kernel calls grid_wait() before it touches memory (an early return included), so
 // that a grid's completion implies its predecessors'; it returns when the kernels before
-// have completed and their writes are visible, and lets the next kernel's blocks in.  A
-// kernel boundary of the solves' many short kernels costs about 1 us less that way.
+// have completed and their writes are visible, and lets the next kernel's blocks in.  The one
+// exception is the coarse solve, which fetches the factor first: that was written on another
+// stream and waited for by an event before the launch, and no kernel of this stream writes it.
+// A kernel boundary of the solves' many short kernels costs about 1 us less that way.
 STT_DEV void grid_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -464,7 +464,7 @@ struct SlotSums {
     __syncthreads();
   }
 };
-// Slots where they fit beside the assemble pass's tile at two blocks an SM.
+// Slots where they fit beside the advance pass's tile at two blocks an SM (advance_rows).
 template <int MB>
 constexpr bool use_slots() {
   return MB <= 24;
@@ -494,12 +494,29 @@ __host__ __device__ inline int packed_index(int i, int k, int m1) { return i * m
 __host__ __device__ inline int assemble_kp(int m, int nd) { return m + 2 * nd + (m + nd) * (m + nd + 1) / 2; }
 // Results: [gvec (m) | A (m x m) | then for each level h (m), sum of squares, max].
 __host__ __device__ inline int assemble_res(int m, int nd) { return m + m * m + nd * (m + 2); }
-// Its dynamic shared memory: the GG tile (or, later, the folded entries), 1/diagx, a
-// block-sum scratch, and when it forms gvec the row-sum slots or shuffle scratch.
-inline size_t assemble_smem(int m, int mb, int nd, bool need_g) {
-  const size_t rows = (size_t)gram_side(m, nd) * 8;
+// The GG tile's doubles (or, later, the folded entries'); `rows` of it are stored.
+__host__ __device__ inline int assemble_head(int m, int nd, int rows) {
+  const int tile = rows * kMmaLd8, fold = assemble_kp(m, nd);
+  return tile > fold ? tile : fold;
+}
+// Its dynamic shared memory: the tile, 1/diagx, a block-sum scratch, and when it forms gvec the
+// row-sum slots or shuffle scratch.
+inline size_t assemble_smem(int m, int mb, int nd, int rows, bool need_g) {
   const size_t tail = !need_g ? 0 : mb <= 24 ? (size_t)mb * kMmaThreads : (size_t)(kMmaThreads / 32) * kMmaMaxM;
-  return 8 * (std::max(rows * kMmaLd8, (size_t)assemble_kp(m, nd)) + kMmaThreads + 8 + tail);
+  return 8 * ((size_t)assemble_head(m, nd, rows) + kMmaThreads + 8 + tail);
+}
+inline int assemble_rows(int m, int nd) { return 8 * gram_side(m, nd); }  // with zero rows up to whole products
+// The advance pass's stored rows.  Its second delx row takes the padded tile of 23, 24, 47 and 48
+// constraints past half an SM's shared memory; without the padding two blocks fit (a fragment's
+// rows past the last repeat it, and their products are not read).  The update at 1M variables:
+// 12.1 -> 9.9, 11.3 -> 9.2, 25.1 -> 20.3 and 25.5 -> 20.5 ms.  With no more blocks than SMs the
+// padding stays: two of them, resident while the step pass drains, would share an SM that it
+// leaves idle (20000 variables, 47 constraints: 2.97 -> 3.36 ms).
+constexpr bool trims_rows(int mb) { return mb == 24 || mb == 48; }
+inline int advance_rows(int m, int mb, int blocks) {
+  constexpr size_t half_sm = (228 << 10) / 2 - (1 << 10) - 512;  // less the system's and the static share
+  const int padded = assemble_rows(m, 2);
+  return trims_rows(mb) && blocks > 148 && assemble_smem(m, mb, 2, padded, true) > half_sm ? m + 2 : padded;
 }
 inline int mma_bucket(int m) {
   return m <= 4 ? 4 : m <= 8 ? 8 : m <= 12 ? 12 : m <= 16 ? 16 : m <= 20 ? 20 : m <= 24 ? 24 : m <= 32 ? 32
@@ -511,7 +528,7 @@ inline int mma_bucket(int m) {
 //   gvec = P (1/ux1) + Q (1/xl1),  h = GG (delx / diagx),  A = GG diag(1/diagx) GG^T
 // with GG = P diag(1/ux2) - Q diag(1/xl2), and the sum of squares and largest magnitude
 // of the residual's n-sized parts.  A block's 256 variables write their GG column and
-// delx into a shared tile; A and h come from DMMA tiles of that tile.  Up to 31
+// delx into a shared tile; A and h come from DMMA tiles of that tile.  Up to 24
 // constraints each warp takes 32 of the tile's variables for every 8 x 8 tile and the
 // warps' sums are folded in warp order; above that the tiles are split among the warps.
 // gvec is formed only with need_g: after a line search it is the accepted candidate's,
@@ -528,7 +545,7 @@ template <int MB, bool G, bool ADV>
 __global__ void __launch_bounds__(kMmaThreads, 2) mma_assemble_kernel(
     MmaCols c, const double* x, const double* xsi, const double* eta, double* xo, double* xsio, double* etao,
     const double* __restrict__ dx, int pend, double t_pend, const double* tdev, double eps_pend, MVec lam0, MVec dlam,
-    double epsi, int need_g_arg, double* __restrict__ partials) {
+    double epsi, int need_g_arg, int rows, double* __restrict__ partials) {
   grid_wait();
   constexpr int ND = ADV ? 2 : 1;
   const bool need_g = ADV || need_g_arg;
@@ -546,10 +563,9 @@ __global__ void __launch_bounds__(kMmaThreads, 2) mma_assemble_kernel(
   constexpr int NT = T8 * (T8 + 1) / 2;
   constexpr bool KSPLIT = T8 <= 4;
   constexpr int TPW = KSPLIT ? NT : (NT + 7) / 8;  // tiles a warp accumulates
-  const int m = c.m, t8 = gram_side(m, ND), rows = t8 * 8, ntile = gram_tiles(m, ND);
-  const int head = max(rows * kMmaLd8, assemble_kp(m, ND));
-  double* gs = sm;                 // [rows][kMmaLd8]
-  double* ws = sm + head;          // [kMmaThreads]: 1 / diagx
+  const int m = c.m, t8 = gram_side(m, ND), ntile = gram_tiles(m, ND);
+  double* gs = sm;                               // [rows][kMmaLd8]
+  double* ws = sm + assemble_head(m, ND, rows);  // [kMmaThreads]: 1 / diagx
   double* wred = ws + kMmaThreads; // [8]
   double* tail = wred + 8;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -638,49 +654,58 @@ __global__ void __launch_bounds__(kMmaThreads, 2) mma_assemble_kernel(
 #pragma unroll
     for (int e = 0; e < ND; ++e) gs[(m + e) * kMmaLd8 + tid] = delx[e];
     ws[tid] = w;
-    // Up to 31 constraints a warp's tiles read only the 32 variables the warp wrote, so
-    // the warps need not wait for one another.
+    // Up to 24 constraints (the K-split) a warp's tiles read only the 32 variables the warp
+    // wrote, so the warps need not wait for one another.
     if constexpr (KSPLIT) {
       __syncwarp();
     } else {
       __syncthreads();
     }
-    if constexpr (KSPLIT) {
+    auto products = [&](auto trimmed) {
+      auto row = [&](int r) { return decltype(trimmed)::value ? min(r, rows - 1) : r; };
+      if constexpr (KSPLIT) {
 #pragma unroll 2
-      for (int k4 = 0; k4 < 8; ++k4) {
-        const int col = warp * 32 + k4 * 4 + fc;
-        const double wc = ws[col];
-        double a[T8], b[T8];
+        for (int k4 = 0; k4 < 8; ++k4) {
+          const int col = warp * 32 + k4 * 4 + fc;
+          const double wc = ws[col];
+          double a[T8], b[T8];
 #pragma unroll
-        for (int I = 0; I < T8; ++I) {
-          a[I] = I < t8 ? gs[(8 * I + fr) * kMmaLd8 + col] : 0.0;
-          b[I] = a[I] * wc;
-        }
-        int q = 0;
-#pragma unroll
-        for (int I = 0; I < T8; ++I)
-#pragma unroll
-          for (int K = I; K < T8; ++K, ++q)
-            if (K < t8) dmma_f64(acc[q], a[I], b[K]);
-      }
-    } else {
-#pragma unroll
-      for (int q = 0; q < TPW; ++q) {
-        const int t = warp + 8 * q;
-        if (t < ntile) {
-          int I = 0, rem = t;
-          while (rem >= t8 - I) {
-            rem -= t8 - I;
-            ++I;
+          for (int I = 0; I < T8; ++I) {
+            a[I] = I < t8 ? gs[row(8 * I + fr) * kMmaLd8 + col] : 0.0;
+            b[I] = a[I] * wc;
           }
-          const int K = I + rem;
-          const double* ga = gs + (8 * I + fr) * kMmaLd8 + fc;
-          const double* gb = gs + (8 * K + fr) * kMmaLd8 + fc;
+          int q = 0;
+#pragma unroll
+          for (int I = 0; I < T8; ++I)
+#pragma unroll
+            for (int K = I; K < T8; ++K, ++q)
+              if (K < t8) dmma_f64(acc[q], a[I], b[K]);
+        }
+      } else {
+#pragma unroll
+        for (int q = 0; q < TPW; ++q) {
+          const int t = warp + 8 * q;
+          if (t < ntile) {
+            int I = 0, rem = t;
+            while (rem >= t8 - I) {
+              rem -= t8 - I;
+              ++I;
+            }
+            const int K = I + rem;
+            const double* ga = gs + row(8 * I + fr) * kMmaLd8 + fc;
+            const double* gb = gs + row(8 * K + fr) * kMmaLd8 + fc;
 #pragma unroll 4
-          for (int k4 = 0; k4 < kMmaThreads / 4; ++k4)
-            dmma_f64(acc[q], ga[4 * k4], gb[4 * k4] * ws[4 * k4 + fc]);
+            for (int k4 = 0; k4 < kMmaThreads / 4; ++k4)
+              dmma_f64(acc[q], ga[4 * k4], gb[4 * k4] * ws[4 * k4 + fc]);
+          }
         }
       }
+    };
+    if constexpr (ADV && trims_rows(MB)) {
+      if (rows < 8 * t8) products(std::true_type{});
+      else products(std::false_type{});
+    } else {
+      products(std::false_type{});
     }
     if constexpr (KSPLIT) {
       __syncwarp();
@@ -962,7 +987,7 @@ constexpr int kMaxHalvings = 50;   // sttopt/mma.py:289
 constexpr int kMaxNewton = 200;    // sttopt/mma.py:442
 
 using AsmFn = void (*)(MmaCols, const double*, const double*, const double*, double*, double*, double*, const double*,
-                       int, double, const double*, double, MVec, MVec, double, int, double*);
+                       int, double, const double*, double, MVec, MVec, double, int, int, double*);
 using StepFn = void (*)(MmaCols, const double*, const double*, const double*, MVec, MVec, double, double, double*,
                         double*, unsigned*, double*);
 using SearchFn = void (*)(MmaCols, const double*, const double*, const double*, const double*, double, const double*,
@@ -1237,8 +1262,9 @@ int device_subsolv(const MmaCols& c, const MData& D, double epsimin, const MmaWs
   const int ga = (int)std::min<long long>(tiles, kAsmBlocks), gp = (int)std::min<long long>(tiles, kPassBlocks);
   const Kernels k = pick_kernels<G>(m);
   const int mb = mma_bucket(m);
-  const size_t smem_g = assemble_smem(m, mb, 1, true), smem = assemble_smem(m, mb, 1, false);
-  const size_t smem_adv = assemble_smem(m, mb, 2, true);
+  const int rows1 = assemble_rows(m, 1), rows2 = advance_rows(m, mb, ga);
+  const size_t smem_g = assemble_smem(m, mb, 1, rows1, true), smem = assemble_smem(m, mb, 1, rows1, false);
+  const size_t smem_adv = assemble_smem(m, mb, 2, rows2, true);
   STT_TRY(k.allow_assemble());
   STT_TRY(k.allow_advance());
   STT_TRY(check_cuda(cudaMemsetAsync(w.counters, 0, 4 * sizeof(unsigned), st), "mma: counters"));
@@ -1278,7 +1304,7 @@ int device_subsolv(const MmaCols& c, const MData& D, double epsimin, const MmaWs
   auto assemble = [&](double epsi, double& ssn, double& mxn) -> int {
     const int need_g = have_g ? 0 : 1;
     launch(k.assemble, ga, kMmaThreads, need_g ? smem_g : smem, st, c, px, pxsi, peta, px, pxsi, peta, w.dx, pend,
-           t_pend, nullptr, eps_pend, mvec(S.lam), MVec{}, epsi, need_g, w.partials);
+           t_pend, nullptr, eps_pend, mvec(S.lam), MVec{}, epsi, need_g, rows1, w.partials);
     pend = 0;
     STT_TRY(check_launch("mma_assemble_kernel"));
     STT_TRY(fold(1));
@@ -1334,7 +1360,7 @@ int device_subsolv(const MmaCols& c, const MData& D, double epsimin, const MmaWs
              w.counters + 1, res_step);
       STT_TRY(check_launch("mma_step_kernel"));
       launch(k.advance, ga, kMmaThreads, smem_adv, st, c, px, pxsi, peta, qx, qxsi, qeta, w.dx, 1, 0.0, res_step + 3,
-             epsi, lam_now, dlam, epsi, 1, w.partials);
+             epsi, lam_now, dlam, epsi, 1, rows2, w.partials);
       STT_TRY(check_launch("mma_assemble_kernel"));
       STT_TRY(fold(2));
       STT_TRY(fetch("mma: step and first candidate"));

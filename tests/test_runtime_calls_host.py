@@ -68,7 +68,7 @@ def fake(tmp_path_factory):
 
 
 MMA = r"""
-n = 600
+n = case.get("n", 600)
 
 def subsolv(m):
     ws = lib.stt_mma_workspace_bytes(m, L(n))
@@ -140,3 +140,15 @@ print(json.dumps(dict(before=before, refused=refused, message=message, after=[vc
     assert got["before"][:2] == [0, 0] and got["before"][2] > 0, got
     assert got["refused"] == [5, 5] and "refused by the test" in got["message"], got  # STT_ERR_CUDA
     assert got["after"] == [0, 0], got
+
+
+@pytest.mark.parametrize("m", [22, 23, 24, 46, 47, 48])
+def test_the_advance_pass_leaves_room_for_two_blocks_an_sm(fake, m):
+    """With more blocks than SMs: 228 KB an SM, less 1 KB a block for the system and 0.5 KB of
+    static memory."""
+    got = fake(MMA + r"""
+rc = subsolv(case["m"])
+print(json.dumps(dict(rc=rc, smem=lib.fake_largest_smem(b"ELb1EE"), launches=lib.fake_launches(b"ELb1EE"))))
+""", m=m, n=148 * 256 + 1)
+    assert got["rc"] == 0 and got["launches"] > 0
+    assert 2 * (got["smem"] + 1536) <= 228 << 10, got

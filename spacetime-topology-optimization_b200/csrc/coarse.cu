@@ -10,13 +10,14 @@
 //     forward   y_i = X_i b_i,  b_{i-s} -= F_l^T y_i,  b_{i+s} -= F_r^T y_i
 //     backward  x_i = X_i^T (y_i - F_l x_{i-s} - F_r x_{i+s}).
 // A chain over the lines (block k needs block k - 1) has nb dependent steps each way; this
-// order has log2(nb), and the steps of one stride run side by side on a cluster of eight
-// CTAs a row, which exchange through distributed shared memory.
+// order has log2(nb), and the steps of one stride run side by side on a cluster of up to eight
+// CTAs a row (fewer where there are many rows), which exchange through distributed shared memory.
 #include "coarse.h"
 
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <mutex>
 
 #include "errors.h"
 #include "smem.h"
@@ -25,9 +26,8 @@ namespace stt {
 
 namespace cg = cooperative_groups;
 
-constexpr int kTreeCluster = 8;                    // CTAs a row
-constexpr int kTreeGroups = 2;                     // thread groups of 4 B threads a CTA
-constexpr int kTreeAll = kTreeCluster * kTreeGroups;
+constexpr int kTreeCluster = 8;  // CTAs a row, at most
+constexpr int kTreeGroups = 2;   // thread groups of 4 B threads a CTA
 constexpr int kTreeMaxUnknowns = 5376;   // nb * B, held in every CTA's shared memory
 constexpr size_t kTreeSmem = 225 << 10;  // dynamic shared memory a CTA of the solve may take
 
@@ -252,13 +252,12 @@ STT_DEV void tree_tiles(const double (&acc)[NB][2], Put put) {
 
 // One row's factorisation on a cluster.  Latency-bound: a block's elimination is a chain of
 // B pivots (about B/8 tile steps of one warp) and three B^3 products on the FP64 tensor
-// cores; a stride's blocks are spread over the eight CTAs.  132 us for 33 lines of 40
-// unknowns at 1 to 16 rows, 96 us for 46 lines of 32, where the banded factorisation (a chain
+// cores; a stride's blocks are spread over the row's CTAs.  132 us for 33 lines of 40
+// unknowns at 1 to 15 rows, 96 us for 46 lines of 32, where the banded factorisation (a chain
 // over all unknowns on one CTA a row) took 871 and 1118 us.  Slots of block i: 0 the matrix
 // block, then X_i; 1 F_l; 2 the coupling to the left neighbour still present; 3 F_r.
 template <int NB>
-__global__ void __cluster_dims__(kTreeCluster, 1, 1) __launch_bounds__(256)
-    tree_factor_kernel(double* blocks, int nb, int* status) {
+__global__ void __launch_bounds__(256) tree_factor_kernel(double* blocks, int nb, int* status) {
   constexpr int B = 8 * NB, BB = B * B;
   extern __shared__ __align__(16) unsigned char tree_raw[];
   TreeShared<NB>& S = *reinterpret_cast<TreeShared<NB>*>(tree_raw);
@@ -313,7 +312,7 @@ __global__ void __cluster_dims__(kTreeCluster, 1, 1) __launch_bounds__(256)
   };
 
   for (int s = 1; s < nb; s *= 2) {
-    const int step = 2 * s * kTreeCluster;
+    const int step = 2 * s * (int)gridDim.x;
     int last = -1;
     for (int i = s * (2 * rank + 1); i < nb; i += step) {
       const int r = i + s < nb ? i + s : -1;
@@ -361,9 +360,10 @@ STT_DEV void tree_cp16(void* smem, const void* gmem) {
 // Shared memory of a CTA (doubles): the solution in block order, then for each group its
 // blocks' right-hand sides, the updates that arrive for them and scratch, then the staged
 // matrices.
-__host__ __device__ inline int tree_own(int nb) { return (nb + kTreeAll - 1) / kTreeAll; }  // blocks a group
-__host__ __device__ inline size_t tree_vectors(int nb, int B) {
-  return (size_t)nb * B + kTreeGroups * (5 * (size_t)tree_own(nb) * B + 10 * B);
+// (all: the row's thread groups)
+__host__ __device__ inline int tree_own(int nb, int all) { return (nb + all - 1) / all; }  // blocks a group
+__host__ __device__ inline size_t tree_vectors(int nb, int B, int all) {
+  return (size_t)nb * B + kTreeGroups * (5 * (size_t)tree_own(nb, all) * B + 10 * B);
 }
 __host__ __device__ inline size_t tree_task(int B) { return 3 * (size_t)B * B; }  // X, F_l, F_r of one block
 
@@ -379,7 +379,7 @@ __host__ __device__ inline size_t tree_task(int B) { return 3 * (size_t)B * B; }
 // same number.  A block's right-hand side lives in the CTA whose group owns it; its two
 // neighbours' updates arrive there by remote stores into a buffer a side (two sets, used by
 // alternate strides, so that a set is read before it is written again) and are added by the
-// owner in a fixed order; a solution block is written to all eight CTAs.
+// owner in a fixed order; a solution block is written to all of the row's CTAs.
 template <int NB>
 struct TreeRow {
   static constexpr int B = 8 * NB, NC = 2 * NB, BB = B * B, kGroup = 4 * B;
@@ -387,6 +387,7 @@ struct TreeRow {
 
   const double* bh;  // the row's factor [nb][4][B][B]
   int nb, staged, own, levels, rank, grp, t, gi;
+  int lg, all;  // the row's thread groups, 2^lg
   double *vx, *vb, *in, *tv, *part, *stage;
 
   STT_DEV void init(double* sm, const double* factor, int nblocks, int nstaged) {
@@ -394,7 +395,9 @@ struct TreeRow {
     bh = factor;
     nb = nblocks;
     staged = nstaged;
-    own = tree_own(nb);
+    all = (int)gridDim.x * kTreeGroups;
+    lg = 31 - __clz(all);
+    own = tree_own(nb, all);
     levels = 0;
     while ((1 << levels) < nb) ++levels;
     rank = (int)cluster.block_rank();
@@ -406,11 +409,11 @@ struct TreeRow {
     in = vb + (size_t)kTreeGroups * own * B;        // [set][side][grp][own][B]
     tv = in + (size_t)4 * kTreeGroups * own * B + grp * 10 * B;
     part = tv + 2 * B;
-    stage = vx + tree_vectors(nb, B) + (size_t)grp * staged * 3 * BB;
+    stage = vx + tree_vectors(nb, B, all) + (size_t)grp * staged * 3 * BB;
   }
 
   // blocks in the order of elimination: those of stride 2^l are numbers base(l) .. base(l + 1),
-  // the root (block 0) is the last; number o is the o / kTreeAll-th block of group o % kTreeAll
+  // the root (block 0) is the last; number o is the o / all-th block of group o % all
   STT_DEV int base(int l) const { return nb - ((nb + (1 << l) - 1) >> l); }
   STT_DEV int number(int e) const {
     if (e == 0) return nb - 1;
@@ -419,17 +422,17 @@ struct TreeRow {
   }
   STT_DEV int block_of(int o, int l) const { return (1 << l) * (2 * (o - base(l)) + 1); }
   // where block e's vectors live: the CTA, and the offset in an array [grp][own][B]
-  STT_DEV int owner(int e) const { return (number(e) % kTreeAll) / kTreeGroups; }
+  STT_DEV int owner(int e) const { return (number(e) & (all - 1)) / kTreeGroups; }
   STT_DEV int place(int e) const {
     const int o = number(e);
-    return ((o % kTreeGroups) * own + o / kTreeAll) * B;
+    return ((o % kTreeGroups) * own + (o >> lg)) * B;
   }
   STT_DEV double* updates(int set, int side) const { return in + (size_t)((2 * set + side) * kTreeGroups) * own * B; }
   // calls f(block, j) for the group's blocks in their order, j = 0, 1, ...
   template <typename F>
   STT_DEV void each_block(F f) const {
     int l = 0, j = 0;
-    for (int o = gi; o < nb; o += kTreeAll, ++j) {
+    for (int o = gi; o < nb; o += all, ++j) {
       while (l < levels && o >= base(l + 1)) ++l;
       f(o == nb - 1 ? 0 : block_of(o, l), j, l);
     }
@@ -510,7 +513,7 @@ struct TreeRow {
       const int s = 1 << l, end = base(l + 1);
       double* inL = updates(l & 1, 0);
       double* inR = updates(l & 1, 1);
-      for (; o < end; o += kTreeAll, ++j) {
+      for (; o < end; o += all, ++j) {
         const int i = block_of(o, l);
         const bool right = i + s < nb;
         wait_stage(j == 0);
@@ -535,7 +538,7 @@ struct TreeRow {
       // the updates of the own blocks that are left
       if (t < B) {
         int l2 = l + 1, j2 = j;
-        for (int o2 = o; o2 < nb; o2 += kTreeAll, ++j2) {
+        for (int o2 = o; o2 < nb; o2 += all, ++j2) {
           while (l2 < levels && o2 >= base(l2 + 1)) ++l2;
           const int a = j2 * B + t;
           if (o2 == nb - 1)
@@ -550,7 +553,8 @@ struct TreeRow {
         const double v = parts(part, t);
         if (share)
 #pragma unroll
-          for (int rk = 0; rk < kTreeCluster; ++rk) cluster.map_shared_rank(vx, rk)[i * B + t] = v;
+          for (int rk = 0; rk < kTreeCluster; ++rk)
+            if (rk < (int)gridDim.x) cluster.map_shared_rank(vx, rk)[i * B + t] = v;
         publish(i, t, v);
       }
     };
@@ -565,12 +569,12 @@ struct TreeRow {
       group_sync<NB>(grp);
       finish(0, nb > 1);
     }
-    o -= kTreeAll;
+    o -= all;
     --j;
     for (int l = levels - 1; l >= 0; --l) {
       const int s = 1 << l, begin = base(l);
       cluster.sync();
-      for (; o >= begin; o -= kTreeAll, --j) {
+      for (; o >= begin; o -= all, --j) {
         const int i = block_of(o, l);
         group_sync<NB>(grp);
         double z = row_dot(matrix(j, i, 1), vx + (i - s) * B);
@@ -588,7 +592,7 @@ struct TreeRow {
 
 // One row's coarse solve on a cluster (TreeRow), between global vectors.
 template <int NB, int D, typename T>
-__global__ void __cluster_dims__(kTreeCluster, 1, 1) __launch_bounds__(TreeRow<NB>::kThreads)
+__global__ void __launch_bounds__(TreeRow<NB>::kThreads)
     tree_solve_kernel(const T* __restrict__ b, T* __restrict__ x, long long rs, const double* __restrict__ blocks,
                       int nb, int staged, int by_col, int nnx, int nny, const uint8_t* __restrict__ fixed,
                       const int* __restrict__ row_map, int hrows, const RowState* __restrict__ rst) {
@@ -666,11 +670,104 @@ void coarse_plan(const LevelDesc& c, int d, CoarseDesc& co) {
   co.nb = (co.n + co.B - 1) / co.B;
 }
 
+// How many clusters of `cluster` CTAs the device holds at once (several kinds of launch a kernel:
+// the answers are kept, at most kMax of them).
+template <auto Kernel>
+static int resident_clusters(int cluster, int threads, size_t smem, int* n) {
+  struct Known {
+    int dev, cluster, n;
+    size_t smem;
+  };
+  constexpr int kMax = 64;
+  static std::mutex mu;
+  static Known known[kMax];
+  static int count = 0;
+  int dev = 0;
+  STT_TRY(check_cuda(cudaGetDevice(&dev), "cudaGetDevice"));
+  std::lock_guard<std::mutex> lock(mu);
+  for (int i = 0; i < count; ++i)
+    if (known[i].dev == dev && known[i].cluster == cluster && known[i].smem == smem) {
+      *n = known[i].n;
+      return STT_OK;
+    }
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = (unsigned)cluster;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(cluster);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  STT_TRY(check_cuda(cudaOccupancyMaxActiveClusters(n, Kernel, &cfg), "resident clusters"));
+  // clusters of eight with more than one CTA an SM leave gaps: of 33 and of 48, 28 and 40 ran at once
+  if (cluster == kTreeCluster && *n * cluster > 148) *n -= *n / 8;
+  if (count == kMax) count = 0;
+  known[count++] = Known{dev, cluster, *n, smem};
+  return STT_OK;
+}
+
+// Dependent block eliminations of one sweep over the strides with `units` blocks side by side.
+static int tree_steps(int nb, int units) {
+  int steps = 1;  // the root
+  for (int n = nb; n > 1; n = (n + 1) / 2) steps += (n / 2 + units - 1) / units;
+  return steps;
+}
+
+// The launch that is expected to end first: its waves of resident clusters times a row's steps,
+// times what a step costs there.  Fewer CTAs a row take more steps but let more rows run at once
+// (15 clusters of eight, 33 of four, 74 of two on B200's 148 SMs at one CTA each).  A V-cycle of a
+// one-level hierarchy, 33 lines of 40 unknowns, always eight CTAs -> this rule: 16 rows 51 -> 39 us,
+// 33 rows 74 -> 45, 64 rows 122 -> 55, 128 rows 223 -> 86 (the chain over the lines: 147 to 162); 27
+// lines of 54 at 128 rows 404 -> 179 (204), their factorisation 2.2 -> 1.35 ms (1.33).  The
+// rows' results do not depend on it.
+struct TreeLaunch {
+  int cluster = 0, staged = 0;
+  size_t smem = 0;
+  long long cost = 0;
+  void consider(int rows, int resident, int cl, int st, size_t bytes, int row_cost) {
+    if (resident < 1) return;
+    const long long c = (long long)((rows + resident - 1) / resident) * row_cost;
+    if (cluster == 0 || c < cost) *this = TreeLaunch{cl, st, bytes, c};
+  }
+};
+
 template <int NB>
 static int tree_factor(const CoarseDesc& co, int hrows, int* status, cudaStream_t st) {
+  constexpr int kThreads = 256;
   STT_TRY(allow_smem<tree_factor_kernel<NB>>());
-  tree_factor_kernel<NB><<<dim3(kTreeCluster, hrows), 256, sizeof(TreeShared<NB>), st>>>(co.blocks, co.nb, status);
+  TreeLaunch best;
+  for (int cl = kTreeCluster; cl >= 1; cl /= 2) {
+    int n = 0;
+    STT_TRY(resident_clusters<tree_factor_kernel<NB>>(cl, kThreads, sizeof(TreeShared<NB>), &n));
+    best.consider(hrows, n, cl, 0, sizeof(TreeShared<NB>), tree_steps(co.nb, cl));
+  }
+  if (best.cluster == 0) return set_error(STT_ERR_CUDA, "coarse factor: no cluster fits the device");
+  launch_clusters(tree_factor_kernel<NB>, best.cluster, dim3(best.cluster, hrows), kThreads, best.smem, st, false,
+                  co.blocks, co.nb, status);
   return check_launch("coarse factor");
+}
+
+// A solve's launch: each cluster size with as many blocks staged as fit its CTAs, and with none
+// (more CTAs an SM).  A step without its block staged takes about 1.4 times as long.
+template <int NB, int D, typename T>
+static int tree_launch(const CoarseDesc& co, int nrows, TreeLaunch& best) {
+  STT_TRY(allow_smem<tree_solve_kernel<NB, D, T>>());
+  const size_t task = 8 * kTreeGroups * tree_task(co.B);
+  for (int cl = kTreeCluster; cl >= 1; cl /= 2) {
+    const int all = cl * kTreeGroups, own = tree_own(co.nb, all), steps = tree_steps(co.nb, all);
+    const size_t vec = 8 * tree_vectors(co.nb, co.B, all);
+    if (vec > kTreeSmem) break;
+    const int most = (int)std::min<size_t>(own, (kTreeSmem - vec) / task);
+    for (int st : {most, 0}) {
+      int n = 0;
+      STT_TRY((resident_clusters<tree_solve_kernel<NB, D, T>>(cl, TreeRow<NB>::kThreads, vec + st * task, &n)));
+      best.consider(nrows, n, cl, st, vec + st * task, steps * (st == own ? 5 : 7));
+    }
+    if (cl == kTreeCluster && most == own && best.cost == 5 * steps) break;  // one wave: nothing is faster
+  }
+  return best.cluster ? STT_OK : set_error(STT_ERR_CUDA, "coarse solve: no cluster fits the device");
 }
 
 template <int NB, int D, typename T>
@@ -678,11 +775,11 @@ static int tree_solve(const stt_hier* h, int nrows, const T* b, T* x, long long 
                       cudaStream_t st) {
   const LevelDesc& lv = h->lv[h->nlevels - 1];
   const CoarseDesc& co = h->co;
-  STT_TRY(allow_smem<tree_solve_kernel<NB, D, T>>());
-  const size_t vec = 8 * tree_vectors(co.nb, co.B), task = 8 * kTreeGroups * tree_task(co.B);
-  const int staged = (int)std::min<size_t>(tree_own(co.nb), (kTreeSmem - vec) / task);
-  launch((tree_solve_kernel<NB, D, T>), dim3(kTreeCluster, nrows), TreeRow<NB>::kThreads, vec + staged * task, st, 
-      b, x, rs, co.blocks, co.nb, staged, co.by_col, lv.nnx, lv.nny, lv.fixed, h->row_map, h->hrows, rst);
+  TreeLaunch l;
+  STT_TRY((tree_launch<NB, D, T>(co, nrows, l)));
+  launch_clusters((tree_solve_kernel<NB, D, T>), l.cluster, dim3(l.cluster, nrows), TreeRow<NB>::kThreads, l.smem, st,
+                  true, b, x, rs, co.blocks, co.nb, l.staged, co.by_col, lv.nnx, lv.nny, lv.fixed, h->row_map, h->hrows,
+                  rst);
   return check_launch("coarse solve");
 }
 

@@ -103,6 +103,26 @@ inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cud
   cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(std::forward<A>(args))...);
 }
 
+// The same in clusters of `cluster` blocks along x; `dependent` as above.
+template <typename... P, typename... A>
+inline void launch_clusters(void (*kernel)(P...), int cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                            bool dependent, A&&... args) {
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)cluster;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = at;
+  cfg.numAttrs = dependent ? 2 : 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(std::forward<A>(args))...);
+}
+
 // ---- block reductions (kNT threads) ---------------------------------------------
 
 STT_DEV double warp_sum(double v) {

@@ -14,7 +14,7 @@ namespace {
 struct Kernel {
   std::string name;
   size_t ceiling = 48 << 10, lowest = 1 << 30, largest = 0;  // lowest: of the ceilings that were set
-  int launches = 0;
+  int launches = 0, cluster = 0;  // cluster: CTAs along x, of the last launch
 };
 std::map<const void*, Kernel>& kernels() {
   static auto* k = new std::map<const void*, Kernel>();
@@ -64,6 +64,10 @@ size_t fake_lowest_ceiling(const char* part) {
   for (const Kernel* k = nullptr; (k = find(part, k));) n = k->lowest < n ? k->lowest : n;
   return n;
 }
+int fake_cluster(const char* part) {
+  const Kernel* k = find(part, nullptr);
+  return k ? k->cluster : 0;
+}
 void fake_forget() {
   for (auto& e : kernels()) e.second.launches = 0, e.second.largest = 0;
 }
@@ -92,6 +96,8 @@ cudaError_t __cudaPopCallConfiguration(dim3* grid, dim3* block, size_t* smem, vo
 }
 cudaError_t cudaLaunchKernel(const void* fn, dim3, dim3, void**, size_t smem, cudaStream_t) { return launched(fn, smem); }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* fn, void**) {
+  for (unsigned i = 0; i < c->numAttrs; ++i)
+    if (c->attrs[i].id == cudaLaunchAttributeClusterDimension) kernels()[fn].cluster = (int)c->attrs[i].val.clusterDim.x;
   return launched(fn, c->dynamicSmemBytes);
 }
 cudaError_t cudaGetLastError() {
@@ -110,6 +116,9 @@ cudaError_t cudaFuncSetAttribute(const void* fn, cudaFuncAttribute at, int v) {
   k.ceiling = (size_t)v;
   if (k.ceiling < k.lowest) k.lowest = k.ceiling;
   return cudaSuccess;
+}
+cudaError_t cudaOccupancyMaxActiveClusters(int* n, const void*, const cudaLaunchConfig_t* c) {
+  return *n = 120 / (int)c->attrs[0].val.clusterDim.x, cudaSuccess;
 }
 cudaError_t cudaGetDevice(int* d) { return *d = 0, cudaSuccess; }
 cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) { return *v = 227 << 10, cudaSuccess; }

@@ -142,6 +142,21 @@ print(json.dumps(dict(before=before, refused=refused, message=message, after=[vc
     assert got["after"] == [0, 0], got
 
 
+@pytest.mark.parametrize("rows", [1, 15, 16, 30, 31, 60, 120])
+@pytest.mark.parametrize("d,nelx,nely", [(2, 32, 16), (2, 26, 26), (1, 32, 16)])
+def test_the_coarse_solve_runs_all_rows_at_once_where_it_can(fake, d, nelx, nely, rows):
+    """The runtime here holds 120 CTAs of any cluster size.  A row takes as many as leave room for
+    all rows (twice as many rows as clusters would run one half after the other)."""
+    got = fake(CYCLE + r"""
+lib.fake_forget()
+rc = vcycle()
+print(json.dumps(dict(rc=rc, solve=lib.fake_cluster(b"tree_solve_kernel"))))
+""", d=d, nelx=nelx, nely=nely, mce=700, prec=0, rows=rows)
+    assert got["rc"] == 0 and got["solve"] in (1, 2, 4, 8), got
+    assert rows * got["solve"] <= 120, got
+    assert rows > 15 or got["solve"] == 8, got
+
+
 @pytest.mark.parametrize("m", [22, 23, 24, 46, 47, 48])
 def test_the_advance_pass_leaves_room_for_two_blocks_an_sm(fake, m):
     """With more blocks than SMs: 228 KB an SM, less 1 KB a block for the system and 0.5 KB of

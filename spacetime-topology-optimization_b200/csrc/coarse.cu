@@ -73,24 +73,47 @@ STT_DEV double line_entry(const double* __restrict__ sn, const uint8_t* __restri
   return sn[(size_t)(blk * D * D + i * D + j) * nnode + n];
 }
 
-// Diagonal blocks (slot 0) and the couplings to the previous line (slot 2), one CTA a line.
-template <int D>
+// A block's unknowns: `per` grid lines of `line` dofs each, one after the other (the last block may
+// have fewer lines).
+struct TreeBlock {
+  int per, line, lines;
+  // unknown i of block k as grid line and dof on it; false past the last
+  STT_DEV bool at(int k, int i, int& row, int& dof) const {
+    const int q = i / line, r = k * per + q;
+    dof = i - q * line;
+    row = r;
+    return q < per && r < lines;
+  }
+};
+
+// Diagonal blocks (slot 0) and the couplings to the previous block (slot 2), one CTA a block.
+template <int D, bool SHARED>
 __global__ void __launch_bounds__(256) tree_assemble_kernel(const double* __restrict__ st,
                                                             const uint8_t* __restrict__ fixed, int nnx, int nny,
-                                                            int by_col, int B, double* __restrict__ blocks) {
+                                                            int by_col, int B, double* __restrict__ blocks,
+                                                            TreeBlock of) {
   const int k = blockIdx.x, h = blockIdx.y, nb = gridDim.x;
   const long long nnode = (long long)nnx * nny;
-  const int used = D * (by_col ? nny : nnx);
   const double* sn = st + (size_t)h * 5 * D * D * nnode;
   double* blk = blocks + ((size_t)h * nb + k) * 4 * B * B;
+  // between dofs p and q of lines l and m
+  auto entry = [&](int l, int p, int m, int q) {
+    const int pa = p / D, i = p - pa * D, pb = q / D, j = q - pb * D;
+    const int ra = by_col ? pa : l, ca = by_col ? l : pa;
+    return line_entry<D>(sn, fixed, nnode, nnx, ra, ca, i, by_col ? pb : m, by_col ? m : pb, j);
+  };
   for (int t = threadIdx.x; t < B * B; t += 256) {
     const int ii = t / B, jj = t - ii * B;
     double v = ii == jj ? 1.0 : 0.0, w = 0.0;  // the padding is an identity
-    if (ii < used && jj < used) {
-      const int pa = ii / D, i = ii - pa * D, pb = jj / D, j = jj - pb * D;
-      const int ra = by_col ? pa : k, ca = by_col ? k : pa;
-      v = line_entry<D>(sn, fixed, nnode, nnx, ra, ca, i, by_col ? pb : k, by_col ? k : pb, j);
-      if (k > 0) w = line_entry<D>(sn, fixed, nnode, nnx, ra, ca, i, by_col ? pb : k - 1, by_col ? k - 1 : pb, j);
+    if constexpr (SHARED) {
+      int l, m, p, q;
+      if (of.at(k, ii, l, p)) {
+        if (of.at(k, jj, m, q)) v = entry(l, p, m, q);
+        if (k > 0 && of.at(k - 1, jj, m, q)) w = entry(l, p, m, q);
+      }
+    } else if (ii < of.line && jj < of.line) {
+      v = entry(k, ii, k, jj);
+      if (k > 0) w = entry(k, ii, k - 1, jj);
     }
     blk[t] = v;
     blk[(size_t)2 * B * B + t] = w;
@@ -590,12 +613,14 @@ struct TreeRow {
   }
 };
 
-// One row's coarse solve on a cluster (TreeRow), between global vectors.
-template <int NB, int D, typename T>
+// One row's coarse solve on a cluster (TreeRow), between global vectors.  SHARED: a block may hold
+// several grid lines (24 or 32 unknowns; without it the index arithmetic of one line a block is
+// simpler, and the kernel 0.7 us shorter).
+template <int NB, int D, typename T, bool SHARED>
 __global__ void __launch_bounds__(TreeRow<NB>::kThreads)
     tree_solve_kernel(const T* __restrict__ b, T* __restrict__ x, long long rs, const double* __restrict__ blocks,
                       int nb, int staged, int by_col, int nnx, int nny, const uint8_t* __restrict__ fixed,
-                      const int* __restrict__ row_map, int hrows, const RowState* __restrict__ rst) {
+                      const int* __restrict__ row_map, int hrows, const RowState* __restrict__ rst, TreeBlock of) {
   constexpr int B = 8 * NB;
   extern __shared__ __align__(16) double sm[];
   const int srow = blockIdx.y;
@@ -614,7 +639,13 @@ __global__ void __launch_bounds__(TreeRow<NB>::kThreads)
   const T* bs = b + (size_t)srow * rs;
   T* xs = x + (size_t)srow * rs;
   const int used = D * (by_col ? nny : nnx);
+  auto has = [&](int k, int ii) {
+    if constexpr (!SHARED) return ii < used;
+    int row, dof;
+    return of.at(k, ii, row, dof);
+  };
   auto dof_of = [&](int k, int ii, long long& node, int& d) {
+    if constexpr (SHARED) of.at(k, ii, k, ii);
     const int pos = ii / D;
     d = ii - pos * D;
     node = by_col ? (long long)pos * nnx + k : (long long)k * nnx + pos;
@@ -622,7 +653,7 @@ __global__ void __launch_bounds__(TreeRow<NB>::kThreads)
   tree.each_block([&](int i, int j, int) {
     if (tree.t >= B) return;
     double v = 0.0;
-    if (tree.t < used) {
+    if (has(i, tree.t)) {
       long long node;
       int d;
       dof_of(i, tree.t, node, d);
@@ -632,7 +663,7 @@ __global__ void __launch_bounds__(TreeRow<NB>::kThreads)
   });
   cg::this_cluster().sync();
   tree.solve([&](int i, int ii, double v) {
-    if (ii >= used) return;
+    if (!has(i, ii)) return;
     long long node;
     int d;
     dof_of(i, ii, node, d);
@@ -656,14 +687,18 @@ __global__ void __launch_bounds__(TreeRow<NB>::kThreads)
 
 // Lines of up to 64 unknowns go by odd-even elimination; wider ones (a coarsest grid of
 // more than ~700 elements) and very long ones by the banded factorisation, whose blocks
-// are a multiple of 32 no smaller than the half bandwidth.
+// are a multiple of 32 no smaller than the half bandwidth.  Many short lines go several to a
+// block of up to 32 unknowns (a step costs hardly more than with 8, and there are fewer): 601
+// lines of 2 unknowns one by one took 91 us a V-cycle at 1 row and 500 at 128, the banded chain
+// 82 and 116, in blocks of 16 lines 28 and 96.
 void coarse_plan(const LevelDesc& c, int d, CoarseDesc& co) {
   co.n = (int)c.ndof;
   co.by_col = c.nny < c.nnx ? 1 : 0;
   const int nmin = co.by_col ? c.nny : c.nnx, lines = co.by_col ? c.nnx : c.nny;
-  co.B = (d * nmin + 7) / 8 * 8;
-  co.nb = lines;
-  co.tree = (co.B <= 64 && (long long)co.B * lines <= kTreeMaxUnknowns) ? 1 : 0;
+  co.per = lines > 64 ? std::max(1, 32 / (d * nmin)) : 1;  // (more than one: 22 to 32 unknowns)
+  co.B = (co.per * d * nmin + 7) / 8 * 8;
+  co.nb = (lines + co.per - 1) / co.per;
+  co.tree = (co.B <= 64 && (long long)co.B * co.nb <= kTreeMaxUnknowns) ? 1 : 0;
   if (co.tree) return;
   const int bw = d * (nmin + 2) - 1;  // max |P - Q| of a nonzero
   co.B = (bw + 31) / 32 * 32;
@@ -733,6 +768,12 @@ struct TreeLaunch {
   }
 };
 
+static TreeBlock tree_block(const stt_hier* h) {
+  const LevelDesc& lv = h->lv[h->nlevels - 1];
+  const bool col = h->co.by_col;
+  return TreeBlock{h->co.per, h->d * (col ? lv.nny : lv.nnx), col ? lv.nnx : lv.nny};
+}
+
 template <int NB>
 static int tree_factor(const CoarseDesc& co, int hrows, int* status, cudaStream_t st) {
   constexpr int kThreads = 256;
@@ -751,9 +792,9 @@ static int tree_factor(const CoarseDesc& co, int hrows, int* status, cudaStream_
 
 // A solve's launch: each cluster size with as many blocks staged as fit its CTAs, and with none
 // (more CTAs an SM).  A step without its block staged takes about 1.4 times as long.
-template <int NB, int D, typename T>
+template <int NB, int D, typename T, bool SHARED>
 static int tree_launch(const CoarseDesc& co, int nrows, TreeLaunch& best) {
-  STT_TRY(allow_smem<tree_solve_kernel<NB, D, T>>());
+  STT_TRY(allow_smem<tree_solve_kernel<NB, D, T, SHARED>>());
   const size_t task = 8 * kTreeGroups * tree_task(co.B);
   for (int cl = kTreeCluster; cl >= 1; cl /= 2) {
     const int all = cl * kTreeGroups, own = tree_own(co.nb, all), steps = tree_steps(co.nb, all);
@@ -762,7 +803,7 @@ static int tree_launch(const CoarseDesc& co, int nrows, TreeLaunch& best) {
     const int most = (int)std::min<size_t>(own, (kTreeSmem - vec) / task);
     for (int st : {most, 0}) {
       int n = 0;
-      STT_TRY((resident_clusters<tree_solve_kernel<NB, D, T>>(cl, TreeRow<NB>::kThreads, vec + st * task, &n)));
+      STT_TRY((resident_clusters<tree_solve_kernel<NB, D, T, SHARED>>(cl, TreeRow<NB>::kThreads, vec + st * task, &n)));
       best.consider(nrows, n, cl, st, vec + st * task, steps * (st == own ? 5 : 7));
     }
     if (cl == kTreeCluster && most == own && best.cost == 5 * steps) break;  // one wave: nothing is faster
@@ -770,27 +811,42 @@ static int tree_launch(const CoarseDesc& co, int nrows, TreeLaunch& best) {
   return best.cluster ? STT_OK : set_error(STT_ERR_CUDA, "coarse solve: no cluster fits the device");
 }
 
-template <int NB, int D, typename T>
-static int tree_solve(const stt_hier* h, int nrows, const T* b, T* x, long long rs, const RowState* rst,
+template <int NB, int D, typename T, bool SHARED>
+static int tree_run(const stt_hier* h, int nrows, const T* b, T* x, long long rs, const RowState* rst,
                       cudaStream_t st) {
   const LevelDesc& lv = h->lv[h->nlevels - 1];
   const CoarseDesc& co = h->co;
   TreeLaunch l;
-  STT_TRY((tree_launch<NB, D, T>(co, nrows, l)));
-  launch_clusters((tree_solve_kernel<NB, D, T>), l.cluster, dim3(l.cluster, nrows), TreeRow<NB>::kThreads, l.smem, st,
+  STT_TRY((tree_launch<NB, D, T, SHARED>(co, nrows, l)));
+  launch_clusters((tree_solve_kernel<NB, D, T, SHARED>), l.cluster, dim3(l.cluster, nrows), TreeRow<NB>::kThreads, l.smem, st,
                   true, b, x, rs, co.blocks, co.nb, l.staged, co.by_col, lv.nnx, lv.nny, lv.fixed, h->row_map, h->hrows,
-                  rst);
+                  rst, tree_block(h));
   return check_launch("coarse solve");
+}
+
+template <int NB, int D, typename T>
+static int tree_solve(const stt_hier* h, int nrows, const T* b, T* x, long long rs, const RowState* rst,
+                      cudaStream_t st) {
+  if constexpr (NB == 3 || NB == 4)
+    if (h->co.per > 1) return tree_run<NB, D, T, true>(h, nrows, b, x, rs, rst, st);
+  return tree_run<NB, D, T, false>(h, nrows, b, x, rs, rst, st);
 }
 
 int coarse_factor(const stt_hier* h, cudaStream_t st) {
   const LevelDesc& lv = h->lv[h->nlevels - 1];
   const CoarseDesc& co = h->co;
   const dim3 g(co.nb, h->hrows);
-  if (h->d == 2)
-    tree_assemble_kernel<2><<<g, 256, 0, st>>>(lv.st64, lv.fixed, lv.nnx, lv.nny, co.by_col, co.B, co.blocks);
-  else
-    tree_assemble_kernel<1><<<g, 256, 0, st>>>(lv.st64, lv.fixed, lv.nnx, lv.nny, co.by_col, co.B, co.blocks);
+#define STT_ASSEMBLE(D, SHARED)                                                                                     \
+  tree_assemble_kernel<D, SHARED><<<g, 256, 0, st>>>(lv.st64, lv.fixed, lv.nnx, lv.nny, co.by_col, co.B, co.blocks, \
+                                                     tree_block(h))
+  if (h->d == 2) {
+    if (co.per > 1) STT_ASSEMBLE(2, true);
+    else STT_ASSEMBLE(2, false);
+  } else {
+    if (co.per > 1) STT_ASSEMBLE(1, true);
+    else STT_ASSEMBLE(1, false);
+  }
+#undef STT_ASSEMBLE
   STT_TRY(check_launch("coarse assemble"));
 #define STT_FACTOR(NB) return tree_factor<NB>(co, h->hrows, h->status, st)
   STT_TREE_DISPATCH(co.B, STT_FACTOR)

@@ -46,8 +46,9 @@ struct LevelDesc {
 struct CoarseDesc {
   int n;             // dofs of the coarsest level
   int tree;          // 1: odd-even elimination of the grid lines (coarse.cu); 0: banded
-  int B;             // block size: a line's dofs padded to 8 (tree), or >= the half bandwidth
-  int nb;            // blocks: the grid lines (tree), or n padded to nb * B
+  int per;           // grid lines a block (tree)
+  int B;             // block size: its lines' dofs padded to 8 (tree), or >= the half bandwidth
+  int nb;            // blocks: the grid lines by per (tree), or n padded to nb * B
   int by_col;        // dof ordering: 1 = column-major nodes (nny < nnx), 0 = row-major
   double* blocks;    // [hrows][nb][4][B][B]: X, F_l, coupling, F_r (tree), or Dinv, Dinv^T,
                      // E, E^T (E_k = L_{k,k-1})

@@ -14,7 +14,7 @@ namespace {
 struct Kernel {
   std::string name;
   size_t ceiling = 48 << 10, lowest = 1 << 30, largest = 0;  // lowest: of the ceilings that were set
-  int launches = 0, cluster = 0;  // cluster: CTAs along x, of the last launch
+  int launches = 0, cluster = 0, blocks = 0;  // the last launch's cluster and grid along x
 };
 std::map<const void*, Kernel>& kernels() {
   static auto* k = new std::map<const void*, Kernel>();
@@ -28,8 +28,9 @@ struct {
   cudaStream_t stream;
 } pushed;
 cudaError_t fail(cudaError_t e) { return last = e; }
-cudaError_t launched(const void* fn, size_t smem) {
+cudaError_t launched(const void* fn, size_t smem, dim3 grid) {
   Kernel& k = kernels()[fn];
+  k.blocks = (int)grid.x;
   ++k.launches;
   if (smem > k.largest) k.largest = smem;
   if (smem > k.ceiling) return fail(cudaErrorInvalidValue);
@@ -68,6 +69,10 @@ int fake_cluster(const char* part) {
   const Kernel* k = find(part, nullptr);
   return k ? k->cluster : 0;
 }
+int fake_blocks(const char* part) {
+  const Kernel* k = find(part, nullptr);
+  return k ? k->blocks : 0;
+}
 void fake_forget() {
   for (auto& e : kernels()) e.second.launches = 0, e.second.largest = 0;
 }
@@ -94,11 +99,13 @@ cudaError_t __cudaPopCallConfiguration(dim3* grid, dim3* block, size_t* smem, vo
   *static_cast<cudaStream_t*>(stream) = pushed.stream;
   return cudaSuccess;
 }
-cudaError_t cudaLaunchKernel(const void* fn, dim3, dim3, void**, size_t smem, cudaStream_t) { return launched(fn, smem); }
+cudaError_t cudaLaunchKernel(const void* fn, dim3 grid, dim3, void**, size_t smem, cudaStream_t) {
+  return launched(fn, smem, grid);
+}
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* fn, void**) {
   for (unsigned i = 0; i < c->numAttrs; ++i)
     if (c->attrs[i].id == cudaLaunchAttributeClusterDimension) kernels()[fn].cluster = (int)c->attrs[i].val.clusterDim.x;
-  return launched(fn, c->dynamicSmemBytes);
+  return launched(fn, c->dynamicSmemBytes, c->gridDim);
 }
 cudaError_t cudaGetLastError() {
   const cudaError_t e = last;

@@ -67,6 +67,18 @@ def fake(tmp_path_factory):
     return run
 
 
+@pytest.mark.parametrize("d,nelx,nely,blocks", [(1, 600, 1, 38), (2, 1, 600, 76), (2, 300, 2, 61), (2, 100, 7, 51),
+                                                (2, 80, 8, 81), (2, 45, 15, 46), (1, 63, 1, 64)])
+def test_short_lines_of_a_long_coarsest_grid_share_blocks(fake, d, nelx, nely, blocks):
+    """The elimination's steps follow from the number of blocks: more than 64 lines go up to 32 unknowns a
+    block."""
+    got = fake(CYCLE + r"""
+print(json.dumps(dict(blocks=lib.fake_blocks(b"tree_assemble_kernel"), rc=vcycle(),
+                      solves=lib.fake_launches(b"tree_solve_kernel"))))
+""", d=d, nelx=nelx, nely=nely, mce=700, prec=0, rows=1)
+    assert got == dict(blocks=blocks, rc=0, solves=1), got
+
+
 MMA = r"""
 n = case.get("n", 600)
 

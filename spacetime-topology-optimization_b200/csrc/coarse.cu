@@ -28,7 +28,6 @@ namespace cg = cooperative_groups;
 
 constexpr int kTreeCluster = 8;  // CTAs a row, at most
 constexpr int kTreeGroups = 2;   // thread groups of 4 B threads a CTA
-constexpr int kTreeMaxUnknowns = 5376;   // nb * B, held in every CTA's shared memory
 constexpr size_t kTreeSmem = 225 << 10;  // dynamic shared memory a CTA of the solve may take
 
 // One 8 x 8 tile product on the FP64 tensor cores (tcgen05 has no FP64 kind): lane
@@ -685,20 +684,27 @@ __global__ void __launch_bounds__(TreeRow<NB>::kThreads)
     default: M(8); break;       \
   }
 
-// Lines of up to 64 unknowns go by odd-even elimination; wider ones (a coarsest grid of
-// more than ~700 elements) and very long ones by the banded factorisation, whose blocks
-// are a multiple of 32 no smaller than the half bandwidth.  Many short lines go several to a
-// block of up to 32 unknowns (a step costs hardly more than with 8, and there are fewer): 601
-// lines of 2 unknowns one by one took 91 us a V-cycle at 1 row and 500 at 128, the banded chain
-// 82 and 116, in blocks of 16 lines 28 and 96.
-void coarse_plan(const LevelDesc& c, int d, CoarseDesc& co) {
+// Lines of up to 64 unknowns go by odd-even elimination; wider ones (a coarsest grid of more
+// than ~700 elements) by the banded factorisation, whose blocks are a multiple of 32 no
+// smaller than the half bandwidth.  Many short lines go several to a block of up to 32 unknowns (a
+// step costs hardly more than with 8, and there are fewer): 601 lines of 2 unknowns one by one took 91 us
+// a V-cycle at 1 row and 500 at 128, the banded chain 82 and 116, in blocks of 16 lines 28 and 96.
+// A long grid's vectors fill a CTA's shared memory, so a row takes all eight CTAs and 15 rows run at
+// once: 501 lines of 28 unknowns 129 us at 1 row, 614 at 33, 1970 at 128, where the chain takes 771,
+// 1110 and 1160.  Past kLongUnknowns (the rule of tree_launch needs that much room) more than
+// kLongRows rows take the chain, and all where the vectors do not fit.
+constexpr int kLongUnknowns = 5376, kLongRows = 64;
+void coarse_plan(const LevelDesc& c, int d, int hrows, CoarseDesc& co) {
   co.n = (int)c.ndof;
   co.by_col = c.nny < c.nnx ? 1 : 0;
   const int nmin = co.by_col ? c.nny : c.nnx, lines = co.by_col ? c.nnx : c.nny;
   co.per = lines > 64 ? std::max(1, 32 / (d * nmin)) : 1;  // (more than one: 22 to 32 unknowns)
   co.B = (co.per * d * nmin + 7) / 8 * 8;
   co.nb = (lines + co.per - 1) / co.per;
-  co.tree = (co.B <= 64 && (long long)co.B * co.nb <= kTreeMaxUnknowns) ? 1 : 0;
+  co.tree = co.B <= 64 && 8 * tree_vectors(co.nb, co.B, kTreeCluster * kTreeGroups) <= kTreeSmem &&
+                    (hrows <= kLongRows || (long long)co.B * co.nb <= kLongUnknowns)
+                ? 1
+                : 0;
   if (co.tree) return;
   const int bw = d * (nmin + 2) - 1;  // max |P - Q| of a nonzero
   co.B = (bw + 31) / 32 * 32;

@@ -10,7 +10,7 @@
 namespace stt {
 
 // Plans the factor for the coarsest level (co.n, co.tree, co.B, co.nb, co.by_col).
-void coarse_plan(const LevelDesc& c, int d, CoarseDesc& co);
+void coarse_plan(const LevelDesc& c, int d, int hrows, CoarseDesc& co);
 // Assembles the coarse matrix from the level's FP64 stencil and factorises it on `st`.
 int coarse_factor(const stt_hier* h, cudaStream_t st);
 // x = A^{-1} b (T = float or double; FP64 arithmetic) for nrows batch rows; only for co.tree.

@@ -210,7 +210,7 @@ long long plan_hierarchy(stt_hier_impl& h, char* base) {
         lv.st32 = (float*)carve(p, used, 4LL * h.hrows * (d == 2 ? st32_nsp<2>() : st32_nsp<1>()) * lv.nnode);
     }
   }
-  coarse_plan(h.lv[L - 1], d, h.co);
+  coarse_plan(h.lv[L - 1], d, h.hrows, h.co);
   h.co.blocks = (double*)carve(p, used, 8LL * h.hrows * h.co.nb * 4 * h.co.B * h.co.B);
   h.tables = (double*)carve(p, used, 8LL * kMaxLevels * 3 * kTableStride);
   h.gtables = (double*)carve(p, used, 8LL * (2 * kGrandStride + kChildStencilSize));
@@ -878,6 +878,240 @@ __global__ void __launch_bounds__(256) band_factor_kernel(double* __restrict__ b
   if (tid == 0 && bad) atomicOr(status, 1);
 }
 
+// 16-byte asynchronous global -> shared copies (sm_80+ cp.async), for prefetching the
+// next blocks while the current one factors.
+STT_DEV void cp_async16(void* smem, const void* gmem) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem));
+}
+STT_DEV void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
+STT_DEV void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+
+// The same factorisation for B = 16 NA (NA = 2, 4), 256 threads as a 16 x 16 grid (501 lines of 28
+// unknowns, 64 rows: 8 ms, 21 with the kernel above):
+//   * thread (ty, tx) owns the strided tile of entries (ty + 16 a, tx + 16 b), a, b < NA,
+//     of every B x B product, so each shared-memory load feeds NA multiply-adds (a warp
+//     reads 2 rows of one operand, broadcast, and 16 rows of the other at a stride of
+//     B + 1 doubles, conflict-free);
+//   * the Cholesky takes two columns per pair of barriers: every thread forms both
+//     pivots and the two scaled columns of its rows and columns in registers (column
+//     j + 1 updated by column j on the fly), then applies the rank-2 trailing update;
+//   * A_{k+1,k+1} and A_{k+1,k} are copied into staging buffers with cp.async while
+//     block k factors; the Schur update and E = A_{k+1,k} X^T read them from there.
+// Upper triangles of the work arrays carry harmless values (only lower triangles are
+// read); X = D^{-1} keeps exact zeros above its diagonal.
+template <int NA>
+__global__ void __launch_bounds__(256) band_factor_tiled_kernel(double* __restrict__ blocks, int nb,
+                                                                int* __restrict__ status) {
+  constexpr int B = 16 * NA, ld = B + 1;
+  extern __shared__ __align__(16) double sm[];
+  double* P0 = sm;           // staged A_{k,k} (B x B, dense rows)
+  double* P1 = P0 + B * B;   // staged A_{k+1,k}
+  double* A = P1 + B * B;    // current diagonal block, then its Cholesky factor (ld)
+  double* X = A + B * ld;    // D_k^{-1}
+  double* Y = X + B * ld;    // E_k
+  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+  double* bh = blocks + (size_t)blockIdx.x * nb * 4 * B * B;
+  __shared__ int bad;
+  __shared__ double rp[B];  // reciprocals of the current block's pivots
+  if (tid == 0) bad = 0;
+  auto stage = [&](double* dst, const double* src) {
+    for (int t = tid; t < B * B / 2; t += 256) cp_async16(dst + 2 * t, src + 2 * t);
+  };
+  stage(P0, bh);
+  cp_async_commit();
+  for (int k = 0; k < nb; ++k) {
+    double* Dk = bh + (size_t)k * 4 * B * B;
+    cp_async_wait_all();
+    __syncthreads();
+    // A = A_kk - E_k E_k^T (k > 0)
+    {
+      double acc[NA][NA];
+#pragma unroll
+      for (int a = 0; a < NA; ++a)
+#pragma unroll
+        for (int b = 0; b < NA; ++b) acc[a][b] = 0.0;
+      if (k > 0) {
+#pragma unroll 4
+        for (int m = 0; m < B; ++m) {
+          double yi[NA], yl[NA];
+#pragma unroll
+          for (int a = 0; a < NA; ++a) yi[a] = Y[(ty + 16 * a) * ld + m];
+#pragma unroll
+          for (int b = 0; b < NA; ++b) yl[b] = Y[(tx + 16 * b) * ld + m];
+#pragma unroll
+          for (int a = 0; a < NA; ++a)
+#pragma unroll
+            for (int b = 0; b < NA; ++b) acc[a][b] = fma(yi[a], yl[b], acc[a][b]);
+        }
+      }
+#pragma unroll
+      for (int a = 0; a < NA; ++a)
+#pragma unroll
+        for (int b = 0; b < NA; ++b) {
+          const int i = ty + 16 * a, l = tx + 16 * b;
+          A[i * ld + l] = P0[i * B + l] - acc[a][b];
+        }
+    }
+    __syncthreads();  // P0 consumed, A complete
+    if (k + 1 < nb) {
+      double* Dn = bh + (size_t)(k + 1) * 4 * B * B;
+      stage(P0, Dn);                    // A_{k+1,k+1}
+      stage(P1, Dn + (size_t)2 * B * B);  // A_{k+1,k}
+      cp_async_commit();
+    }
+    // Cholesky, a panel of four columns per step: every thread factors the 4 x 4 pivot
+    // block (one rsqrt a pivot, L_jj = t rsqrt(t), its reciprocal kept for the
+    // substitution), then the panel entries of its rows and a rank-4 update
+    for (int j = 0; j < B; j += 4) {
+      double a[4][4];
+#pragma unroll
+      for (int p = 0; p < 4; ++p)
+#pragma unroll
+        for (int q = 0; q <= p; ++q) a[p][q] = A[(j + p) * ld + j + q];
+      double l[4][4], r[4];
+      bool ok = true;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        double t = a[q][q];
+#pragma unroll
+        for (int m = 0; m < q; ++m) t = fma(-l[q][m], l[q][m], t);
+        ok = ok && t > 0.0;
+        const double tt = t > 0.0 ? t : 1.0;
+        r[q] = rsqrt(tt);
+        l[q][q] = tt * r[q];
+#pragma unroll
+        for (int p = q + 1; p < 4; ++p) {
+          double v = a[p][q];
+#pragma unroll
+          for (int m = 0; m < q; ++m) v = fma(-l[p][m], l[q][m], v);
+          l[p][q] = v * r[q];
+        }
+      }
+      // the panel columns of rows i (this thread's rows) and of rows c (its columns)
+      auto panel = [&](int i, double (&cv)[4]) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          double v = 0.0;
+          if (i > j + q) {
+            v = A[i * ld + j + q];
+#pragma unroll
+            for (int m = 0; m < q; ++m) v = fma(-cv[m], l[q][m], v);
+            v *= r[q];
+          }
+          cv[q] = v;
+        }
+      };
+      double ci[NA][4], cl[NA][4];
+#pragma unroll
+      for (int a2 = 0; a2 < NA; ++a2) panel(ty + 16 * a2, ci[a2]);
+#pragma unroll
+      for (int b = 0; b < NA; ++b) panel(tx + 16 * b, cl[b]);
+      __syncthreads();
+      if (tx == 0) {
+#pragma unroll
+        for (int a2 = 0; a2 < NA; ++a2) {
+          const int i = ty + 16 * a2;
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (i > j + q) A[i * ld + j + q] = ci[a2][q];
+        }
+      }
+      if (tid == 0) {
+        if (!ok) bad = 1;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          A[(j + q) * ld + j + q] = l[q][q];
+          rp[j + q] = r[q];
+        }
+      }
+#pragma unroll
+      for (int a2 = 0; a2 < NA; ++a2)
+#pragma unroll
+        for (int b = 0; b < NA; ++b) {
+          const int i = ty + 16 * a2, c = tx + 16 * b;
+          if (i > j + 3 && c > j + 3) {
+            double v = A[i * ld + c];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) v = fma(-ci[a2][q], cl[b][q], v);
+            A[i * ld + c] = v;
+          }
+        }
+      __syncthreads();
+    }
+    // X = A^{-1}: forward substitution with the pivots' reciprocals, a quad of threads a
+    // column, each thread's share of a dot product in two independent chains
+    {
+      const int q = tid & 3;
+      for (int c0 = 0; c0 < B; c0 += 64) {
+        const int c = c0 + tid / 4;
+        const bool col = c < B;
+        if (col && q == 0) {
+          for (int i = 0; i < c; ++i) X[i * ld + c] = 0.0;
+          X[c * ld + c] = rp[c];
+        }
+        __syncwarp();
+        for (int i = c0 + 1; i < B; ++i) {
+          double s0 = 0.0, s1 = 0.0;
+          if (col && i > c) {
+            int l2 = c + q;
+            for (; l2 + 4 < i; l2 += 8) {
+              s0 = fma(A[i * ld + l2], X[l2 * ld + c], s0);
+              s1 = fma(A[i * ld + l2 + 4], X[(l2 + 4) * ld + c], s1);
+            }
+            if (l2 < i) s0 = fma(A[i * ld + l2], X[l2 * ld + c], s0);
+          }
+          double sacc = s0 + s1;
+          sacc += __shfl_xor_sync(0xffffffffu, sacc, 1);
+          sacc += __shfl_xor_sync(0xffffffffu, sacc, 2);
+          if (col && i > c && q == 0) X[i * ld + c] = -sacc * rp[i];
+          __syncwarp();
+        }
+      }
+    }
+    __syncthreads();
+    for (int t = tid; t < B * B; t += 256) {
+      const int i = t / B, j = t % B;
+      Dk[t] = X[i * ld + j];                  // Dinv
+      Dk[(size_t)B * B + t] = X[j * ld + i];  // Dinv^T
+    }
+    if (k + 1 < nb) {
+      double* Dn = bh + (size_t)(k + 1) * 4 * B * B;
+      cp_async_wait_all();
+      __syncthreads();  // P1 (and P0) landed for every thread
+      // E = A_{k+1,k} X^T (X is zero above its diagonal)
+      double acc[NA][NA];
+#pragma unroll
+      for (int a = 0; a < NA; ++a)
+#pragma unroll
+        for (int b = 0; b < NA; ++b) acc[a][b] = 0.0;
+#pragma unroll 4
+      for (int l = 0; l < B; ++l) {
+        double ai[NA], xj[NA];
+#pragma unroll
+        for (int a = 0; a < NA; ++a) ai[a] = P1[(ty + 16 * a) * B + l];
+#pragma unroll
+        for (int b = 0; b < NA; ++b) xj[b] = X[(tx + 16 * b) * ld + l];
+#pragma unroll
+        for (int a = 0; a < NA; ++a)
+#pragma unroll
+          for (int b = 0; b < NA; ++b) acc[a][b] = fma(ai[a], xj[b], acc[a][b]);
+      }
+#pragma unroll
+      for (int a = 0; a < NA; ++a)
+#pragma unroll
+        for (int b = 0; b < NA; ++b) {
+          const int i = ty + 16 * a, j = tx + 16 * b;
+          Y[i * ld + j] = acc[a][b];
+          Dn[(size_t)2 * B * B + i * B + j] = acc[a][b];  // E
+        }
+      __syncthreads();
+      for (int t = tid; t < B * B; t += 256) Dn[(size_t)3 * B * B + t] = Y[(t % B) * ld + t / B];  // E^T
+    }
+  }
+  if (tid == 0 && bad) atomicOr(status, 1);
+}
+
 }  // namespace stt
 
 using namespace stt;
@@ -1142,8 +1376,17 @@ static int build_coarse(stt_hier* h, cudaStream_t st) {
       cl.st64, cl.fixed, cl.nnx, cl.nny, co.by_col, co.B, co.nb, co.blocks, h->status);
   STT_TRY(check_launch("band assemble"));
   const size_t smem = (size_t)3 * co.B * (co.B + 1) * sizeof(double);
-  STT_TRY(allow_smem<band_factor_kernel>());
-  band_factor_kernel<<<H, 256, smem, st>>>(co.blocks, co.B, co.nb, h->status);
+  const size_t tiled = smem + (size_t)2 * co.B * co.B * sizeof(double);  // and two staging blocks
+  if (co.B == 32) {
+    STT_TRY(allow_smem<band_factor_tiled_kernel<2>>());
+    band_factor_tiled_kernel<2><<<H, 256, tiled, st>>>(co.blocks, co.nb, h->status);
+  } else if (co.B == 64) {
+    STT_TRY(allow_smem<band_factor_tiled_kernel<4>>());
+    band_factor_tiled_kernel<4><<<H, 256, tiled, st>>>(co.blocks, co.nb, h->status);
+  } else {
+    STT_TRY(allow_smem<band_factor_kernel>());
+    band_factor_kernel<<<H, 256, smem, st>>>(co.blocks, co.B, co.nb, h->status);
+  }
   return check_launch("band factor");
 }
 

@@ -3,8 +3,8 @@
 Coarsest grids of more than 64 lines take up to 32 unknowns a block, so a block may hold whole lines
 and the last one fewer; the grids here put the lines on either side of that number and of a
 whole number of blocks, with one line a block where two do not fit, in both line directions, and go on
-to grids whose vectors no longer fit a row's shared memory (the banded factorisation).  A one-level
-hierarchy's V-cycle is the solve alone: ``z = A^{-1} r``, against scipy's sparse factorisation.
+to grids whose vectors fill a row's shared memory or no longer fit it (the banded factorisation with blocks
+of 32 and of 64, which more than 64 rows of the former take too).  A one-level hierarchy's V-cycle is the solve alone: ``z = A^{-1} r``, against scipy's sparse factorisation.
 
 Tolerance: with dofs held every four nodes the matrices' condition numbers stay under 1e3 (measured on
 the CPU), so two backward-stable FP64 solves agree to 1e-12 or so; FP32 rounding of the right-hand
@@ -23,7 +23,8 @@ from oracle import sttopt_oracle as O
 pytestmark = pytest.mark.gpu
 
 GRIDS = [(62, 1, 2), (63, 1, 2), (64, 1, 2), (65, 2, 1), (70, 7, 2), (71, 8, 2), (95, 1, 1), (3, 150, 2), (300, 2, 2),
-         (600, 1, 1), (700, 1, 2), (1200, 3, 1), (500, 13, 2), (250, 30, 2), (2047, 3, 2), (3000, 3, 2)]
+         (600, 1, 1), (700, 1, 2), (1200, 3, 1), (500, 13, 2), (250, 30, 2), (2047, 3, 2), (3000, 3, 2), (700, 20, 2)]
+CASES = [(*g, 3) for g in GRIDS] + [(400, 13, 2, 64), (400, 13, 2, 65), (200, 27, 2, 65)]
 
 
 def _problem(nelx, nely, d, rows):
@@ -47,11 +48,11 @@ def _matrix(rho, mask, nelx, nely, d):
 
 
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
-@pytest.mark.parametrize("nelx,nely,d", GRIDS)
-def test_short_lines_share_a_block(pkg, nelx, nely, d, precision):
+@pytest.mark.parametrize("nelx,nely,d,rows", CASES)
+def test_short_lines_and_long_grids(pkg, nelx, nely, d, rows, precision):
     from sttopt_b200 import torch_mg
 
-    rows, dev = 3, torch.device("cuda")
+    dev = torch.device("cuda")
     rho, mask, r = _problem(nelx, nely, d, rows)
     KE = O.plane_stress_KE(0.3) if d == 2 else O.diffusion_KE()
     levels = torch_mg.build_hierarchy(torch.tensor(rho, device=dev),
@@ -61,7 +62,7 @@ def test_short_lines_share_a_block(pkg, nelx, nely, d, precision):
     assert len(levels) == 1
     z = torch_mg.VCycle(levels)(torch.tensor(r, device=dev)).cpu().numpy()
     tol = 1e-11 if precision == "fp64" else 1e-5
-    for s in range(rows):
+    for s in sorted({0, 1, rows // 2, rows - 1}):
         K, free = _matrix(rho[s], mask, nelx, nely, d)
         want = np.zeros(mask.size)
         want[free] = spl.spsolve(K, r[s][free])

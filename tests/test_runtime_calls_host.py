@@ -79,6 +79,17 @@ print(json.dumps(dict(blocks=lib.fake_blocks(b"tree_assemble_kernel"), rc=vcycle
     assert got == dict(blocks=blocks, rc=0, solves=1), got
 
 
+@pytest.mark.parametrize("nelx,nely,rows,kernel", [
+    (32, 16, 128, "tree_factor_kernel"), (500, 13, 64, "tree_factor_kernel"),
+    (500, 13, 65, "band_factor_tiled_kernelILi2E"), (3000, 3, 1, "band_factor_tiled_kernelILi2E"),
+    (700, 20, 1, "band_factor_tiled_kernelILi4E"), (40, 38, 1, "band_factor_kernel")])
+def test_long_and_wide_coarsest_grids_take_their_factorisation(fake, nelx, nely, rows, kernel):
+    got = fake(CYCLE + r"""
+print(json.dumps([lib.fake_launches(case["kernel"].encode()), vcycle()]))
+""", d=2, nelx=nelx, nely=nely, mce=nelx * nely, prec=0, rows=rows, kernel=kernel)
+    assert got == [1, 0], got
+
+
 MMA = r"""
 n = case.get("n", 600)
 

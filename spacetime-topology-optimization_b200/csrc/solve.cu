@@ -287,10 +287,11 @@ struct Cycle {
       if (rc == STT_OK) rc = solved;
       return;
     }
-#define STT_COARSE(NC)                                                                          \
-  launch((coarse_solve_kernel<D, T, NC>), nrows, 16 * NC, 0, st, b, x, vstride(lv.ndof), co.blocks, co.nb, co.by_col, \
-                                                          lv.nnx, lv.nny, lv.fixed, w.cscratch,       \
-                                                          h->row_map, h->hrows, rst)
+    // (not launched early: its blocks would share the SMs that the kernel before leaves idle, one
+    // long chain beside another; 451 blocks of 32 at 128 rows 1310 us a V-cycle so, 1150 this way)
+#define STT_COARSE(NC)                                                                                                 \
+  coarse_solve_kernel<D, T, NC><<<nrows, 16 * NC, 0, st>>>(b, x, vstride(lv.ndof), co.blocks, co.nb, co.by_col, lv.nnx, \
+                                                           lv.nny, lv.fixed, w.cscratch, h->row_map, h->hrows, rst)
     switch (co.B) {
       case 32: STT_COARSE(8); break;
       case 64: STT_COARSE(16); break;

@@ -14,7 +14,7 @@ namespace {
 struct Kernel {
   std::string name;
   size_t ceiling = 48 << 10, lowest = 1 << 30, largest = 0;  // lowest: of the ceilings that were set
-  int launches = 0, cluster = 0, blocks = 0;  // the last launch's cluster and grid along x
+  int launches = 0, cluster = 0, blocks = 0, early = 0;  // the last launch: cluster and grid along x, dependent
 };
 std::map<const void*, Kernel>& kernels() {
   static auto* k = new std::map<const void*, Kernel>();
@@ -69,6 +69,10 @@ int fake_cluster(const char* part) {
   const Kernel* k = find(part, nullptr);
   return k ? k->cluster : 0;
 }
+int fake_early(const char* part) {
+  const Kernel* k = find(part, nullptr);
+  return k ? k->early : -1;
+}
 int fake_blocks(const char* part) {
   const Kernel* k = find(part, nullptr);
   return k ? k->blocks : 0;
@@ -103,8 +107,11 @@ cudaError_t cudaLaunchKernel(const void* fn, dim3 grid, dim3, void**, size_t sme
   return launched(fn, smem, grid);
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* fn, void**) {
-  for (unsigned i = 0; i < c->numAttrs; ++i)
-    if (c->attrs[i].id == cudaLaunchAttributeClusterDimension) kernels()[fn].cluster = (int)c->attrs[i].val.clusterDim.x;
+  Kernel& k = kernels()[fn];
+  for (unsigned i = 0; i < c->numAttrs; ++i) {
+    if (c->attrs[i].id == cudaLaunchAttributeClusterDimension) k.cluster = (int)c->attrs[i].val.clusterDim.x;
+    if (c->attrs[i].id == cudaLaunchAttributeProgrammaticStreamSerialization) k.early = 1;
+  }
   return launched(fn, c->dynamicSmemBytes, c->gridDim);
 }
 cudaError_t cudaGetLastError() {

@@ -90,6 +90,14 @@ print(json.dumps([lib.fake_launches(case["kernel"].encode()), vcycle()]))
     assert got == [1, 0], got
 
 
+@pytest.mark.parametrize("mce,kernel,early", [(1520, "coarse_solve_kernel", 0), (700, "tree_solve_kernel", 1)])
+def test_the_chain_of_a_banded_coarse_solve_is_not_launched_early(fake, mce, kernel, early):
+    got = fake(CYCLE + r"""
+print(json.dumps([vcycle(), lib.fake_early(case["kernel"].encode()), lib.fake_early(b"restrict")]))
+""", d=2, nelx=80, nely=76, mce=mce, prec=0, rows=2, kernel=kernel)
+    assert got == [0, early, 1], got
+
+
 MMA = r"""
 n = case.get("n", 600)
 

@@ -6,7 +6,7 @@
 // heaviside_projection_derivative (:109-133).  H is a stencil with zero padding outside
 // the grid, so it is applied as one here: a block stages its output tile plus the stencil's
 // halo in shared memory (coalesced rows), and a thread slides down its column, holding the
-// sums of VY rows, so that an input value is read once for the up to VY rows it enters.
+// sums of one or two rows, so that an input value is read once for the rows it enters.
 // Hs is the sum of the in-grid weights: a constant away from the border (summed on the
 // host), formed from the element's position near it (no matrix, no row-sum array).  H is
 // symmetric, so the adjoint, H (g * P'(xTilde) / Hs), is the same stencil applied to the
@@ -20,8 +20,7 @@
 namespace stt {
 
 constexpr int kFiltMaxR = 7;  // ceil(rmin) - 1 <= 7 (rmin <= 8)
-constexpr int kFiltTX = 32, kFiltTY = 16;  // threads a block
-constexpr int kFiltVY = 2;                 // rows a thread: a tile is 32 x 32 elements
+constexpr int kFiltTX = 32;  // threads along x: a tile's width
 
 struct FiltW {
   double w[(2 * kFiltMaxR + 1) * (2 * kFiltMaxR + 1)];  // w[(dj + R) * (2R + 1) + (di + R)]
@@ -43,7 +42,7 @@ STT_DEV double filt_hs(const FiltW& W, int i, int j, int nelx, int nely) {
 #pragma unroll 1
   for (int dj = -R; dj <= R; ++dj) {
     if (j + dj < 0 || j + dj >= nely) continue;
-#pragma unroll 1
+#pragma unroll
     for (int di = -R; di <= R; ++di)
       if (i + di >= 0 && i + di < nelx) s += W.w[(dj + R) * n + (di + R)];
   }
@@ -62,25 +61,26 @@ STT_DEV double heaviside_d(double x, const FiltP& P) {
 
 // ADJ = 0: xt = H x / Hs (and xp = P(xt) when beta > 0);
 // ADJ = 1: out = H (g * s / Hs), s = P'(xt) when beta > 0 (xt given), else 1.
-// Bound by instruction issue (0.55-0.6 of the cycles: (2R + 1)^2 FP64 multiply-adds, a tanh
-// and two divisions an element) and by the staging loads' latency, so a thread takes only
-// two rows: more rows mean fewer shared-memory loads but fewer warps (8 rows a thread, 5
-// blocks of 256 an SM: 45 and 55 us; 4 rows 36 and 45; 1 row 40 and 51).  With the weights
-// read from the constant bank, Hs summed for every element and three tanh each (in the
-// adjoint for every staged element, twice over with an 8-row tile's halo), 2048 x 1024 at
-// rmin 4 took 95 us forward with the projection and 171 us the adjoint; now 34 and 41.
-template <int ADJ, int R>
-__global__ void __launch_bounds__(kFiltTX * kFiltTY) cone_filter_kernel(
+// Bound by instruction issue ((2R + 1)^2 FP64 multiply-adds, a tanh and two divisions an element)
+// and by the latency of the staging loads and of Hs near the border, a chain of up to (2R + 1)^2
+// sums, with a row of it unrolled.  A thread takes two rows of a 32 x 32 tile: more rows mean
+// fewer shared-memory loads but fewer warps (at rmin 4 and 2048 x 1024, before the unrolling: 8 rows a
+// thread 45 us forward with the projection and 55 the adjoint, 4 rows 36 and 45, 2 rows 32 and 40, 1
+// row 40 and 51; now 29 and 36).  Launches of fewer such tiles than SMs take 32 x 8 tiles and one row:
+// 180 x 60 at rmin 4 3.8 and 5.9 us, 5.8 and 6.9 with the other, at rmin 8 8 and 16 against 14 and 20;
+// at 540 x 270 (153 tiles) 5.4 and 7.8 against 6.4 and 7.4.
+template <int ADJ, int R, int VY, int TY>
+__global__ void __launch_bounds__(kFiltTX * TY) cone_filter_kernel(
     const double* __restrict__ in, long long in_rs, const double* __restrict__ xt_in, long long xt_rs,
     double* __restrict__ out, double* __restrict__ xp, long long o_rs, int nelx, int nely, FiltW W, FiltP P) {
-  constexpr int VY = kFiltVY, n = 2 * R + 1, tw = kFiltTX + 2 * R, th = kFiltTY * VY + 2 * R;
+  constexpr int n = 2 * R + 1, tw = kFiltTX + 2 * R, th = TY * VY + 2 * R;
   __shared__ double tile[th * tw];
   const int s = blockIdx.z;
-  const int i0 = blockIdx.x * kFiltTX, j0 = blockIdx.y * (kFiltTY * VY);
+  const int i0 = blockIdx.x * kFiltTX, j0 = blockIdx.y * (TY * VY);
   const double* xs = in + (size_t)s * in_rs;
   const double* ts = ADJ ? xt_in + (size_t)s * xt_rs : nullptr;
   const bool proj = P.beta > 0.0;
-  for (int t = threadIdx.y * kFiltTX + threadIdx.x; t < tw * th; t += kFiltTX * kFiltTY) {
+  for (int t = threadIdx.y * kFiltTX + threadIdx.x; t < tw * th; t += kFiltTX * TY) {
     const int tj = t / tw, ti = t - tj * tw;
     const int i = i0 - R + ti, j = j0 - R + tj;
     double v = 0.0;
@@ -102,19 +102,10 @@ __global__ void __launch_bounds__(kFiltTX * kFiltTY) cone_filter_kernel(
   double acc[VY];
 #pragma unroll
   for (int y = 0; y < VY; ++y) acc[y] = 0.0;
-  // the distinct weights (they depend on |di|, |dj|, in either order) held in registers: a
-  // multiply-add takes no constant-bank operand in FP64, so each would reload its weight
-  double w[R + 1][R + 1];
-#pragma unroll
-  for (int a = 0; a <= R; ++a)
-#pragma unroll
-    for (int b = 0; b <= a; ++b) {
-      w[a][b] = W.w[(a + R) * n + (b + R)];
-      asm volatile("" : "+d"(w[a][b]));
-    }
+  // (a weight depends on |di| and |dj|, in either order: (R + 1)(R + 2) / 2 distinct ones)
   auto weight = [&](int dj, int di) {
     const int a = dj < 0 ? -dj : dj, b = di < 0 ? -di : di;
-    return a >= b ? w[a][b] : w[b][a];
+    return W.w[((a >= b ? a : b) + R) * n + (a >= b ? b : a) + R];
   };
 #pragma unroll
   for (int r = 0; r < VY + 2 * R; ++r) {
@@ -169,21 +160,41 @@ static int launch_filter(int nelx, int nely, int nrows, double rmin, const doubl
     P.t0 = std::tanh(beta * eta);
     P.den = P.t0 + std::tanh(beta * (1.0 - eta));
   }
-  const unsigned th = kFiltTY * kFiltVY;
-  const dim3 grid((nelx + kFiltTX - 1) / kFiltTX, (nely + th - 1) / th, nrows), block(kFiltTX, kFiltTY);
-#define STT_FILT(RR)                                                                                        \
-  cone_filter_kernel<ADJ, RR><<<grid, block, 0, st>>>(in, in_rs, xt, xt_rs, out, xp, o_rs, nelx, nely, W, P)
+  const int gx = (nelx + kFiltTX - 1) / kFiltTX;
+  // 32 x 32 tiles, two rows a thread; 32 x 8 and one row where there are fewer of those than SMs
+  const bool small = (long long)gx * ((nely + 31) / 32) * nrows < 148;
+#define STT_FILT_TILE(RR, VY, TY)                                                                       \
+  cone_filter_kernel<ADJ, RR, VY, TY><<<dim3(gx, (nely + VY * TY - 1) / (VY * TY), nrows), dim3(kFiltTX, TY), 0, st>>>( \
+      in, in_rs, xt, xt_rs, out, xp, o_rs, nelx, nely, W, P)
+#define STT_FILT(RR)                  \
+  if (small) STT_FILT_TILE(RR, 1, 8); \
+  else STT_FILT_TILE(RR, 2, 16)
   switch (R) {
-    case 0: STT_FILT(0); break;
-    case 1: STT_FILT(1); break;
-    case 2: STT_FILT(2); break;
-    case 3: STT_FILT(3); break;
-    case 4: STT_FILT(4); break;
-    case 5: STT_FILT(5); break;
-    case 6: STT_FILT(6); break;
+    case 0:
+      STT_FILT(0);
+      break;
+    case 1:
+      STT_FILT(1);
+      break;
+    case 2:
+      STT_FILT(2);
+      break;
+    case 3:
+      STT_FILT(3);
+      break;
+    case 4:
+      STT_FILT(4);
+      break;
+    case 5:
+      STT_FILT(5);
+      break;
+    case 6:
+      STT_FILT(6);
+      break;
     default: STT_FILT(7);
   }
 #undef STT_FILT
+#undef STT_FILT_TILE
   return check_launch("cone filter");
 }
 

@@ -126,6 +126,22 @@ print(json.dumps(dict(rcs=rcs, launches=lib.fake_launches(b"mma_assemble_kernel"
     assert got["lowest"] >= got["largest"], got
 
 
+@pytest.mark.parametrize("nelx,nely,rows,small", [(180, 60, 1, 1), (180, 60, 12, 1), (180, 60, 13, 0), (256, 128, 4, 1),
+                                                  (540, 270, 1, 0), (2048, 1024, 1, 0)])
+def test_small_filter_launches_take_small_tiles(fake, nelx, nely, rows, small):
+    """Fewer 32 x 32 tiles than SMs: tiles of 32 x 8, one row a thread."""
+    got = fake(r"""
+nx, ny, rows = case["nelx"], case["nely"], case["rows"]
+x, a, b = (mem(rows * nx * ny) for _ in range(3))
+rcs = [lib.stt_cone_filter(I(nx), I(ny), I(rows), D(4.0), x, L(nx * ny), a, b, L(nx * ny), D(8.0), D(0.5), None),
+       lib.stt_cone_filter_adjoint(I(nx), I(ny), I(rows), D(4.0), x, L(nx * ny), a, L(nx * ny), D(8.0), D(0.5), b,
+                                   L(nx * ny), None)]
+print(json.dumps(rcs + [lib.fake_launches(b"cone_filter_kernelILi%dELi3ELi%dELi%dE" % (adj, *tile))
+                        for adj in (0, 1) for tile in ((1, 8), (2, 16))]))
+""", nelx=nelx, nely=nely, rows=rows)
+    assert got == [0, 0] + 2 * [small, 1 - small], got
+
+
 CYCLE = r"""
 from oracle import sttopt_oracle as O
 

@@ -51,7 +51,8 @@ __global__ void __launch_bounds__(kQThreads) q4_apply_kernel(
 
 // The same operator with KE in modal form; FL selects the options at compile time:
 // bit 0 projects the input, bit 1 the output, bit 2 adds the reaction term.
-template <int D, typename T, int FL>
+// SPLIT: march_modal's.
+template <int D, typename T, int FL, bool SPLIT>
 __global__ void __launch_bounds__(kQThreads) q4_apply_modal_kernel(
     const T* __restrict__ u, long long u_rs, T* __restrict__ out, long long out_rs,
     const T* __restrict__ rho, long long rho_rs, const T* __restrict__ rdiag, long long rdiag_rs,
@@ -63,7 +64,7 @@ __global__ void __launch_bounds__(kQThreads) q4_apply_modal_kernel(
   const T* rr = rho + (size_t)row * rho_rs;
   const T* rdr = RD ? rdiag + (size_t)row * rdiag_rs : nullptr;
   T* outr = out + (size_t)row * out_rs;
-  march_modal<D, T, true, false, PIN>(
+  march_modal<D, T, true, false, PIN, NoExtra, T[D], 2, kQRows, SPLIT>(
       mq, nnx, nny,
       [&](int r, int c) -> uint8_t { return (PIN || POUT) ? __ldg(fixed + r * nnx + c) : (uint8_t)0; },
       [&](int r, int c, uint8_t, T(&v)[D]) { load_node<D, T>(ur, r * nnx + c, v); },
@@ -213,10 +214,18 @@ int launch_apply(int nelx, int nely, int nrows, const void* u, long long u_rs, v
   if (modal_from_ke(D, KE, m)) {
     const MQ<T> mq = mq_cast<T>(m);
     const int fl = pin | (pout << 1) | (rdiag ? 4 : 0);
-#define STT_MODAL_APPLY(FL)                                                                          \
-  q4_apply_modal_kernel<D, T, FL><<<grid, kQThreads, 0, st>>>((const T*)u, u_rs, (T*)out, out_rs,    \
-                                                              (const T*)rho, rho_rs, (const T*)rdiag, \
-                                                              rdiag_rs, fixed, nelx, nely, mq)
+    // one dof a node: the loop without range tests pays from about 1.5M nodes in FP64 and 4M in FP32
+    // (with and without it: 24x24 6.5 and 6.0 us, 7.6 and 7.2; 540x270 x 16 rows 12.7 and 13.2, 12.6
+    // and 12.2; 1024x512 x 16 44.3 and 45.4, 33.9 and 34.6; 2047x1023 x 16 156 and 162, 106 and 113)
+    const long long nodes = (long long)(nelx + 1) * (nely + 1) * nrows;
+    const bool split = D == 2 || nodes >= (sizeof(T) == 8 ? 3LL << 19 : 4LL << 20);
+#define STT_MODAL_APPLY2(FL, SPLIT)                                                                             \
+  q4_apply_modal_kernel<D, T, FL, SPLIT><<<grid, kQThreads, 0, st>>>((const T*)u, u_rs, (T*)out, out_rs,        \
+                                                                     (const T*)rho, rho_rs, (const T*)rdiag,    \
+                                                                     rdiag_rs, fixed, nelx, nely, mq)
+#define STT_MODAL_APPLY(FL)                        \
+  if (split) STT_MODAL_APPLY2(FL, true);           \
+  else if constexpr (D == 1) STT_MODAL_APPLY2(FL, false)
     switch (fl) {
       case 0: STT_MODAL_APPLY(0); break;
       case 1: STT_MODAL_APPLY(1); break;
@@ -228,6 +237,7 @@ int launch_apply(int nelx, int nely, int nrows, const void* u, long long u_rs, v
       default: STT_MODAL_APPLY(7); break;
     }
 #undef STT_MODAL_APPLY
+#undef STT_MODAL_APPLY2
   } else {
     q4_apply_kernel<D, T><<<grid, kQThreads, 0, st>>>(
         (const T*)u, u_rs, (T*)out, out_rs, (const T*)rho, rho_rs, (const T*)rdiag, rdiag_rs,

@@ -296,8 +296,8 @@ constexpr uint8_t kInGrid = 0x80;  // march_modal's flag bit: the row was in the
 // that beat deeper lookahead (4 rows: -20 %, 8 rows: -50 % for the FP32 apply at
 // 2048x1024 x 16 rows) and two grid columns per lane (-12 %), all measured.
 template <int D, typename T, bool KU, bool DG, bool PIN, typename Extra = NoExtra, typename In = T[D],
-          int AHEAD = 2, int BAND = kQRows, typename LoadF, typename LoadU, typename LoadR, typename LoadX,
-          typename Emit, typename Value = CopyIn>
+          int AHEAD = 2, int BAND = kQRows, bool SPLIT = (D == 2), typename LoadF, typename LoadU, typename LoadR,
+          typename LoadX, typename Emit, typename Value = CopyIn>
 STT_DEV void march_modal(const MQ<T>& q, int nnx, int nny, LoadF loadf, LoadU loadu, LoadR loadr, LoadX loadx,
                          Emit emit, Value value = Value{}) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -404,7 +404,8 @@ STT_DEV void march_modal(const MQ<T>& q, int nnx, int nny, LoadF loadf, LoadU lo
   // operator at 2048x1024 x 16 rows: FP32 149 -> 136 us (103 at the copy rate), FP64 286 -> 234;
   // one dof a node, 8 rows, FP32 63 -> 58.  Extra keeps its test: without it nothing gained.
   // (The chained smoothing passes lose by the same split, and their FP64 forms spill: V-cycle
-  // there 1710 -> 1773 us.)
+  // there 1710 -> 1773 us.)  SPLIT: whether there is such a loop; with one dof a node it costs
+  // every launch about 0.6 us, so only the large applies take it.
   auto rows = [&](auto inner) {
     constexpr bool INNER = decltype(inner)::value;
     const int cn = min(max(c, 0), nnx - 1), ce = min(max(c, 0), nelx - 1);
@@ -480,10 +481,13 @@ STT_DEV void march_modal(const MQ<T>& q, int nnx, int nny, LoadF loadf, LoadU lo
       }
     }
   };
-  if (r0 > 0 && r1 - r0 == band && band % AHEAD == 0 && r1 + 2 * AHEAD + 1 < nely)
-    rows(std::true_type{});
-  else
-    rows(std::false_type{});
+  if constexpr (SPLIT) {
+    if (r0 > 0 && r1 - r0 == band && band % AHEAD == 0 && r1 + 2 * AHEAD + 1 < nely) {
+      rows(std::true_type{});
+      return;
+    }
+  }
+  rows(std::false_type{});
 }
 
 // Launch grid of the marching kernels (generic and modal share it).

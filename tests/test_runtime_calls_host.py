@@ -142,6 +142,21 @@ print(json.dumps(rcs + [lib.fake_launches(b"cone_filter_kernelILi%dELi3ELi%dELi%
     assert got == [0, 0] + 2 * [small, 1 - small], got
 
 
+@pytest.mark.parametrize("d,nelx,nely,rows,split", [(1, 24, 24, 1, 0), (1, 1023, 1023, 1, 0), (1, 1023, 1023, 2, 1),
+                                                    (2, 24, 24, 1, 1)])
+def test_small_one_dof_applies_take_one_loop(fake, d, nelx, nely, rows, split):
+    got = fake(r"""
+from oracle import sttopt_oracle as O
+
+d, nx, ny, rows = (case[k] for k in ("d", "nelx", "nely", "rows"))
+n = d * (nx + 1) * (ny + 1)
+rc = lib.stt_q4_apply(I(0), I(d), I(nx), I(ny), I(rows), mem(8), L(n), mem(8), L(n), mem(8), L(nx * ny), None, L(0), None,
+                      I(0), arr(O.plane_stress_KE(0.3) if d == 2 else O.diffusion_KE()), None)
+print(json.dumps([rc] + [lib.fake_launches(b"q4_apply_modal_kernelILi%dEdLi0ELb%dE" % (d, k)) for k in (0, 1)]))
+""", d=d, nelx=nelx, nely=nely, rows=rows)
+    assert got == [0, 1 - split, split], got
+
+
 CYCLE = r"""
 from oracle import sttopt_oracle as O
 

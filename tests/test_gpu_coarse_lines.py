@@ -1,10 +1,12 @@
-"""Several short grid lines a block, and long coarsest grids, in the coarse solve.
+"""Several short grid lines a block, wide lines, and long coarsest grids, in the coarse solve.
 
 Coarsest grids of more than 64 lines take up to 32 unknowns a block, so a block may hold whole lines
 and the last one fewer; the grids here put the lines on either side of that number and of a
-whole number of blocks, with one line a block where two do not fit, in both line directions, and go on
-to grids whose vectors fill a row's shared memory or no longer fit it (the banded factorisation with blocks
-of 32 and of 64, which more than 64 rows of the former take too).  A one-level hierarchy's V-cycle is the solve alone: ``z = A^{-1} r``, against scipy's sparse factorisation.
+whole number of blocks, with one line a block where two do not fit, in both line directions, take
+lines of 58 to 64 unknowns (64 a block, of which none is staged in shared memory), and go on to grids
+whose vectors fill a row's shared memory or no longer fit it (the banded factorisation with blocks of
+32 and of 64, which more than 64 rows of the former take too).  A one-level hierarchy's V-cycle is the
+solve alone: ``z = A^{-1} r``, against scipy's sparse factorisation.
 
 Tolerance: with dofs held every four nodes the matrices' condition numbers stay under 1e3 (measured on
 the CPU), so two backward-stable FP64 solves agree to 1e-12 or so; FP32 rounding of the right-hand
@@ -22,8 +24,9 @@ from oracle import sttopt_oracle as O
 
 pytestmark = pytest.mark.gpu
 
-GRIDS = [(62, 1, 2), (63, 1, 2), (64, 1, 2), (65, 2, 1), (70, 7, 2), (71, 8, 2), (95, 1, 1), (3, 150, 2), (300, 2, 2),
-         (600, 1, 1), (700, 1, 2), (1200, 3, 1), (500, 13, 2), (250, 30, 2), (2047, 3, 2), (3000, 3, 2), (700, 20, 2)]
+GRIDS = [(28, 28, 2), (31, 31, 2), (40, 30, 2), (30, 44, 2), (80, 31, 2), (62, 1, 2), (63, 1, 2), (64, 1, 2),
+         (65, 2, 1), (70, 7, 2), (71, 8, 2), (95, 1, 1), (3, 150, 2), (300, 2, 2), (600, 1, 1), (700, 1, 2),
+         (1200, 3, 1), (500, 13, 2), (250, 30, 2), (2047, 3, 2), (3000, 3, 2), (700, 20, 2)]
 CASES = [(*g, 3) for g in GRIDS] + [(400, 13, 2, 64), (400, 13, 2, 65), (200, 27, 2, 65)]
 
 

@@ -294,9 +294,11 @@ constexpr uint8_t kInGrid = 0x80;  // march_modal's flag bit: the row was in the
 // around a load in this loop cost the FP32 apply 2x on B200 (measured).  AHEAD rows of
 // loads stay in flight; at ~46 registers a thread the SM holds 11 blocks, and on B200
 // that beat deeper lookahead (4 rows: -20 %, 8 rows: -50 % for the FP32 apply at
-// 2048x1024 x 16 rows) and two grid columns per lane (-12 %), all measured.
+// 2048x1024 x 16 rows) and two grid columns per lane (-12 %), all measured.  (That was with plain
+// operations and loads.  The chained smoothing passes gained from two columns once the operations were
+// paired and the rows came through a ring of asynchronous copies; this march has not been tried so.)
 template <int D, typename T, bool KU, bool DG, bool PIN, typename Extra = NoExtra, typename In = T[D],
-          int AHEAD = 2, int BAND = kQRows, bool SPLIT = (D == 2), typename LoadF, typename LoadU, typename LoadR,
+          int AHEAD = 2, int BAND = kQRows, bool SPLIT = true, typename LoadF, typename LoadU, typename LoadR,
           typename LoadX, typename Emit, typename Value = CopyIn>
 STT_DEV void march_modal(const MQ<T>& q, int nnx, int nny, LoadF loadf, LoadU loadu, LoadR loadr, LoadX loadx,
                          Emit emit, Value value = Value{}) {
@@ -405,7 +407,8 @@ STT_DEV void march_modal(const MQ<T>& q, int nnx, int nny, LoadF loadf, LoadU lo
   // one dof a node, 8 rows, FP32 63 -> 58.  Extra keeps its test: without it nothing gained.
   // (The chained smoothing passes lose by the same split, and their FP64 forms spill: V-cycle
   // there 1710 -> 1773 us.)  SPLIT: whether there is such a loop; with one dof a node it costs
-  // every launch about 0.6 us, so only the large applies take it.
+  // a launch about 0.6 us, so small applies go without.  (The heat solve's p.Ap pass at 2048x1024
+  // takes 45 us with it and 57 without, from memory.)
   auto rows = [&](auto inner) {
     constexpr bool INNER = decltype(inner)::value;
     const int cn = min(max(c, 0), nnx - 1), ce = min(max(c, 0), nelx - 1);

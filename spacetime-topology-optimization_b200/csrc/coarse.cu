@@ -12,6 +12,10 @@
 // A chain over the lines (block k needs block k - 1) has nb dependent steps each way; this
 // order has log2(nb), and the steps of one stride run side by side on a cluster of up to eight
 // CTAs a row (fewer where there are many rows), which exchange through distributed shared memory.
+//
+// The order of the sums below was chosen among equally accurate ones: the parity tests of the
+// product element form hold FP64 results to 1e-9 of dc and 5e-8 of the floating stage's c, which is
+// what a change of omega by 1e-13 moves them by, so a change of rounding here can trip them.
 #include "coarse.h"
 
 #include <cooperative_groups.h>
@@ -275,7 +279,7 @@ STT_DEV void tree_tiles(const double (&acc)[NB][2], Put put) {
 // One row's factorisation on a cluster.  Latency-bound: a block's elimination is a chain of
 // B pivots (about B/8 tile steps of one warp) and three B^3 products on the FP64 tensor
 // cores; a stride's blocks are spread over the row's CTAs.  132 us for 33 lines of 40
-// unknowns at 1 to 15 rows, 96 us for 46 lines of 32, where the banded factorisation (a chain
+// unknowns at 1 to 15 rows, 190 at 16 to 33, 706 at 128, 95 us for 46 lines of 32, where the banded factorisation (a chain
 // over all unknowns on one CTA a row) took 871 and 1118 us.  Slots of block i: 0 the matrix
 // block, then X_i; 1 F_l; 2 the coupling to the left neighbour still present; 3 F_r.
 template <int NB>
@@ -394,15 +398,17 @@ __host__ __device__ inline size_t tree_task(int B) { return 3 * (size_t)B * B; }
 // fetched once, at the start, into the shared memory of the CTA that will use them (the
 // first `staged` blocks of a group; later ones are read from L2 when their turn comes):
 // loads issued before a cluster barrier are waited for by it, and cost a memory latency a
-// step (26 us a solve of 33 lines of 40 unknowns, against 21 us staged; the chain of banded
-// block solves this replaces took 125 us, one product with an explicit inverse 26 us at one
-// row and 36 us at 16, after 0.5 to 0.8 ms of forming the inverse).  The blocks are
+// step.  33 lines of 40 unknowns, from L2 and from memory: 24 and 24 to 27 us at 1 to 15 rows (30
+// unstaged), 34 and 46 to 48 at 16 to 33, 42 and 63 at 64, 75 and 92 at 128; the chain of banded
+// block solves this replaces took 125 us.  (One product with an explicit inverse took less for few
+// rows of wide lines: a V-cycle over 27 lines of 54 at one row in FP32 29 us, 37 with this, after
+// 1.7 ms of forming the hierarchy where 0.33 are enough.)  The blocks are
 // dealt out to the groups in the order of their elimination, so every group has nearly the
 // same number.  A block's right-hand side lives in the CTA whose group owns it; its two
 // neighbours' updates arrive there by remote stores into a buffer a side (two sets, used by
 // alternate strides, so that a set is read before it is written again) and are added by the
 // owner in a fixed order; a solution block is written to all of the row's CTAs.
-template <int NB>
+template <int NB, int CL>
 struct TreeRow {
   static constexpr int B = 8 * NB, NC = 2 * NB, BB = B * B, kGroup = 4 * B;
   static constexpr int kThreads = kTreeGroups * kGroup;
@@ -417,7 +423,7 @@ struct TreeRow {
     bh = factor;
     nb = nblocks;
     staged = nstaged;
-    all = (int)gridDim.x * kTreeGroups;
+    all = (CL ? CL : (int)gridDim.x) * kTreeGroups;
     lg = 31 - __clz(all);
     own = tree_own(nb, all);
     levels = 0;
@@ -576,7 +582,7 @@ struct TreeRow {
         if (share)
 #pragma unroll
           for (int rk = 0; rk < kTreeCluster; ++rk)
-            if (rk < (int)gridDim.x) cluster.map_shared_rank(vx, rk)[i * B + t] = v;
+            if (rk < (CL ? CL : (int)gridDim.x)) cluster.map_shared_rank(vx, rk)[i * B + t] = v;
         publish(i, t, v);
       }
     };
@@ -614,16 +620,17 @@ struct TreeRow {
 
 // One row's coarse solve on a cluster (TreeRow), between global vectors.  SHARED: a block may hold
 // several grid lines (24 or 32 unknowns; without it the index arithmetic of one line a block is
-// simpler, and the kernel 0.7 us shorter).
-template <int NB, int D, typename T, bool SHARED>
-__global__ void __launch_bounds__(TreeRow<NB>::kThreads)
+// simpler, and the kernel 0.7 us shorter).  CL: the CTAs a row, or 0
+// for any (tree_eight).
+template <int NB, int D, typename T, bool SHARED, int CL>
+__global__ void __launch_bounds__(TreeRow<NB, CL>::kThreads)
     tree_solve_kernel(const T* __restrict__ b, T* __restrict__ x, long long rs, const double* __restrict__ blocks,
                       int nb, int staged, int by_col, int nnx, int nny, const uint8_t* __restrict__ fixed,
                       const int* __restrict__ row_map, int hrows, const RowState* __restrict__ rst, TreeBlock of) {
   constexpr int B = 8 * NB;
   extern __shared__ __align__(16) double sm[];
   const int srow = blockIdx.y;
-  TreeRow<NB> tree;
+  TreeRow<NB, CL> tree;
   // The factor is fetched beside the kernel before: it is complete when its solves are launched
   // (the stream has waited for its event).  A row map is the caller's, and on a hierarchy of one
   // level the kernel before may be the one that writes it.
@@ -796,11 +803,23 @@ static int tree_factor(const CoarseDesc& co, int hrows, int* status, cudaStream_
   return check_launch("coarse factor");
 }
 
+// The form of the kernel for eight CTAs a row: with their number fixed it is 0.5 us shorter up to 32
+// unknowns a block (17.0 us for 25 lines of 26), and longer from 40 on (24.1 and 23.7 us for 33
+// lines of 34, 39.8 and 33.6 for 27 of 54).
+template <int NB>
+constexpr int tree_eight() {
+  return NB <= 4 ? kTreeCluster : 0;
+}
+
 // A solve's launch: each cluster size with as many blocks staged as fit its CTAs, and with none
 // (more CTAs an SM).  A step without its block staged takes about 1.4 times as long.
 template <int NB, int D, typename T, bool SHARED>
 static int tree_launch(const CoarseDesc& co, int nrows, TreeLaunch& best) {
-  STT_TRY(allow_smem<tree_solve_kernel<NB, D, T, SHARED>>());
+  constexpr auto eight = tree_solve_kernel<NB, D, T, SHARED, tree_eight<NB>()>;
+  constexpr auto any = tree_solve_kernel<NB, D, T, SHARED, 0>;
+  constexpr int kThreads = TreeRow<NB, 0>::kThreads;
+  STT_TRY(allow_smem<eight>());
+  STT_TRY(allow_smem<any>());
   const size_t task = 8 * kTreeGroups * tree_task(co.B);
   for (int cl = kTreeCluster; cl >= 1; cl /= 2) {
     const int all = cl * kTreeGroups, own = tree_own(co.nb, all), steps = tree_steps(co.nb, all);
@@ -808,9 +827,11 @@ static int tree_launch(const CoarseDesc& co, int nrows, TreeLaunch& best) {
     if (vec > kTreeSmem) break;
     const int most = (int)std::min<size_t>(own, (kTreeSmem - vec) / task);
     for (int st : {most, 0}) {
+      const size_t bytes = vec + st * task;
       int n = 0;
-      STT_TRY((resident_clusters<tree_solve_kernel<NB, D, T, SHARED>>(cl, TreeRow<NB>::kThreads, vec + st * task, &n)));
-      best.consider(nrows, n, cl, st, vec + st * task, steps * (st == own ? 5 : 7));
+      STT_TRY(cl == kTreeCluster ? resident_clusters<eight>(cl, kThreads, bytes, &n)
+                                 : resident_clusters<any>(cl, kThreads, bytes, &n));
+      best.consider(nrows, n, cl, st, bytes, steps * (st == own ? 5 : 7));
     }
     if (cl == kTreeCluster && most == own && best.cost == 5 * steps) break;  // one wave: nothing is faster
   }
@@ -819,14 +840,16 @@ static int tree_launch(const CoarseDesc& co, int nrows, TreeLaunch& best) {
 
 template <int NB, int D, typename T, bool SHARED>
 static int tree_run(const stt_hier* h, int nrows, const T* b, T* x, long long rs, const RowState* rst,
-                      cudaStream_t st) {
+                    cudaStream_t st) {
   const LevelDesc& lv = h->lv[h->nlevels - 1];
   const CoarseDesc& co = h->co;
   TreeLaunch l;
   STT_TRY((tree_launch<NB, D, T, SHARED>(co, nrows, l)));
-  launch_clusters((tree_solve_kernel<NB, D, T, SHARED>), l.cluster, dim3(l.cluster, nrows), TreeRow<NB>::kThreads, l.smem, st,
-                  true, b, x, rs, co.blocks, co.nb, l.staged, co.by_col, lv.nnx, lv.nny, lv.fixed, h->row_map, h->hrows,
-                  rst, tree_block(h));
+  auto* const kernel = l.cluster == kTreeCluster ? tree_solve_kernel<NB, D, T, SHARED, tree_eight<NB>()>
+                                                 : tree_solve_kernel<NB, D, T, SHARED, 0>;
+  launch_clusters(kernel, l.cluster, dim3(l.cluster, nrows), TreeRow<NB, 0>::kThreads, l.smem, st, true, b, x, rs,
+                  co.blocks, co.nb, l.staged, co.by_col, lv.nnx, lv.nny, lv.fixed, h->row_map, h->hrows, rst,
+                  tree_block(h));
   return check_launch("coarse solve");
 }
 

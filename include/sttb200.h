@@ -151,7 +151,7 @@ long long stt_hier_workspace_bytes(int d, int nelx, int nely, int hrows,
 /* Build the Galerkin hierarchy on the device (torch_mg.build_hierarchy): level 0 is
  * K(rho) (+ lumped reaction), coarser levels the exact Galerkin products stored as
  * symmetric 9-point block stencils, the coarsest factorised in FP64 (odd-even elimination
- * of its grid lines; block-banded Cholesky for lines above 64 unknowns).
+ * of its grid lines; block-banded Cholesky for lines above 64 unknowns and very long grids).
  * precision STT_FP32 keeps FP32 copies for an FP32 V-cycle.  reaction may be NULL. */
 int stt_hier_create(stt_hier** out, void* workspace, long long ws_bytes, int d, int nelx,
                     int nely, int hrows, const double* rho, long long rho_rs,
@@ -182,8 +182,8 @@ int stt_hier_info(const stt_hier* h, int* nlevels, int* dims, int max_levels);
 
 /* Launch shapes of the solves on h (stt_vcycle, stt_pcg_mg, stt_level_apply; views made
  * afterwards inherit them): pcg_band, the grid rows a block of the PCG's level-0 passes
- * marches (8, 16 or 32; 0: the built-in choice, 32 or shorter while the rows give fewer
- * than two waves of blocks), and level_waves, the blocks the stencil levels' kernels aim
+ * marches (8, 16 or 32; 0: the built-in choice, 32 or shorter, down to 4, while the rows give
+ * fewer than two waves of blocks), and level_waves, the blocks the stencil levels' kernels aim
  * at in waves of one block per SM (1..64; 0: four).  Results do not depend on them beyond
  * the order of the block reductions.  No reference counterpart: set by this library's
  * autotuner (sttopt_b200.autotune), which times the candidates on the hierarchy. */

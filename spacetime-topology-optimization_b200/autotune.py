@@ -8,7 +8,9 @@ measurement: for a hierarchy it times a few PCG iterations of each candidate on 
 hierarchy itself (CUDA events on the current stream, the heuristic always among the
 candidates, best of two sweeps) and caches the fastest per key
 ``(dofs per node, nelx, nely, precision, batch rows, gamma)``.  Launch shapes change no
-result beyond the order of the blocks' partial sums.
+result beyond the order of the blocks' partial sums.  The heuristic's PCG bands go down to 4
+rows, which only candidate 0 reaches; the bands of the chained smoothing passes and the coarse
+solve's cluster size follow from the grid and the rows alone and are not tuned.
 
 Modes: off (default; the heuristics), ``enable()`` (tune every key the solves meet the
 first time, then reuse it), ``freeze()`` (apply cached choices, tune nothing new).  The

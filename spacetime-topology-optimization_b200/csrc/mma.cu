@@ -509,7 +509,7 @@ inline int assemble_rows(int m, int nd) { return 8 * gram_side(m, nd); }  // wit
 // The advance pass's stored rows.  Its second delx row takes the padded tile of 23, 24, 47 and 48
 // constraints past half an SM's shared memory; without the padding two blocks fit (a fragment's
 // rows past the last repeat it, and their products are not read).  The update at 1M variables:
-// 12.1 -> 9.9, 11.3 -> 9.2, 25.1 -> 20.3 and 25.5 -> 20.5 ms.  With no more blocks than SMs the
+// 12.1 -> 9.9, 11.2 -> 9.2, 25.1 -> 20.3 and 25.5 -> 20.7 ms.  With no more blocks than SMs the
 // padding stays: two of them, resident while the step pass drains, would share an SM that it
 // leaves idle (20000 variables, 47 constraints: 2.97 -> 3.36 ms).
 constexpr bool trims_rows(int mb) { return mb == 24 || mb == 48; }

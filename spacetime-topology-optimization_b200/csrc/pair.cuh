@@ -15,7 +15,7 @@ namespace stt {
 // residual as it appears (it is never written), the post-smoothing pass adds the prolonged
 // correction to the iterate as it loads it.
 //
-// The state of two columns takes 150-168 registers, so 12 warps an SM, too few to wait out a
+// The state of two columns takes 142-152 registers, so 12 warps an SM, too few to wait out a
 // memory latency at each row: a row's data comes by asynchronous copies into a ring of four to
 // seven rows ahead in shared memory.  All of it does, flags and coarse values too: plain
 // loads two rows ahead of their use, queued behind the copies in the L1, cost half the time.

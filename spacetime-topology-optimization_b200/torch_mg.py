@@ -161,7 +161,7 @@ class _Level:
         self.density = density
         self.reaction_diag = reaction_diag
         self.keff = None  # coarse operators live on the device as stencils
-        self.chol = None  # the coarse factor lives on the device in band blocks
+        self.chol = None  # the coarse factor lives on the device in blocks
         self._edofMat = edofMat
         self._diag = None
         self._mask = None

@@ -718,8 +718,8 @@ void coarse_plan(const LevelDesc& c, int d, int hrows, CoarseDesc& co) {
   co.nb = (co.n + co.B - 1) / co.B;
 }
 
-// How many clusters of `cluster` CTAs the device holds at once (several kinds of launch a kernel:
-// the answers are kept, at most kMax of them).
+// How many clusters of `cluster` CTAs the device holds at once, 0 if none (several kinds of launch a
+// kernel: the answers are kept, at most kMax of them).
 template <auto Kernel>
 static int resident_clusters(int cluster, int threads, size_t smem, int* n) {
   struct Known {
@@ -748,7 +748,10 @@ static int resident_clusters(int cluster, int threads, size_t smem, int* n) {
   cfg.dynamicSmemBytes = smem;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  STT_TRY(check_cuda(cudaOccupancyMaxActiveClusters(n, Kernel, &cfg), "resident clusters"));
+  if (cudaOccupancyMaxActiveClusters(n, Kernel, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    *n = 0;  // the device takes none of this size
+  }
   // clusters of eight with more than one CTA an SM leave gaps: of 33 and of 48, 28 and 40 ran at once
   if (cluster == kTreeCluster && *n * cluster > 148) *n -= *n / 8;
   if (count == kMax) count = 0;
@@ -767,7 +770,7 @@ static int tree_steps(int nb, int units) {
 // times what a step costs there.  Fewer CTAs a row take more steps but let more rows run at once
 // (15 clusters of eight, 33 of four, 74 of two on B200's 148 SMs at one CTA each).  A V-cycle of a
 // one-level hierarchy, 33 lines of 40 unknowns, always eight CTAs -> this rule: 16 rows 51 -> 39 us,
-// 33 rows 74 -> 45, 64 rows 122 -> 55, 128 rows 223 -> 86 (the chain over the lines: 147 to 162); 27
+// 33 rows 74 -> 40, 64 rows 122 -> 55, 128 rows 223 -> 86 (the chain over the lines: 147 to 162); 27
 // lines of 54 at 128 rows 404 -> 179 (204), their factorisation 2.2 -> 1.35 ms (1.33).  The
 // rows' results do not depend on it.
 struct TreeLaunch {

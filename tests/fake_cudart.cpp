@@ -21,6 +21,7 @@ std::map<const void*, Kernel>& kernels() {
   return *k;
 }
 std::string refuse;
+int most = 8;  // CTAs a cluster
 cudaError_t last = cudaSuccess;
 struct {
   dim3 grid, block;
@@ -50,6 +51,7 @@ const Kernel* find(const char* part, const Kernel* after) {
 extern "C" {
 // ---- the test's side: of the launched kernels whose (mangled) name contains `part`
 void fake_refuse(const char* part) { refuse = part; }
+void fake_most(int ctas) { most = ctas; }
 int fake_launches(const char* part) {
   int n = 0;
   for (const Kernel* k = nullptr; (k = find(part, k));) n += k->launches;
@@ -132,7 +134,9 @@ cudaError_t cudaFuncSetAttribute(const void* fn, cudaFuncAttribute at, int v) {
   return cudaSuccess;
 }
 cudaError_t cudaOccupancyMaxActiveClusters(int* n, const void*, const cudaLaunchConfig_t* c) {
-  return *n = 120 / (int)c->attrs[0].val.clusterDim.x, cudaSuccess;
+  const int cl = (int)c->attrs[0].val.clusterDim.x;
+  if (cl > most) return fail(cudaErrorInvalidClusterSize);
+  return *n = 120 / cl, cudaSuccess;
 }
 cudaError_t cudaGetDevice(int* d) { return *d = 0, cudaSuccess; }
 cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) { return *v = 227 << 10, cudaSuccess; }

@@ -67,6 +67,21 @@ def fake(tmp_path_factory):
     return run
 
 
+@pytest.mark.parametrize("most", [4, 1, 0])
+def test_a_device_with_smaller_clusters_takes_those(fake, most):
+    """(A partition of a GPU may have fewer SMs together than a cluster of eight needs.)"""
+    got = fake(r"""
+lib.fake_most(I(case["most"]))
+try:
+""" + "".join("    " + line + "\n" for line in CYCLE.splitlines()) + r"""
+except AssertionError:
+    print(json.dumps("none"))
+else:
+    print(json.dumps([vcycle(), pcg(), lib.fake_cluster(b"tree_factor_kernel"), lib.fake_cluster(b"tree_solve_kernel")]))
+""", d=2, nelx=40, nely=20, mce=200, prec=1, rows=2, most=most)
+    assert got == ("none" if most == 0 else [0, 0, most, most]), got
+
+
 @pytest.mark.parametrize("d,nelx,nely,blocks", [(1, 600, 1, 38), (2, 1, 600, 76), (2, 300, 2, 61), (2, 100, 7, 51),
                                                 (2, 80, 8, 81), (2, 45, 15, 46), (1, 63, 1, 64)])
 def test_short_lines_of_a_long_coarsest_grid_share_blocks(fake, d, nelx, nely, blocks):
